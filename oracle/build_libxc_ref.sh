@@ -10,7 +10,8 @@
 # named that way must be a DEReK checkout (Source/electronic.f90 and the
 # vendored libxc present), else this fails.  With neither given, the build
 # container's mount point below is tried, and the checker is skipped (exit 0)
-# when no DEReK tree is there; a directory there that is not one also fails.
+# when that is absent or empty; another directory there that is not a DEReK
+# tree also fails.
 set -e
 HERE=$(cd "$(dirname "$0")" && pwd)
 REF=${1:-$DEREK_REFERENCE}
@@ -18,7 +19,7 @@ EXPLICIT=1
 if [ -z "$REF" ]; then
   REF=/root/reference
   EXPLICIT=0
-  if [ ! -e "$REF" ]; then
+  if [ ! -e "$REF" ] || [ -z "$(ls -A "$REF" 2>/dev/null)" ]; then
     echo "no DEReK tree (set DEREK_REFERENCE); skipping the libxc checker" >&2
     exit 0
   fi
