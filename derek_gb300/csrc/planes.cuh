@@ -144,14 +144,4 @@ template <int N, int RY, bool DENSITY> struct RowsShape {
   static constexpr size_t SMEM = (size_t)XP * PLANE + 2 * N + 16;
 };
 
-inline int sm_count() {
-  static int n = [] {
-    int dev = 0, c = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-    return c > 0 ? c : 1;
-  }();
-  return n;
-}
-
 }  // namespace derek

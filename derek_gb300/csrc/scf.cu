@@ -55,11 +55,11 @@ int overlap_all(derek_gpu *h, const void *A, const void *B, double2 *out, int he
                       (const float2 *)B, h->d_opart, h->d_opart_off, out, h->d_mat_off, hermitize,
                       h->d_status, h->stream);
   else if (h->prec == DEREK_PREC_FP64)
-    launch_overlap<double>(h->tab_band, 0, h->nks, h->max_nb_band, h->max_npw_band, ks,
+    launch_overlap<double>(h->tab_band, 0, h->nks, h->max_nb_band, h->max_npw_band, ks, h->split_min,
                            (const double2 *)A, (const double2 *)B, h->d_opart, h->d_opart_off, out,
                            h->d_mat_off, hermitize, h->stream);
   else
-    launch_overlap<float>(h->tab_band, 0, h->nks, h->max_nb_band, h->max_npw_band, ks,
+    launch_overlap<float>(h->tab_band, 0, h->nks, h->max_nb_band, h->max_npw_band, ks, h->split_min,
                           (const float2 *)A, (const float2 *)B, h->d_opart, h->d_opart_off, out,
                           h->d_mat_off, hermitize, h->stream);
   return DEREK_OK;
@@ -367,11 +367,14 @@ extern "C" int derek_scf_alloc(derek_gpu_t *h) {
   }
   long long moff = 0, poff = 0;
   std::vector<long long> opart_off;
+  long long total_npw = 0;
+  for (const auto &K : h->ks) total_npw += K.npw;
+  h->split_min = overlap_split_min(total_npw);
   for (const auto &K : h->ks) {
     h->mat_off.push_back(moff);
     moff += (long long)K.nb * K.nb;
     opart_off.push_back(poff);
-    poff += (long long)((K.npw + kOverlapSplitMin - 1) / kOverlapSplitMin) * K.nb * K.nb;
+    poff += (long long)((K.npw + h->split_min - 1) / h->split_min) * K.nb * K.nb;
     h->max_npw = std::max(h->max_npw, K.npw);
   }
   for (const auto &K : h->ks_band) {
@@ -478,11 +481,11 @@ int derek_gpu_overlap(derek_gpu_t *h, int s, int k, double *out) {
     }
   }
   else if (h->prec == DEREK_PREC_FP64)
-    launch_overlap<double>(h->tab, ki, 1, K.nb, K.npw, h->tune.ksplit, (const double2 *)h->cur_psi(),
+    launch_overlap<double>(h->tab, ki, 1, K.nb, K.npw, h->tune.ksplit, h->split_min, (const double2 *)h->cur_psi(),
                            (const double2 *)h->cur_psi(), h->d_opart, h->d_opart_off, h->d_S,
                            h->d_mat_off, 0, h->stream);
   else
-    launch_overlap<float>(h->tab, ki, 1, K.nb, K.npw, h->tune.ksplit, (const float2 *)h->cur_psi(),
+    launch_overlap<float>(h->tab, ki, 1, K.nb, K.npw, h->tune.ksplit, h->split_min, (const float2 *)h->cur_psi(),
                           (const float2 *)h->cur_psi(), h->d_opart, h->d_opart_off, h->d_S,
                           h->d_mat_off, 0, h->stream);
   DEREK_CUDA(h, cudaGetLastError());

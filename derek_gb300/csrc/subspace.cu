@@ -5,6 +5,7 @@
 //   Hermitian Jacobi eigensolver of the projected Hamiltonian (FP64)
 // These replace the empty wave_dot_* routines (Source/wave.f90:929-1036)
 // with the full matrices a Rayleigh-Ritz step needs.
+#include <algorithm>
 #include <cstdio>
 
 #include "subspace.cuh"
@@ -15,89 +16,180 @@ namespace derek {
 
 // ---------------------------------------------------------------------------
 // Overlap: part[ks][split] = sum_{G in split} conj(A_i(G)) B_j(G)
+//
+// Bound by the FP64 pipe (GB300: 2 lanes per clock and SM, and a warp
+// instruction costs its 16 clocks however few of its lanes are active) or, in
+// FP32, by shared-memory loads.  So the unit of work is one MT x MT tile of
+// band pairs and the tiles of a k-set are numbered one after another and dealt
+// to the threads (P per thread): no lane idles on a band count that is no
+// multiple of a tile, and A = B computes the upper triangle only (the lower
+// one is its exact conjugate).  Every block stages OKC coefficients of all
+// bands.  The split along G is as fine as it takes to give every SM blocks
+// (launch_overlap).  Measured, FP64: 12 bands x 1,510 plane waves 716 -> 12 us
+// (A = B) and 15 us; 84 bands x 17,529 on 4 k-points 8.2 -> 2.8 ms (A = B) and
+// 5.5 ms (1.0 and 2.0 x 10^9 multiply-adds at the pipe's rate: 1.6 and 3.2 ms).
 // ---------------------------------------------------------------------------
-constexpr int OT = 16;   // output tile
-constexpr int OKC = 32;  // K chunk staged in shared memory
+template <typename R> struct OverlapShape;
+// FP64: one pair per tile, its four fused multiply-adds hide both loads
+template <> struct OverlapShape<double> {
+  static constexpr int MT = 1, OKC = 16, PMAX = 8;
+};
+// FP32: 2 x 2 pairs, half the shared loads per multiply-add
+template <> struct OverlapShape<float> {
+  static constexpr int MT = 2, OKC = 32, PMAX = 4;
+};
 
-template <typename R>
-__global__ void __launch_bounds__(256) k_overlap_partial(const Tables t, int ks_begin,
-                                                         const cplx<R> *__restrict__ A,
-                                                         const cplx<R> *__restrict__ B,
-                                                         double2 *__restrict__ part,
-                                                         const long long *__restrict__ part_off,
-                                                         int ksplit) {
-  __shared__ cplx<R> As[OT][OKC + 1];
-  __shared__ cplx<R> Bs[OT][OKC + 1];
+template <typename R, int P, bool SAME>
+__global__ void __launch_bounds__(256) k_overlap_pairs(const Tables t, int ks_begin,
+                                                       const cplx<R> *__restrict__ A,
+                                                       const cplx<R> *__restrict__ B,
+                                                       double2 *__restrict__ part,
+                                                       const long long *__restrict__ part_off,
+                                                       int ksplit) {
+  constexpr int MT = OverlapShape<R>::MT, OKC = OverlapShape<R>::OKC, LD = OKC + 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ksi = ks_begin + blockIdx.z;
   const KSetDev &K = t.ks[ksi];
   if (!t.sys[K.sys].active) return;
   const int nb = K.nb;
-  const int nt = (nb + OT - 1) / OT;
-  const int ti = blockIdx.x / nt, tj = blockIdx.x - (blockIdx.x / nt) * nt;
-  if (ti >= nt) return;
-  const int split = blockIdx.y;
-  const int g0 = split * ksplit;
-  if (g0 >= K.npw) return;
+  const int nt = (nb + MT - 1) / MT, rows = nt * MT;
+  const int np = SAME ? nt * (nt + 1) / 2 : nt * nt;
+  const int p0 = blockIdx.x * blockDim.x * P;
+  const int g0 = blockIdx.y * ksplit;
+  if (p0 >= np || g0 >= K.npw) return;
   const int g1 = min(K.npw, g0 + ksplit);
-  const int ty = threadIdx.x / OT, tx = threadIdx.x % OT;
-  const int i0 = ti * OT, j0 = tj * OT;
+  cplx<R> *As = reinterpret_cast<cplx<R> *>(smem_raw);   // [rows][LD]
+  cplx<R> *Bs = SAME ? As : As + rows * LD;
   const cplx<R> *Ab = A + K.psi_off;
   const cplx<R> *Bb = B + K.psi_off;
-  R ar = 0, ai = 0;
+  int oi[P], oj[P];   // shared rows of the thread's tiles (-1: none)
+  cplx<R> acc[P][MT][MT];
+#pragma unroll
+  for (int q = 0; q < P; ++q) {
+    const int p = p0 + (int)threadIdx.x + q * (int)blockDim.x;
+    oi[q] = oj[q] = -1;
+    if (p < np) {
+      int i, j;
+      if (SAME) {
+        // row i of the upper triangle starts at i nt - i (i - 1) / 2
+        const float w = 2.f * nt + 1.f;
+        i = min(nt - 1, max(0, (int)(0.5f * (w - sqrtf(fmaxf(w * w - 8.f * p, 0.f))))));
+        while (i * nt - i * (i - 1) / 2 > p) --i;
+        while ((i + 1) * nt - (i + 1) * i / 2 <= p) ++i;
+        j = i + p - (i * nt - i * (i - 1) / 2);
+      } else {
+        i = p / nt;
+        j = p - i * nt;
+      }
+      oi[q] = i * MT * LD;
+      oj[q] = j * MT * LD;
+    }
+#pragma unroll
+    for (int a = 0; a < MT; ++a)
+#pragma unroll
+      for (int b = 0; b < MT; ++b) acc[q][a][b] = mk<R>(0, 0);
+  }
   for (int k0 = g0; k0 < g1; k0 += OKC) {
-    for (int e = threadIdx.x; e < OT * OKC; e += blockDim.x) {
+    for (int e = threadIdx.x; e < rows * OKC; e += blockDim.x) {
       const int r = e / OKC, c = e % OKC;
       const int g = k0 + c;
-      const int ia = i0 + r, jb = j0 + r;
-      As[r][c] = (ia < nb && g < g1) ? Ab[(long long)ia * K.npw_pad + g] : mk<R>(0, 0);
-      Bs[r][c] = (jb < nb && g < g1) ? Bb[(long long)jb * K.npw_pad + g] : mk<R>(0, 0);
+      const bool in = r < nb && g < g1;
+      As[r * LD + c] = in ? Ab[(long long)r * K.npw_pad + g] : mk<R>(0, 0);
+      if (!SAME) Bs[r * LD + c] = in ? Bb[(long long)r * K.npw_pad + g] : mk<R>(0, 0);
     }
     __syncthreads();
-#pragma unroll 8
+#pragma unroll 2
     for (int c = 0; c < OKC; ++c) {
-      const cplx<R> a = As[ty][c], b = Bs[tx][c];
-      ar += a.x * b.x + a.y * b.y;
-      ai += a.x * b.y - a.y * b.x;
+#pragma unroll
+      for (int q = 0; q < P; ++q) {
+        if (oi[q] < 0) continue;
+        cplx<R> a[MT], b[MT];
+#pragma unroll
+        for (int u = 0; u < MT; ++u) {
+          a[u] = As[oi[q] + u * LD + c];
+          b[u] = Bs[oj[q] + u * LD + c];
+        }
+#pragma unroll
+        for (int u = 0; u < MT; ++u)
+#pragma unroll
+          for (int v = 0; v < MT; ++v) {
+            acc[q][u][v].x += a[u].x * b[v].x + a[u].y * b[v].y;
+            acc[q][u][v].y += a[u].x * b[v].y - a[u].y * b[v].x;
+          }
+      }
     }
     __syncthreads();
   }
-  const int i = i0 + ty, j = j0 + tx;
-  if (i < nb && j < nb)
-    part[part_off[ksi] + ((long long)split * nb + i) * nb + j] = make_double2((double)ar, (double)ai);
+  double2 *dst = part + part_off[ksi] + (long long)blockIdx.y * nb * nb;
+#pragma unroll
+  for (int q = 0; q < P; ++q) {
+    if (oi[q] < 0) continue;
+    const int i0 = oi[q] / LD, j0 = oj[q] / LD;
+#pragma unroll
+    for (int u = 0; u < MT; ++u)
+#pragma unroll
+      for (int v = 0; v < MT; ++v)
+        if (i0 + u < nb && j0 + v < nb)
+          dst[(i0 + u) * nb + j0 + v] = make_double2((double)acc[q][u][v].x, (double)acc[q][u][v].y);
+  }
 }
 
-__global__ void k_overlap_reduce(const Tables t, int ks_begin, const double2 *__restrict__ part,
-                                 const long long *__restrict__ part_off, int ksplit,
-                                 double2 *__restrict__ out, const long long *__restrict__ mat_off,
-                                 int hermitize) {
+// Sum of the splits, one pair (i, j), i <= j, by kReduceLanes lanes: each adds
+// every kReduceLanes-th split, then a fixed shuffle tree (one thread per pair
+// waited on a chain of up to ~50 dependent FP64 additions, 23 us at 12 bands).
+// half: only the upper triangle was computed, the matrix is Hermitian by
+// construction; hermitize: the mean of the two triangles.
+constexpr int kReduceLanes = 8;
+__global__ void __launch_bounds__(256) k_overlap_reduce(const Tables t, int ks_begin, const double2 *__restrict__ part,
+                                                        const long long *__restrict__ part_off, int ksplit,
+                                                        double2 *__restrict__ out,
+                                                        const long long *__restrict__ mat_off, int hermitize,
+                                                        int half) {
   const int ksi = ks_begin + blockIdx.x;
   const KSetDev &K = t.ks[ksi];
   if (!t.sys[K.sys].active) return;
   const int nb = K.nb;
+  const int lane = threadIdx.x % kReduceLanes;
+  const int e = (blockIdx.y * blockDim.x + threadIdx.x) / kReduceLanes;
+  const int i = e / nb, j = e - i * nb;
+  const bool on = e < nb * nb && i <= j;
   const int nsplit = (K.npw + ksplit - 1) / ksplit;
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    double x = 0, y = 0;
-    for (int s = 0; s < nsplit; ++s) {
-      const double2 v = part[part_off[ksi] + (long long)s * nb * nb + e];
-      x += v.x;
-      y += v.y;
+  const double2 *src = part + part_off[ksi];
+  const int f = j * nb + i;
+  const bool lower = on && !half && i < j;
+  double2 u = make_double2(0, 0), l = make_double2(0, 0);
+#pragma unroll 4
+  for (int s = lane; s < (on ? nsplit : 0); s += kReduceLanes) {
+    const double2 v = src[(long long)s * nb * nb + e];
+    u.x += v.x;
+    u.y += v.y;
+    if (lower) {
+      const double2 w = src[(long long)s * nb * nb + f];
+      l.x += w.x;
+      l.y += w.y;
     }
-    out[mat_off[ksi] + e] = make_double2(x, y);
   }
-  if (hermitize) {
-    __syncthreads();
-    double2 *M = out + mat_off[ksi];
-    for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-      const int i = e / nb, j = e % nb;
-      if (i < j) {
-        const double2 a = M[i * nb + j], b = M[j * nb + i];
-        const double2 h = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y - b.y));
-        M[i * nb + j] = h;
-        M[j * nb + i] = make_double2(h.x, -h.y);
-      } else if (i == j) {
-        M[e].y = 0.0;
-      }
-    }
+#pragma unroll
+  for (int w = kReduceLanes / 2; w > 0; w >>= 1) {
+    u.x += __shfl_down_sync(0xffffffffu, u.x, w, kReduceLanes);
+    u.y += __shfl_down_sync(0xffffffffu, u.y, w, kReduceLanes);
+    l.x += __shfl_down_sync(0xffffffffu, l.x, w, kReduceLanes);
+    l.y += __shfl_down_sync(0xffffffffu, l.y, w, kReduceLanes);
+  }
+  if (!on || lane) return;
+  double2 *M = out + mat_off[ksi];
+  if (i == j) {
+    M[e] = make_double2(u.x, hermitize || half ? 0.0 : u.y);
+  } else if (half) {
+    M[e] = u;
+    M[f] = make_double2(u.x, -u.y);
+  } else if (hermitize) {
+    const double2 h = make_double2(0.5 * (u.x + l.x), 0.5 * (u.y - l.y));
+    M[e] = h;
+    M[f] = make_double2(h.x, -h.y);
+  } else {
+    M[e] = u;
+    M[f] = l;
   }
 }
 
@@ -690,21 +782,60 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256)
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+int overlap_split_min(long long total_npw) {
+  const long long s = (total_npw / (4 * sm_count()) + 31) / 32 * 32;
+  return (int)std::max<long long>(32, std::min<long long>(kOverlapSplitMin, s));
+}
+
+template <typename R, bool SAME>
+static void overlap_go(const Tables &t, int ks_begin, int nks, int max_nb, int max_npw, int ksplit, int split_min,
+                       const cplx<R> *A, const cplx<R> *B, double2 *part, const long long *part_off, double2 *out,
+                       const long long *mat_off, int hermitize, cudaStream_t st) {
+  using Sh = OverlapShape<R>;
+  const int nt = (max_nb + Sh::MT - 1) / Sh::MT;
+  const int np = SAME ? nt * (nt + 1) / 2 : nt * nt;
+  int P = 1;
+  while (P < Sh::PMAX && P * 256 < np) P *= 2;
+  const int groups = (np + 256 * P - 1) / (256 * P);
+  const int threads = ((np + groups * P - 1) / (groups * P) + 31) / 32 * 32;
+  // four blocks per SM where the buffers of the partial sums allow it, never
+  // longer than the planned split
+  const int want = std::max(1, (4 * sm_count() + groups * nks - 1) / (groups * nks));
+  const int fill = ((max_npw + want - 1) / want + Sh::OKC - 1) / Sh::OKC * Sh::OKC;
+  ksplit = std::min(ksplit, std::max(split_min, fill));
+  const size_t sm = (size_t)nt * Sh::MT * (Sh::OKC + 1) * sizeof(cplx<R>) * (SAME ? 1 : 2);
+  const dim3 grid(groups, (max_npw + ksplit - 1) / ksplit, nks);
+  auto go = [&](auto kern) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    derek::note_launch(), kern<<<grid, threads, sm, st>>>(t, ks_begin, A, B, part, part_off, ksplit);
+  };
+  switch (P) {
+    case 1: go(k_overlap_pairs<R, 1, SAME>); break;
+    case 2: go(k_overlap_pairs<R, 2, SAME>); break;
+    case 4: go(k_overlap_pairs<R, 4, SAME>); break;
+    default: go(k_overlap_pairs<R, Sh::PMAX, SAME>); break;
+  }
+  launch_overlap_reduce(t, ks_begin, nks, max_nb, part, part_off, ksplit, out, mat_off, hermitize, SAME, st);
+}
+
 template <typename R>
-void launch_overlap(const Tables &t, int ks_begin, int nks, int max_nb, int max_npw, int ksplit,
+void launch_overlap(const Tables &t, int ks_begin, int nks, int max_nb, int max_npw, int ksplit, int split_min,
                     const cplx<R> *A, const cplx<R> *B, double2 *part, const long long *part_off,
                     double2 *out, const long long *mat_off, int hermitize, cudaStream_t st) {
   if (nks <= 0) return;
-  const int nt = (max_nb + OT - 1) / OT;
-  dim3 grid(nt * nt, (max_npw + ksplit - 1) / ksplit, nks);
-  derek::note_launch(), k_overlap_partial<R><<<grid, 256, 0, st>>>(t, ks_begin, A, B, part, part_off, ksplit);
-  launch_overlap_reduce(t, ks_begin, nks, part, part_off, ksplit, out, mat_off, hermitize, st);
+  if (A == B)
+    overlap_go<R, true>(t, ks_begin, nks, max_nb, max_npw, ksplit, split_min, A, B, part, part_off, out, mat_off,
+                        hermitize, st);
+  else
+    overlap_go<R, false>(t, ks_begin, nks, max_nb, max_npw, ksplit, split_min, A, B, part, part_off, out, mat_off,
+                         hermitize, st);
 }
 
-void launch_overlap_reduce(const Tables &t, int ks_begin, int nks, const double2 *part,
+void launch_overlap_reduce(const Tables &t, int ks_begin, int nks, int max_nb, const double2 *part,
                            const long long *part_off, int ksplit, double2 *out,
-                           const long long *mat_off, int hermitize, cudaStream_t st) {
-  derek::note_launch(), k_overlap_reduce<<<nks, 256, 0, st>>>(t, ks_begin, part, part_off, ksplit, out, mat_off, hermitize);
+                           const long long *mat_off, int hermitize, int half, cudaStream_t st) {
+  const dim3 grid(nks, (max_nb * max_nb * kReduceLanes + 255) / 256);
+  derek::note_launch(), k_overlap_reduce<<<grid, 256, 0, st>>>(t, ks_begin, part, part_off, ksplit, out, mat_off, hermitize, half);
 }
 
 template <typename R>
@@ -775,7 +906,7 @@ void launch_jacobi(const Tables &t, int ks_begin, int nks, int max_nb, const dou
 }
 
 #define DEREK_INST(R)                                                                          \
-  template void launch_overlap<R>(const Tables &, int, int, int, int, int, const cplx<R> *,    \
+  template void launch_overlap<R>(const Tables &, int, int, int, int, int, int, const cplx<R> *, \
                                   const cplx<R> *, double2 *, const long long *, double2 *,   \
                                   const long long *, int, cudaStream_t);                      \
   template void launch_rotate<R>(const Tables &, int, int, int, int, cplx<R> *,               \

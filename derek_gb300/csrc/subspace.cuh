@@ -8,15 +8,21 @@ namespace derek {
 
 constexpr int kMaxBands = 128;   // per k-set (rotation kernel register tile)
 constexpr int kOverlapSplit = 2048;      // default split-K (complex coefficients per CTA)
-constexpr int kOverlapSplitMin = 512;    // smallest split the partial buffers hold
+constexpr int kOverlapSplitMin = 512;    // smallest split a plan may choose
+// Smallest split the partial buffers hold: a batch too small to give every SM
+// blocks at kOverlapSplitMin (total_npw: plane waves of all its k-sets) is cut
+// finer, down to 32 coefficients.
+int overlap_split_min(long long total_npw);
 
 template <typename R>
-void launch_overlap(const Tables &t, int ks_begin, int nks, int max_nb, int max_npw, int ksplit,
+// ksplit: the planned split, an upper bound; split_min: the smallest one that
+// `part` holds.  A == B computes one triangle.
+void launch_overlap(const Tables &t, int ks_begin, int nks, int max_nb, int max_npw, int ksplit, int split_min,
                     const cplx<R> *A, const cplx<R> *B, double2 *part, const long long *part_off,
                     double2 *out, const long long *mat_off, int hermitize, cudaStream_t st);
-void launch_overlap_reduce(const Tables &t, int ks_begin, int nks, const double2 *part,
+void launch_overlap_reduce(const Tables &t, int ks_begin, int nks, int max_nb, const double2 *part,
                            const long long *part_off, int ksplit, double2 *out,
-                           const long long *mat_off, int hermitize, cudaStream_t st);
+                           const long long *mat_off, int hermitize, int half, cudaStream_t st);
 // split-BF16 tcgen05 overlap (complex64 inputs, nb <= 128), same partial layout
 size_t overlap_tc_smem(int max_nb);
 void launch_overlap_tc(const Tables &t, int ks_begin, int nks, int max_nb, int max_npw, int ksplit,

@@ -361,7 +361,7 @@ void launch_overlap_tc(const Tables &t, int ks_begin, int nks, int max_nb, int m
   cudaFuncSetAttribute(k_overlap_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   dim3 grid((max_npw + ksplit - 1) / ksplit, nks);
   derek::note_launch(), k_overlap_tc<<<grid, TC_THREADS, sm, st>>>(t, ks_begin, X, Y, part, part_off, ksplit, status);
-  launch_overlap_reduce(t, ks_begin, nks, part, part_off, ksplit, out, mat_off, hermitize, st);
+  launch_overlap_reduce(t, ks_begin, nks, max_nb, part, part_off, ksplit, out, mat_off, hermitize, 0, st);
 }
 
 }  // namespace derek
