@@ -173,18 +173,18 @@ int density_items(derek_gpu *h, const void *psi, double *rho) {
 // 2x2 plane pass per band, the filter epilogue per component
 template <typename R>
 static void apply_spinor_class(derek_gpu *h, const Tables &t, int item_begin, int nitems, int nchunk,
-                               const int n[3], const void *in, const void *prev, void *out,
+                               const int n[3], int max_m, const void *in, const void *prev, void *out,
                                const Axpby *coef) {
   const cplx<R> *vnc;
   if constexpr (std::is_same<R, double>::value)
     vnc = h->d_vnc64;
   else
     vnc = h->d_vnc32;
-  launch_x_inv_lines<R>(t, item_begin, nitems, nchunk, n[0], n[0], (const cplx<R> *)in,
-                        (cplx<R> *)h->d_abuf, nullptr, h->stream);
-  launch_plane_spinor<R>(t, item_begin, nitems, n, (cplx<R> *)h->d_abuf, vnc, h->stream);
-  launch_x_fwd_lines<R>(t, item_begin, nitems, nchunk, n[0], n[0], (const cplx<R> *)h->d_abuf,
-                        (const cplx<R> *)in, (const cplx<R> *)prev, (cplx<R> *)out, coef, h->stream);
+  launch_x_inv<R>(t, item_begin, nitems, nchunk, n[0], n[0], max_m, (const cplx<R> *)in,
+                  (cplx<R> *)h->d_abuf, nullptr, h->stream);
+  launch_plane_spinor<R>(t, item_begin, nitems, n, max_m, (cplx<R> *)h->d_abuf, vnc, h->stream);
+  launch_x_fwd<R>(t, item_begin, nitems, nchunk, n[0], n[0], max_m, (const cplx<R> *)h->d_abuf,
+                  (const cplx<R> *)in, (const cplx<R> *)prev, (cplx<R> *)out, coef, h->stream);
 }
 
 template <typename R>
@@ -194,13 +194,13 @@ static void apply_spinor_t(derek_gpu *h, int item_begin, int nitems, const void 
     for (const auto &c : h->classes) {
       Tables t = h->tab;
       t.item_list = c.d_list;
-      apply_spinor_class<R>(h, t, 0, c.count, c.nchunk, c.n, in, prev, out, coef);
+      apply_spinor_class<R>(h, t, 0, c.count, c.nchunk, c.n, c.max_m, in, prev, out, coef);
     }
     return;
   }
   const KSetDev &K = h->ks[h->item_ks[item_begin]];
   apply_spinor_class<R>(h, h->tab, item_begin, nitems, (K.ncol + kColChunk - 1) / kColChunk,
-                        h->sys[K.sys].n, in, prev, out, coef);
+                        h->sys[K.sys].n, h->ks_max_m[h->item_ks[item_begin]], in, prev, out, coef);
 }
 
 int apply_spinor_items(derek_gpu *h, int item_begin, int nitems, const void *in, const void *prev,
@@ -219,8 +219,8 @@ template <typename R> static void density_spinor_t(derek_gpu *h, const void *psi
   for (const auto &c : h->classes) {
     Tables t = h->tab;
     t.item_list = c.d_list;
-    launch_x_inv_lines<R>(t, 0, c.count, c.nchunk, c.n[0], c.n[0], (const cplx<R> *)psi,
-                          (cplx<R> *)h->d_abuf, h->d_occw, h->stream);
+    launch_x_inv<R>(t, 0, c.count, c.nchunk, c.n[0], c.n[0], c.max_m, (const cplx<R> *)psi,
+                    (cplx<R> *)h->d_abuf, h->d_occw, h->stream);
   }
   launch_density_spinor<R>(h->tab, h->nks, h->max_n, (const cplx<R> *)h->d_abuf, h->d_occw,
                            h->d_partial, h->d_partial_off, h->stream);
@@ -425,9 +425,10 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
         FAIL(DEREK_ERR_UNSUPPORTED, "grid size " + std::to_string(nfine[i]) + " not 13-smooth");
       LinePlan &lp = S.lp[i];
       lp.n = nfine[i];
-      if (!line_plan(nfine[i], &lp.a, &lp.b))
+      int la = 0, lb = 0;
+      if (!line_plan(nfine[i], &la, &lb))
         FAIL(DEREK_ERR_UNSUPPORTED, "grid size " + std::to_string(nfine[i]) + " has no a*b <= 16*16 split");
-      lp.group = 32 / std::max(lp.a, lp.b);
+      set_line_split(lp, la, lb);
       auto it = tw_of.find(nfine[i]);
       if (it == tw_of.end()) {
         std::vector<double> w;

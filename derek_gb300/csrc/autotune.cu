@@ -7,8 +7,8 @@
 //   fft    the radix sequence of each grid-FFT length (Stockham stages of
 //          radix 2, 3, 4, 5, 7, 8, 11, 13 in any order: Hartree, Kerker and
 //          fft3d transforms), timed on a forward + backward full-grid pass;
-//   lines  register / fixed-length line kernels against the shared-memory
-//          four-step kernels with a runtime split n = a * b (a, b <= 16) per
+//   lines  register-line kernels against the shared-memory line kernels (FP64
+//          has only those), with the split n = a * b (a, b <= 16) of each
 //          length, timed on a full H.psi;
 //   rows   the row layout each grid-size class's H.psi stage kernels are
 //          dispatched with (the tightest layout holding the class's spheres,
@@ -261,11 +261,7 @@ void set_radices(derek_gpu *h, int n, const FftPlan &p) {
 void set_split(derek_gpu *h, int n, int a, int b) {
   for (auto &S : h->sys)
     for (int i = 0; i < 3; ++i)
-      if (S.lp[i].n == n) {
-        S.lp[i].a = a;
-        S.lp[i].b = b;
-        S.lp[i].group = 32 / std::max(a, b);
-      }
+      if (S.lp[i].n == n) set_line_split(S.lp[i], a, b);
 }
 
 std::vector<int> lengths(const derek_gpu *h) {
@@ -365,6 +361,9 @@ struct Tuner {
     h->tune.generic_lines = 1;
     float t_gen = time_hpsi();
     std::string splits;
+    std::map<int, std::pair<int, int>> planned;   // the untuned split of each length
+    for (const auto &S : h->sys)
+      for (int i = 0; i < 3; ++i) planned[S.lp[i].n] = {S.lp[i].a, S.lp[i].b};
     if (t_gen < 1.5f * t_fixed) {
       // search the splits of each length in turn (others at their current split)
       for (int n : ns) {
@@ -393,7 +392,9 @@ struct Tuner {
     h->tune.generic_lines = t_gen < t_fixed ? 1 : 0;
     cache[key] = h->tune.generic_lines ? "split" + splits : "fixed";
     ++tuned;
-    return DEREK_OK;
+    if (!h->tune.generic_lines)
+      for (const auto &p : planned) set_split(h, p.first, p.second.first, p.second.second);
+    return upload_sys(h);
   }
 
   int rows() {
@@ -571,7 +572,7 @@ std::string plan_json(const derek_gpu *h) {
         }
     o << "}";
   } else {
-    o << "\"" << (h->prec == DEREK_PREC_FP64 ? "fixed-length shared-memory kernels" : "register-line kernels")
+    o << "\"" << (h->prec == DEREK_PREC_FP64 ? "shared-memory line kernels" : "register-line kernels")
       << "\"";
   }
   o << ", \"rows\": {";

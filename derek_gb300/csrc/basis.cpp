@@ -132,6 +132,25 @@ bool radix_plan(int n, int radices[8], int *nstages) {
 }
 
 bool line_plan(int n, int *a, int *b) {
+  // a coprime pair when there is one (no twiddles), the smallest larger factor
+  // first, larger factor as a: the step over b holds V(r) too
+  int best = 0;
+  for (int x = 1; x <= 16; ++x) {
+    if (n % x || n / x > 16) continue;
+    const int y = n / x;
+    int p = x, q = y;
+    while (q) {
+      const int t = p % q;
+      p = q;
+      q = t;
+    }
+    if (p == 1 && x >= y && (!best || x < best)) best = x;
+  }
+  if (best) {
+    *a = best;
+    *b = n / best;
+    return true;
+  }
   int best_a = 0, best_span = 1 << 30, best_pow2 = 0;
   for (int x = 1; x <= 16; ++x) {
     if (n % x) continue;

@@ -46,12 +46,29 @@ struct FftPlan {
   long long tw_off;   // offset of this length's twiddle table (n entries)
 };
 
-// Factorisation of one transform length for the four-step line kernels:
-// n = a * b with a, b <= 16; group = lines per warp (32 / max(a, b)).
+// Factorisation of one transform length for the shared-memory line kernels
+// (fft4.cuh): n = a * b with a, b <= 16.
 struct LinePlan {
-  int n, a, b, group;
+  int n, a, b;
+  int pfa;                 // a, b coprime: prime-factor index maps, no twiddles
+  int inv;                 // pfa: inverse of a + b modulo n
   long long tw_off;        // twiddle table exp(-2 pi i t / n), t < n
 };
+
+inline void set_line_split(LinePlan &p, int a, int b) {
+  p.a = a;
+  p.b = b;
+  int x = a, y = b;
+  while (y) {
+    const int t = x % y;
+    x = y;
+    y = t;
+  }
+  p.pfa = x == 1;
+  p.inv = 1;
+  if (p.pfa)
+    while ((long long)p.inv * (a + b) % p.n != 1 % p.n) ++p.inv;
+}
 
 // One independent Kohn-Sham system of a batch.
 struct SysDev {

@@ -1,14 +1,25 @@
-// Four-step line DFTs in shared memory, one warp per group of lines.
+// Line DFTs over shared memory: two digit steps, every lane busy.
 //
-// A line of length N = A * B is transformed as
-//   step 1: for each n2 < B:  y[n2][k1] = W_N^{n2 k1} sum_{n1} x[B n1 + n2] W_A^{n1 k1}
-//   step 2: for each k1 < A:  X[k1 + A k2] = sum_{n2} y[n2][k1] W_B^{n2 k2}
-// (Cooley-Tukey with the twiddle folded into step 1).  Step 1 writes y[n2][k1]
-// back into the slots x[B k1 + n2] it read, so it is in place per thread;
-// step 2 reads the B values y[.][k1] of one k1 and writes them to the
-// natural-order slots k1 + A k2, which only the threads of the same line
-// touch.  A warp owns G = floor(32 / max(A, B)) whole lines, so the only
-// synchronisation inside a transform is __syncwarp -- no block barrier.
+// A line of n = a b points (a, b <= 16) is an a x b array of digits.  Backward:
+// radix-a transforms over the first digit, then radix-b ones over the second;
+// forward: the same two steps in the other order.  Both work in place on the
+// slots of the line, so after the backward transform element m sits in slot
+// line_slot_of(m), and a forward transform takes it from there back to the
+// natural order: the passes multiply by V(r) or sum densities at permuted
+// slots and never move data to undo the permutation.
+//   Coprime a, b: prime-factor maps (Good-Thomas), slot (b n1 + a n2) mod n and
+//   slot(m) = (a + b) m mod n; no twiddles.
+//   Otherwise Cooley-Tukey: slot b n1 + n2, slot(m) = b (m mod a) + m div a,
+//   twiddles W_n^{n2 k1} after the first step of either direction.
+// The unit of work is one radix transform of one line, and the units of all
+// lines of a pass are dealt to the block's threads one after another (lines
+// fastest), with a block barrier per step.  GB300's FP64 pipe takes 16 clocks
+// of an SM per warp instruction however few of its lanes are active, so the
+// earlier form (a warp per group of floor(32 / max(a, b)) whole lines, 27 and
+// 24 of 32 lanes at n = 72) lost a fifth of the pipe.  With the leaner radix
+// transforms (fft_smem.cuh) and two blocks per SM the FP64 plane pass went from
+// 18.5 to 11.8 ms (72^3, 336 items; 9.9 ms of pipe time), an FP64 SCF on 44^3
+// (radix 11) from 525 to 59 ms.
 // SIGN = -1 is the forward transform (exponent -i, FFTW_FORWARD), +1 the
 // backward one; neither is normalised (Source/fft.f90:204-212).
 #pragma once
@@ -17,130 +28,204 @@
 
 namespace derek {
 
-template <typename R_, int R, int SIGN>
-__device__ __forceinline__ void dft_r(cplx<R_> *v) {
-  Dft<R_, R, SIGN>::run(v);
+// slot that holds element m after a backward transform, and the element a
+// slot holds
+__device__ __forceinline__ int line_slot_of(const LinePlan &p, int m) {
+  return p.pfa ? (m * (p.a + p.b)) % p.n : p.b * (m % p.a) + m / p.a;
+}
+__device__ __forceinline__ int line_elem_of(const LinePlan &p, int s) {
+  return p.pfa ? (s * p.inv) % p.n : s / p.b + p.a * (s % p.b);
 }
 
-// Step 1 for one (line, n2): radix-A DFT over n1, twiddle, store in place.
-template <typename R_, int SIGN, int A>
-__device__ __noinline__ void step1(cplx<R_> *line, int es, int B, int N, int n2,
-                                      const cplx<R_> *__restrict__ tw) {
-  cplx<R_> v[A];
-#pragma unroll
-  for (int n1 = 0; n1 < A; ++n1) v[n1] = line[(B * n1 + n2) * es];
-  dft_r<R_, A, SIGN>(v);
-  int idx = 0;
-#pragma unroll
-  for (int k1 = 1; k1 < A; ++k1) {
-    idx += n2;
-    if (idx >= N) idx -= N;
-    cplx<R_> w = tw[idx];
-    if (SIGN > 0) w.y = -w.y;
-    v[k1] = cmul<R_>(v[k1], w);
-  }
-#pragma unroll
-  for (int k1 = 0; k1 < A; ++k1) line[(B * k1 + n2) * es] = v[k1];
+// The steps are separate functions (one per radix), so they take offsets into
+// the block's dynamic shared memory instead of pointers: their accesses stay
+// shared-memory instructions.
+template <typename R_> __device__ __forceinline__ int smem_offset(const cplx<R_> *p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  return (int)(reinterpret_cast<const unsigned char *>(p) - smem_raw);
 }
-
-// Step 2 for one (line, k1): load B values, warp-sync, radix-B DFT, store.
-template <typename R_, int SIGN, int B>
-__device__ __noinline__ void step2(cplx<R_> *line, int es, int A, int k1, bool active) {
-  cplx<R_> v[B];
-  if (active) {
-#pragma unroll
-    for (int n2 = 0; n2 < B; ++n2) v[n2] = line[(B * k1 + n2) * es];
-  }
-  __syncwarp();
-  if (active) {
-    dft_r<R_, B, SIGN>(v);
-#pragma unroll
-    for (int k2 = 0; k2 < B; ++k2) line[(k1 + A * k2) * es] = v[k2];
-  }
+template <typename R_> __device__ __forceinline__ cplx<R_> *smem_at(int off) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  return reinterpret_cast<cplx<R_> *>(smem_raw + off);
 }
+// i / d for 0 <= i < 2^13, 1 <= d <= 128 as (i * line_magic(d)) >> 20: the
+// magic number exceeds 2^20 / d by less than 1, so the quotient is exact while
+// i d < 2^20
+__device__ __forceinline__ unsigned line_magic(int d) { return ((1u << 20) + d - 1) / d; }
 
-template <typename R_, int SIGN>
-__device__ __forceinline__ void step1_dispatch(int A, cplx<R_> *line, int es, int B, int N, int n2,
-                                               const cplx<R_> *tw) {
-  switch (A) {
-    case 1: {
-      break;
+// One digit step of a line set: units u < nu of every line, unit u's elements
+// at slots u start + k inc (mod n), k < R.  tw: twiddles W_n^{u k} after the
+// transform (offset, or -1 for none).
+template <typename R_, int SIGN, int R>
+__device__ __noinline__ void line_step(int buf_off, int nlines, int ldist, int es, const short *lines, int n, int nu,
+                                       int start, int inc, int tw_off) {
+  cplx<R_> *buf = smem_at<R_>(buf_off);
+  const int total = nlines * nu;
+  const unsigned magic = line_magic(nlines);
+  const int ne = n * es;
+  start *= es;
+  inc *= es;
+  for (int i = threadIdx.x; i < total; i += blockDim.x) {
+    const int u = (i * magic) >> 20, l = i - u * nlines;
+    cplx<R_> *line = buf + (lines ? (int)lines[l] : l) * ldist;
+    int o[R];
+    int s = u * start;
+    cplx<R_> v[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      o[k] = s;
+      v[k] = line[s];
+      s += inc;
+      if (s >= ne) s -= ne;
     }
-    case 2: step1<R_, SIGN, 2>(line, es, B, N, n2, tw); break;
-    case 3: step1<R_, SIGN, 3>(line, es, B, N, n2, tw); break;
-    case 4: step1<R_, SIGN, 4>(line, es, B, N, n2, tw); break;
-    case 5: step1<R_, SIGN, 5>(line, es, B, N, n2, tw); break;
-    case 6: step1<R_, SIGN, 6>(line, es, B, N, n2, tw); break;
-    case 7: step1<R_, SIGN, 7>(line, es, B, N, n2, tw); break;
-    case 8: step1<R_, SIGN, 8>(line, es, B, N, n2, tw); break;
-    case 9: step1<R_, SIGN, 9>(line, es, B, N, n2, tw); break;
-    case 10: step1<R_, SIGN, 10>(line, es, B, N, n2, tw); break;
-    case 11: step1<R_, SIGN, 11>(line, es, B, N, n2, tw); break;
-    case 12: step1<R_, SIGN, 12>(line, es, B, N, n2, tw); break;
-    case 13: step1<R_, SIGN, 13>(line, es, B, N, n2, tw); break;
-    case 14: step1<R_, SIGN, 14>(line, es, B, N, n2, tw); break;
-    case 15: step1<R_, SIGN, 15>(line, es, B, N, n2, tw); break;
-    case 16: step1<R_, SIGN, 16>(line, es, B, N, n2, tw); break;
-    default: break;
+    Dft<R_, R, SIGN>::run(v);
+    if (tw_off >= 0) {
+      const cplx<R_> *tw = smem_at<R_>(tw_off);
+      int idx = 0;
+#pragma unroll
+      for (int k = 1; k < R; ++k) {
+        idx += u;
+        if (idx >= n) idx -= n;
+        cplx<R_> w = tw[idx];
+        if (SIGN > 0) w.y = -w.y;
+        v[k] = cmul<R_>(v[k], w);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) line[o[k]] = v[k];
   }
 }
 
-template <typename R_, int SIGN>
-__device__ __forceinline__ void step2_dispatch(int B, cplx<R_> *line, int es, int A, int k1,
-                                               bool active) {
-  switch (B) {
-    case 1: __syncwarp(); break;
-    case 2: step2<R_, SIGN, 2>(line, es, A, k1, active); break;
-    case 3: step2<R_, SIGN, 3>(line, es, A, k1, active); break;
-    case 4: step2<R_, SIGN, 4>(line, es, A, k1, active); break;
-    case 5: step2<R_, SIGN, 5>(line, es, A, k1, active); break;
-    case 6: step2<R_, SIGN, 6>(line, es, A, k1, active); break;
-    case 7: step2<R_, SIGN, 7>(line, es, A, k1, active); break;
-    case 8: step2<R_, SIGN, 8>(line, es, A, k1, active); break;
-    case 9: step2<R_, SIGN, 9>(line, es, A, k1, active); break;
-    case 10: step2<R_, SIGN, 10>(line, es, A, k1, active); break;
-    case 11: step2<R_, SIGN, 11>(line, es, A, k1, active); break;
-    case 12: step2<R_, SIGN, 12>(line, es, A, k1, active); break;
-    case 13: step2<R_, SIGN, 13>(line, es, A, k1, active); break;
-    case 14: step2<R_, SIGN, 14>(line, es, A, k1, active); break;
-    case 15: step2<R_, SIGN, 15>(line, es, A, k1, active); break;
-    case 16: step2<R_, SIGN, 16>(line, es, A, k1, active); break;
-    default: __syncwarp(); break;
+// Last backward step, times V, first forward step, over the second digit:
+// both transforms of a unit touch the same slots, so V(r) is applied in
+// registers.  Line l's element m multiplies with v[m vstride + line_elem_of(pl, l)].
+template <typename R_, int R>
+__device__ __noinline__ void line_step_v(int buf_off, int nlines, int es, const LinePlan &p, const LinePlan &pl,
+                                         const R_ *__restrict__ v, int vstride, int tw_off) {
+  cplx<R_> *buf = smem_at<R_>(buf_off);
+  const int n = p.n, total = nlines * p.a, pfa = p.pfa;
+  const unsigned magic = line_magic(nlines);
+  const int ne = n * es;
+  const int inc = (pfa ? p.a : 1) * es;
+  const int minc = pfa ? (p.a * p.inv) % n : p.a;
+  for (int i = threadIdx.x; i < total; i += blockDim.x) {
+    const int u = (i * magic) >> 20, l = i - u * nlines;
+    cplx<R_> *line = buf + l;
+    int m = line_elem_of(p, p.b * u);
+    int s = p.b * u * es;
+    const R_ *vl = v + line_elem_of(pl, l);
+    int o[R];
+    R_ w[R];
+    cplx<R_> x[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      o[k] = s;
+      w[k] = vl[m * vstride];
+      x[k] = line[s];
+      s += inc;
+      if (s >= ne) s -= ne;
+      m += minc;
+      if (m >= n) m -= n;
+    }
+    Dft<R_, R, +1>::run(x);
+#pragma unroll
+    for (int k = 0; k < R; ++k) x[k] = cscale<R_>(x[k], w[k]);
+    Dft<R_, R, -1>::run(x);
+    if (!pfa) {
+      const cplx<R_> *tw = smem_at<R_>(tw_off);
+      int idx = 0;
+#pragma unroll
+      for (int k = 1; k < R; ++k) {
+        idx += u;
+        if (idx >= n) idx -= n;
+        x[k] = cmul<R_>(x[k], tw[idx]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) line[o[k]] = x[k];
   }
+}
+
+#define DEREK_RADIX_SWITCH(r, F) \
+  switch (r) {                   \
+    case 2: F(2); break;         \
+    case 3: F(3); break;         \
+    case 4: F(4); break;         \
+    case 5: F(5); break;         \
+    case 6: F(6); break;         \
+    case 7: F(7); break;         \
+    case 8: F(8); break;         \
+    case 9: F(9); break;         \
+    case 10: F(10); break;       \
+    case 11: F(11); break;       \
+    case 12: F(12); break;       \
+    case 13: F(13); break;       \
+    case 14: F(14); break;       \
+    case 15: F(15); break;       \
+    case 16: F(16); break;       \
+    default: break;              \
+  }
+
+// the step over the first digit (a points) or the second one (b points)
+template <typename R_, int SIGN>
+__device__ __forceinline__ void line_step_a(cplx<R_> *buf, const LinePlan &p, int nlines, int ldist, int es,
+                                            const short *lines, const cplx<R_> *tw) {
+  const int off = smem_offset<R_>(buf), tw_off = tw ? smem_offset<R_>(tw) : -1;
+#define F(r) line_step<R_, SIGN, r>(off, nlines, ldist, es, lines, p.n, p.b, p.pfa ? p.a : 1, p.b, tw_off)
+  DEREK_RADIX_SWITCH(p.a, F)
+#undef F
+}
+template <typename R_, int SIGN>
+__device__ __forceinline__ void line_step_b(cplx<R_> *buf, const LinePlan &p, int nlines, int ldist, int es,
+                                            const short *lines, const cplx<R_> *tw) {
+  const int off = smem_offset<R_>(buf), tw_off = tw ? smem_offset<R_>(tw) : -1;
+#define F(r) line_step<R_, SIGN, r>(off, nlines, ldist, es, lines, p.n, p.a, p.b, p.pfa ? p.a : 1, tw_off)
+  DEREK_RADIX_SWITCH(p.b, F)
+#undef F
 }
 
 // In-place transform of `nlines` lines held in shared memory: line l (or
-// lines[l] when a list is given) starts at buf + line * ldist, element i at
-// + i * es.  All threads of the block call it; it ends with __syncthreads().
+// lines[l] when a list is given) starts at buf + line * ldist, slot i at
+// + i * es.  Backward: natural order in, slot order out; forward: slot order
+// in, natural order out.  All threads of the block call it; it ends with
+// __syncthreads().
 template <typename R_, int SIGN>
 __device__ void fft4_lines(cplx<R_> *buf, const LinePlan &p, int nlines, int ldist, int es,
                            const short *lines, const cplx<R_> *__restrict__ tw) {
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int nwarps = blockDim.x >> 5;
-  const int A = p.a, B = p.b, N = p.n, G = p.group;
-  const int span = A > B ? A : B;          // lanes per line
-  const int g = lane / span;               // line within the warp's group
-  const int r = lane - g * span;           // lane within the line
-  for (int l0 = warp * G; l0 < nlines; l0 += nwarps * G) {
-    const int l = l0 + g;
-    const bool live = g < G && l < nlines;
-    cplx<R_> *line = buf;
-    if (live) line = buf + (long)(lines ? (int)lines[l] : l) * ldist;
-    if (live && r < B) step1_dispatch<R_, SIGN>(A, line, es, B, N, r, tw);
-    __syncwarp();
-    step2_dispatch<R_, SIGN>(B, line, es, A, r, live && r < A);
-    __syncwarp();
+  const cplx<R_> *w = p.pfa ? nullptr : tw;
+  if (SIGN > 0) {
+    line_step_a<R_, SIGN>(buf, p, nlines, ldist, es, lines, w);
+    __syncthreads();
+    line_step_b<R_, SIGN>(buf, p, nlines, ldist, es, lines, nullptr);
+  } else {
+    line_step_b<R_, SIGN>(buf, p, nlines, ldist, es, lines, w);
+    __syncthreads();
+    line_step_a<R_, SIGN>(buf, p, nlines, ldist, es, lines, nullptr);
   }
   __syncthreads();
 }
 
-}  // namespace derek
+// The backward and forward transforms of a plane's columns around V(r): column
+// l (slot l of plan pl's lines) at buf + l, slots es apart; the three steps
+// are a-radix, b-radix times V times b-radix, a-radix.
+template <typename R_>
+__device__ void fft4_columns_v(cplx<R_> *buf, const LinePlan &p, const LinePlan &pl, int ncols, int es,
+                               const R_ *__restrict__ v, int vstride, const cplx<R_> *__restrict__ tw) {
+  line_step_a<R_, +1>(buf, p, ncols, 1, es, nullptr, p.pfa ? nullptr : tw);
+  __syncthreads();
+  const int off = smem_offset<R_>(buf), tw_off = smem_offset<R_>(tw);
+#define F(r) line_step_v<R_, r>(off, ncols, es, p, pl, v, vstride, tw_off)
+  if (p.b > 1) {
+    DEREK_RADIX_SWITCH(p.b, F)
+  } else {
+    line_step_v<R_, 1>(off, ncols, es, p, pl, v, vstride, tw_off);
+  }
+#undef F
+  __syncthreads();
+  line_step_a<R_, -1>(buf, p, ncols, 1, es, nullptr, nullptr);
+  __syncthreads();
+}
 
-namespace derek {
-
-// ---- compile-time variant: n = A * B, element stride ES and line distance
-// LD known at compile time (the (y,z) planes of cubic grids).
 constexpr int plan_a(int n) {
   int best = 0, span = 1 << 30, p2 = 0;
   for (int x = 1; x <= 16; ++x) {
@@ -156,56 +241,6 @@ constexpr int plan_a(int n) {
     }
   }
   return best;
-}
-
-template <typename R_, int SIGN, int N, int ES, int LD>
-__device__ __forceinline__ void fft4_fixed(cplx<R_> *buf, int nlines, const short *lines,
-                                           const cplx<R_> *__restrict__ tw) {
-  constexpr int A = plan_a(N);
-  constexpr int B = N / A;
-  constexpr int SPAN = A > B ? A : B;
-  constexpr int G = 32 / SPAN;
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int nwarps = blockDim.x >> 5;
-  const int g = lane / SPAN;
-  const int r = lane - g * SPAN;
-  for (int l0 = warp * G; l0 < nlines; l0 += nwarps * G) {
-    const int l = l0 + g;
-    const bool live = g < G && l < nlines;
-    cplx<R_> *line = buf + (live ? (lines ? (int)lines[l] : l) * LD : 0);
-    if (live && r < B && A > 1) {
-      cplx<R_> v[A];
-#pragma unroll
-      for (int n1 = 0; n1 < A; ++n1) v[n1] = line[(B * n1 + r) * ES];
-      Dft<R_, A, SIGN>::run(v);
-#pragma unroll
-      for (int k1 = 1; k1 < A; ++k1) {
-        cplx<R_> w = tw[(r * k1) % N];
-        if (SIGN > 0) w.y = -w.y;
-        v[k1] = cmul<R_>(v[k1], w);
-      }
-#pragma unroll
-      for (int k1 = 0; k1 < A; ++k1) line[(B * k1 + r) * ES] = v[k1];
-    }
-    __syncwarp();
-    if (B > 1) {
-      cplx<R_> v[B];
-      const bool act = live && r < A;
-      if (act) {
-#pragma unroll
-        for (int n2 = 0; n2 < B; ++n2) v[n2] = line[(B * r + n2) * ES];
-      }
-      __syncwarp();
-      if (act) {
-        Dft<R_, B, SIGN>::run(v);
-#pragma unroll
-        for (int k2 = 0; k2 < B; ++k2) line[(r + A * k2) * ES] = v[k2];
-      }
-    }
-    __syncwarp();
-  }
-  __syncthreads();
 }
 
 }  // namespace derek

@@ -126,65 +126,109 @@ template <> struct RadixConst<16> {
   }
 };
 
-// In-register DFT of length R with exponent sign SIGN.  Prime lengths use the
-// direct O(R^2) sum; composite lengths R = P * Q (P the smallest prime
-// factor) split Cooley-Tukey style into P-point and Q-point DFTs with
+// In-register DFT of length R with exponent sign SIGN, written for the fewest
+// multiply-add pipe slots (an FP64 warp instruction takes 16 clocks of an SM).
+// Odd prime lengths pair x_j with x_{R-j}: (R-1)^2 fused multiply-adds instead
+// of the direct sum's 4 (R-1)^2 (7 points: 66 slots against 150).  Composite
+// lengths with coprime factors are a plain P x Q transform over prime-factor
+// index maps, without twiddles; 9 and 16 split Cooley-Tukey style with
 // compile-time twiddles; 2, 3, 4 and 8 are written out below.
 constexpr int smallest_factor(int r) {
   for (int p = 2; p * p <= r; ++p)
     if (r % p == 0) return p;
   return r;
 }
+// first factor of a composite length: a coprime split where there is one,
+// else the square root's side (9 = 3 x 3, 16 = 4 x 4)
+constexpr int dft_first_factor(int r) {
+  for (int p = 2; p * p <= r; ++p) {
+    if (r % p) continue;
+    int x = p, y = r / p;
+    while (y) {
+      const int t = x % y;
+      x = y;
+      y = t;
+    }
+    if (x == 1) return p;
+  }
+  for (int p = 2; p * p <= r; ++p)
+    if (r % p == 0 && p * p >= r) return p;
+  return smallest_factor(r);
+}
+constexpr bool dft_coprime(int p, int q) {
+  while (q) {
+    const int t = p % q;
+    p = q;
+    q = t;
+  }
+  return p == 1;
+}
 
 template <typename R_, int R, int SIGN, bool PRIME = (smallest_factor(R) == R)> struct DftGen;
 
 template <typename R_, int R, int SIGN> struct DftGen<R_, R, SIGN, true> {
   __device__ __forceinline__ static void run(cplx<R_> *v) {
-    cplx<R_> out[R];
+    constexpr int H = (R - 1) / 2;
+    cplx<R_> s[H], d[H];
+    cplx<R_> x0 = v[0];
 #pragma unroll
-    for (int k = 0; k < R; ++k) {
-      R_ ax = v[0].x, ay = v[0].y;
-#pragma unroll
-      for (int j = 1; j < R; ++j) {
-        const int m = (j * k) % R;
-        const R_ c = (R_)RadixConst<R>::c(m);
-        const R_ s = (R_)(SIGN * RadixConst<R>::s(m));
-        ax += v[j].x * c - v[j].y * s;
-        ay += v[j].x * s + v[j].y * c;
-      }
-      out[k] = mk<R_>(ax, ay);
+    for (int j = 0; j < H; ++j) {
+      s[j] = cadd<R_>(v[j + 1], v[R - 1 - j]);
+      d[j] = csub<R_>(v[j + 1], v[R - 1 - j]);
+      x0 = cadd<R_>(x0, s[j]);
     }
+    const cplx<R_> base = v[0];
+    v[0] = x0;
 #pragma unroll
-    for (int k = 0; k < R; ++k) v[k] = out[k];
+    for (int k = 1; k <= H; ++k) {
+      R_ mx = base.x, my = base.y, nx = 0, ny = 0;
+#pragma unroll
+      for (int j = 0; j < H; ++j) {
+        const int m = ((j + 1) * k) % R;
+        const R_ c = (R_)RadixConst<R>::c(m);
+        const R_ w = (R_)(SIGN * RadixConst<R>::s(m));
+        mx += s[j].x * c;
+        my += s[j].y * c;
+        nx += d[j].x * w;
+        ny += d[j].y * w;
+      }
+      // m + i n and m - i n
+      v[k] = mk<R_>(mx - ny, my + nx);
+      v[R - k] = mk<R_>(mx + ny, my - nx);
+    }
   }
 };
 
 template <typename R_, int R, int SIGN> struct Dft;
 
 template <typename R_, int R, int SIGN> struct DftGen<R_, R, SIGN, false> {
-  static constexpr int P = smallest_factor(R);
+  static constexpr int P = dft_first_factor(R);
   static constexpr int Q = R / P;
+  static constexpr bool PFA = dft_coprime(P, Q);
   __device__ __forceinline__ static void run(cplx<R_> *v) {
-    // y[n2][k1] = W_R^{n2 k1} sum_{n1} x[Q n1 + n2] W_P^{n1 k1}
+    // y[n2][k1] = W_R^{n2 k1} sum_{n1} x[Q n1 + n2] W_P^{n1 k1}; with coprime
+    // factors x[(Q n1 + P n2) mod R] and no twiddle
     cplx<R_> y[R];
 #pragma unroll
     for (int n2 = 0; n2 < Q; ++n2) {
       cplx<R_> t[P];
 #pragma unroll
-      for (int n1 = 0; n1 < P; ++n1) t[n1] = v[Q * n1 + n2];
+      for (int n1 = 0; n1 < P; ++n1) t[n1] = v[PFA ? (Q * n1 + P * n2) % R : Q * n1 + n2];
       Dft<R_, P, SIGN>::run(t);
 #pragma unroll
       for (int k1 = 0; k1 < P; ++k1) {
         const int m = (n2 * k1) % R;
-        if (m == 0) {
+        if (PFA || m == 0) {
           y[n2 * P + k1] = t[k1];
+        } else if (4 * m == R) {
+          y[n2 * P + k1] = SIGN > 0 ? mk<R_>(-t[k1].y, t[k1].x) : mk<R_>(t[k1].y, -t[k1].x);
         } else {
           const cplx<R_> w = mk<R_>((R_)RadixConst<R>::c(m), (R_)(SIGN * RadixConst<R>::s(m)));
           y[n2 * P + k1] = cmul<R_>(t[k1], w);
         }
       }
     }
-    // X[k1 + P k2] = sum_{n2} y[n2][k1] W_Q^{n2 k2}
+    // X[k1 + P k2] (coprime: X[m], m = k1 mod P and k2 mod Q) = sum_{n2} y[n2][k1] W_Q^{n2 k2}
 #pragma unroll
     for (int k1 = 0; k1 < P; ++k1) {
       cplx<R_> t[Q];
@@ -192,7 +236,14 @@ template <typename R_, int R, int SIGN> struct DftGen<R_, R, SIGN, false> {
       for (int n2 = 0; n2 < Q; ++n2) t[n2] = y[n2 * P + k1];
       Dft<R_, Q, SIGN>::run(t);
 #pragma unroll
-      for (int k2 = 0; k2 < Q; ++k2) v[k1 + P * k2] = t[k2];
+      for (int k2 = 0; k2 < Q; ++k2) {
+        int m = k1 + P * k2;
+        if (PFA) {
+          m = k1;
+          while (m % Q != k2) m += P;
+        }
+        v[m] = t[k2];
+      }
     }
   }
 };
@@ -249,21 +300,20 @@ template <typename R_, int SIGN> struct Dft<R_, 8, SIGN> {
     cplx<R_> o[4] = {v[1], v[3], v[5], v[7]};
     Dft<R_, 4, SIGN>::run(e);
     Dft<R_, 4, SIGN>::run(o);
+    // the eighth turns of o[1], o[3] are r (1 + SIGN i), r (-1 + SIGN i): r goes
+    // into the fused multiply-adds that combine them with the even half
     const R_ r = (R_)0.70710678118654752440;
-    // w8^k for k = 0..3 with exponent sign SIGN
-    cplx<R_> w1 = mk<R_>(r, (R_)SIGN * r);
-    cplx<R_> w3 = mk<R_>(-r, (R_)SIGN * r);
-    cplx<R_> o1 = cmul<R_>(o[1], w1);
-    cplx<R_> o2 = mul_si<R_, SIGN>(o[2]);
-    cplx<R_> o3 = cmul<R_>(o[3], w3);
+    const cplx<R_> o1 = SIGN > 0 ? mk<R_>(o[1].x - o[1].y, o[1].x + o[1].y) : mk<R_>(o[1].x + o[1].y, o[1].y - o[1].x);
+    const cplx<R_> o2 = mul_si<R_, SIGN>(o[2]);
+    const cplx<R_> o3 = SIGN > 0 ? mk<R_>(-o[3].x - o[3].y, o[3].x - o[3].y) : mk<R_>(o[3].y - o[3].x, -o[3].x - o[3].y);
     v[0] = cadd<R_>(e[0], o[0]);
     v[4] = csub<R_>(e[0], o[0]);
-    v[1] = cadd<R_>(e[1], o1);
-    v[5] = csub<R_>(e[1], o1);
+    v[1] = mk<R_>(e[1].x + r * o1.x, e[1].y + r * o1.y);
+    v[5] = mk<R_>(e[1].x - r * o1.x, e[1].y - r * o1.y);
     v[2] = cadd<R_>(e[2], o2);
     v[6] = csub<R_>(e[2], o2);
-    v[3] = cadd<R_>(e[3], o3);
-    v[7] = csub<R_>(e[3], o3);
+    v[3] = mk<R_>(e[3].x + r * o3.x, e[3].y + r * o3.y);
+    v[7] = mk<R_>(e[3].x - r * o3.x, e[3].y - r * o3.y);
   }
 };
 

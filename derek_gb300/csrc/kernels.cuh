@@ -56,8 +56,8 @@ template <typename R>
 void launch_x_inv(const Tables &t, int item_begin, int nitems, int max_nchunk, int max_n1,
                   int min_n1, int max_m, const cplx<R> *psi, cplx<R> *abuf, const double *occ_skip,
                   cudaStream_t st);
-// (y,z)-plane pass; a compile-time kernel is used when every system has
-// n2 = n3 = N for N in {32, 36, 48, 54, 64, 72}
+// (y,z)-plane pass; FP32 register lines when every system has n2 = n3 = N for a
+// compiled N, else shared-memory lines
 // max_m: largest |centred Miller index| (x, y or z) of a sphere entry among the items
 template <typename R>
 void launch_plane(const Tables &t, int item_begin, int nitems, int max_n1, int max_n2, int max_n3,
@@ -70,24 +70,17 @@ template <typename R>
 void launch_density_plane(const Tables &t, int ks_begin, int nks, int max_n1, int max_n2, int max_n3,
                           int min_n2, int min_n3, int max_m, const cplx<R> *abuf, const double *occ,
                           double *partial, const long long *partial_off, cudaStream_t st);
-// The x passes on shared-memory lines only (the layout k_plane and the
-// spinor passes read), never the FP32 register kernels' row layouts.
-template <typename R>
-void launch_x_inv_lines(const Tables &t, int item_begin, int nitems, int max_nchunk, int max_n1,
-                        int min_n1, const cplx<R> *psi, cplx<R> *abuf, const double *occ_skip,
-                        cudaStream_t st);
-template <typename R>
-void launch_x_fwd_lines(const Tables &t, int item_begin, int nitems, int max_nchunk, int max_n1,
-                        int min_n1, const cplx<R> *abuf, const cplx<R> *psi, const cplx<R> *prev,
-                        cplx<R> *out, const Axpby *coef, cudaStream_t st);
-
 // Non-collinear spinors (spinor.cu).  Band b of a spinor system is items 2b
 // (up) and 2b + 1 (down), so a launch covers an even number of items starting
 // on a pair.  vnc holds the 2x2 potential per grid point as four complex
 // numbers V11, V21, V12, V22 (the reference's nc_pot(n, i, j) order).
 template <typename R>
-void launch_plane_spinor(const Tables &t, int item_begin, int nitems, const int n[3], cplx<R> *abuf,
+void launch_plane_spinor(const Tables &t, int item_begin, int nitems, const int n[3], int max_m, cplx<R> *abuf,
                          const cplx<R> *vnc, cudaStream_t st);
+// register-line form for the FP32 lengths of launch_plane_reg with n2 = n3
+// (spinor_reg.cu); false for any other grid
+bool launch_plane_spinor_reg(const Tables &t, int item_begin, int nitems, const int n[3], int max_m, float2 *abuf,
+                             const float2 *vnc, cudaStream_t st);
 // Charge and magnetisation partials per k-set: four planes (n, mx, my, mz)
 // of nr values at partial + partial_off[k-set], from the x-line buffer the
 // x_inv pass filled for the items with nonzero weight.

@@ -29,7 +29,7 @@
 namespace derek {
 
 size_t spinor_plane_smem(int n2, int n3, size_t elem) {
-  return (2 * (size_t)n2 * (n3 + 1) + (size_t)n2 + n3) * elem;
+  return (2 * (size_t)n2 * (n3 | 1) + (size_t)n2 + n3) * elem;
 }
 
 template <typename R>
@@ -44,7 +44,7 @@ template <typename R>
 __device__ __forceinline__ void spinor_planes_backward(const Tables &t, const KSetDev &K, const SysDev &S,
                                                        const cplx<R> *a0, const cplx<R> *a1, cplx<R> *P0,
                                                        cplx<R> *P1, const cplx<R> *twy, const cplx<R> *twz) {
-  const int n2 = S.n[1], n3 = S.n[2], pz = n3 + 1;
+  const int n2 = S.n[1], n3 = S.n[2], pz = n3 | 1;
   for (int i = threadIdx.x; i < 2 * n2 * pz; i += blockDim.x) P0[i] = mk<R>(0, 0);
   __syncthreads();
   const short *cy = t.col_y + K.col_off;
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(512) k_plane_spinor(Tables t, int item_begin, 
   const int n1 = S.n[0], n2 = S.n[1], n3 = S.n[2];
   const int b = t.item_band[item];
   if (x >= n1 || (b & 1)) return;   // b is the up component; b + 1 < K.nb is the down one
-  const int pz = n3 + 1;
+  const int pz = n3 | 1;
   cplx<R> *P0 = reinterpret_cast<cplx<R> *>(smem_raw);
   cplx<R> *P1 = P0 + n2 * pz;
   cplx<R> *twy = P1 + n2 * pz;
@@ -90,13 +90,17 @@ __global__ void __launch_bounds__(512) k_plane_spinor(Tables t, int item_begin, 
   cplx<R> *a1 = a0 + plane;
   spinor_planes_backward<R>(t, K, S, a0, a1, P0, P1, twy, twz);
   const cplx<R> *v = vnc + 4 * (S.grid_off + (long long)x * n2 * n3);
-  for (int i = threadIdx.x; i < n2 * n3; i += blockDim.x) {
-    const int y = i / n3, z = i - y * n3;
-    const int o = y * pz + z;
-    const cplx<R> u = P0[o], d = P1[o];
-    const cplx<R> v11 = v[4 * i], v21 = v[4 * i + 1], v12 = v[4 * i + 2], v22 = v[4 * i + 3];
-    P0[o] = cadd<R>(cmul<R>(v11, u), cmul<R>(v12, d));
-    P1[o] = cadd<R>(cmul<R>(v21, u), cmul<R>(v22, d));
+  // a warp per real-space row; the backward transforms left it in slot order
+  for (int y = threadIdx.x >> 5; y < n2; y += blockDim.x >> 5) {
+    const int sy = line_slot_of(S.lp[1], y) * pz;
+    for (int z = threadIdx.x & 31; z < n3; z += 32) {
+      const int o = sy + line_slot_of(S.lp[2], z);
+      const cplx<R> *w = v + 4 * (y * n3 + z);
+      const cplx<R> u = P0[o], d = P1[o];
+      const cplx<R> v11 = w[0], v21 = w[1], v12 = w[2], v22 = w[3];
+      P0[o] = cadd<R>(cmul<R>(v11, u), cmul<R>(v12, d));
+      P1[o] = cadd<R>(cmul<R>(v21, u), cmul<R>(v22, d));
+    }
   }
   __syncthreads();
   const short *rows = t.rows + K.row_off;
@@ -130,7 +134,7 @@ __global__ void __launch_bounds__(512) k_density_spinor(Tables t, const cplx<R> 
   if (!S.active || S.nspinor != 2) return;
   const int n1 = S.n[0], n2 = S.n[1], n3 = S.n[2];
   if (x >= n1) return;
-  const int pz = n3 + 1;
+  const int pz = n3 | 1;
   cplx<R> *P0 = reinterpret_cast<cplx<R> *>(smem_raw);
   cplx<R> *P1 = P0 + n2 * pz;
   cplx<R> *twy = P1 + n2 * pz;
@@ -154,7 +158,8 @@ __global__ void __launch_bounds__(512) k_density_spinor(Tables t, const cplx<R> 
     spinor_planes_backward<R>(t, K, S, a0, a0 + plane, P0, P1, twy, twz);
     for (int i = threadIdx.x; i < n2 * n3; i += blockDim.x) {
       const int y = i / n3, z = i - y * n3;
-      const cplx<R> u = P0[y * pz + z], d = P1[y * pz + z];
+      const int o = line_slot_of(S.lp[1], y) * pz + line_slot_of(S.lp[2], z);
+      const cplx<R> u = P0[o], d = P1[o];
       const double ux = u.x, uy = u.y, dx = d.x, dy = d.y;
       const double uu = ux * ux + uy * uy, dd = dx * dx + dy * dy;
       dst[i] += w * (uu + dd);
@@ -166,9 +171,12 @@ __global__ void __launch_bounds__(512) k_density_spinor(Tables t, const cplx<R> 
 }
 
 template <typename R>
-void launch_plane_spinor(const Tables &t, int item_begin, int nitems, const int n[3], cplx<R> *abuf,
+void launch_plane_spinor(const Tables &t, int item_begin, int nitems, const int n[3], int max_m, cplx<R> *abuf,
                          const cplx<R> *vnc, cudaStream_t st) {
   if (nitems <= 1) return;
+  if constexpr (std::is_same<R, float>::value) {
+    if (launch_plane_spinor_reg(t, item_begin, nitems, n, max_m, abuf, vnc, st)) return;
+  }
   const size_t sm = spinor_plane_smem(n[1], n[2], sizeof(cplx<R>));
   cudaFuncSetAttribute(k_plane_spinor<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   derek::note_launch(), k_plane_spinor<R><<<dim3(nitems / 2, n[0]), 512, sm, st>>>(t, item_begin, abuf, vnc);
@@ -185,7 +193,7 @@ void launch_density_spinor(const Tables &t, int nks, const int max_n[3], const c
 }
 
 #define DEREK_INST(R)                                                                                  \
-  template void launch_plane_spinor<R>(const Tables &, int, int, const int *, cplx<R> *, const cplx<R> *, \
+  template void launch_plane_spinor<R>(const Tables &, int, int, const int *, int, cplx<R> *, const cplx<R> *, \
                                        cudaStream_t);                                                  \
   template void launch_density_spinor<R>(const Tables &, int, const int *, const cplx<R> *,            \
                                          const double *, double *, const long long *, cudaStream_t);

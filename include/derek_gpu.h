@@ -282,8 +282,8 @@ int derek_gpu_time_apply_h(derek_gpu_t *h, int nrep, double *ms_apply, double *m
 
 /* Autotuner.  Times the candidate plans of this handle's shapes on its own
  * tables and buffers and keeps the fastest: the radix sequence of every
- * grid-FFT length, register/fixed-length line kernels against shared-memory
- * four-step kernels with a runtime split per length, the row layout of each
+ * grid-FFT length, register-line kernels against shared-memory
+ * line kernels with a runtime split per length, the row layout of each
  * grid class's H.psi kernels, tensor or CUDA cores and the split-K length of
  * the overlaps, the rotation path and the Jacobi launch shape.  Every
  * candidate computes the same result.  With cache_path (NULL: no cache) the

@@ -31,3 +31,49 @@ def test_overlap_pairs(nb, buf, L, precision, tol):
             ref = psi.conj() @ psi.T
             assert rel_err(got, ref) < tol
             assert np.array_equal(got, got.conj().T)
+
+
+# every radix 2..16 of the shared-memory lines, coprime splits (26 = 13 x 2,
+# 77 = 11 x 7) and Cooley-Tukey ones (25, 32, 49), a prime length, a length
+# below a warp, unequal axes
+LINES = [(13, 26, 25), (32, 49, 30), (77, 12, 14), (33, 70, 39), (16, 11, 128), (52, 64, 45), (20, 60, 27)]
+
+
+@pytest.mark.parametrize("precision,tol", [(0, 1e-11), (1, 2e-5)])
+@pytest.mark.parametrize("n", LINES)
+def test_shared_memory_lines(oracle, n, precision, tol):
+    """H.psi and the density on grids that only the shared-memory lines serve."""
+    import derek_gb300 as dg
+    from test_gpu_primitives import make_pair
+    s, spec = make_pair(oracle, L=6.0, ecut=2.9, nb=3, n_fine=n, seed=n[0])
+    kb = oracle.KBasis(s, 0)
+    rng = np.random.default_rng(n[1])
+    psi = rng.standard_normal((s.nbands, kb.npw)) + 1j * rng.standard_normal((s.nbands, kb.npw))
+    v = s.vext + 0.3 * rng.standard_normal(s.nr)
+    occ = np.array([[2.0, 0.0, 0.7]])
+    with dg.Handle(spec, precision=precision) as h:
+        h.set_vloc(v)
+        h.set_wfn(psi)
+        got, rho = h.pot_apply_wfn(), h.density_calculate(occ)
+    assert rel_err(got, oracle.apply_h(s, kb, v, psi)) < tol
+    assert rel_err(rho, oracle.band_density(s, kb, psi, occ[0])) < tol
+
+
+@pytest.mark.parametrize("rows", ["tight", "compact", "all"])
+@pytest.mark.parametrize("n", [24, 27, 32, 36, 48, 54, 64, 72])
+def test_spinor_register_planes(oracle, n, rows):
+    """FP32 spinor H.psi at every length with register lines."""
+    import derek_gb300 as dg
+    from test_gpu_primitives import reg_plane_pair
+    s, spec = reg_plane_pair(oracle, n, rows, ((0.1, 0.2, -0.3),), 3, seed=n)
+    spec.nspinor = 2
+    spec.nelec = 2.0
+    kb = oracle.KBasis(s, 0)
+    rng = np.random.default_rng(n + 1)
+    psi = rng.standard_normal((2, s.nbands, kb.npw)) + 1j * rng.standard_normal((2, s.nbands, kb.npw))
+    nc = rng.standard_normal((s.nr, 2, 2)) + 1j * rng.standard_normal((s.nr, 2, 2))
+    with dg.Handle(spec, precision=1) as h:
+        h.set_nc_pot(nc)
+        h.set_wfn(psi)
+        got = h.pot_apply_wfn()
+    assert rel_err(got, oracle.apply_h_spinor(s, kb, nc, psi)) < 2e-5
