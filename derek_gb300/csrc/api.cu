@@ -26,16 +26,26 @@ int cuda_status(cudaError_t e, derek_gpu *h, const char *what) {
   return e == cudaErrorMemoryAllocation ? DEREK_ERR_OOM : DEREK_ERR_CUDA;
 }
 
-__global__ void k_reduce_partials(const SysDev *__restrict__ sys, const KSetDev *__restrict__ ks,
-                                  int s, const double *__restrict__ partial,
-                                  const long long *__restrict__ poff, double *__restrict__ rho) {
-  const SysDev &S = sys[s];
-  if (!S.active) return;
+// Sum of a system's partial grids (blockIdx.y: system, blockIdx.z: component of
+// a spinor density, n, mx, my, mz), units in order.
+__global__ void __launch_bounds__(256) k_reduce_partials(const SysDev *__restrict__ sys,
+                                                         const double *__restrict__ partial,
+                                                         const long long *__restrict__ sys_part,
+                                                         const int *__restrict__ sys_units,
+                                                         double *__restrict__ rho, double *__restrict__ mag,
+                                                         long long mag_stride) {
+  const SysDev &S = sys[blockIdx.y];
+  const int c = blockIdx.z, nc = S.nspinor == 2 ? 4 : 1;
+  if (!S.active || c >= nc || (gridDim.z == 4 && nc == 1)) return;
+  const double *src = partial + sys_part[blockIdx.y] + (long long)c * S.nr;
+  double *dst = (c == 0 ? rho : mag + (c - 1) * mag_stride) + S.grid_off;
+  const int nu = sys_units[blockIdx.y];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < S.nr;
        i += (long long)gridDim.x * blockDim.x) {
     double acc = 0.0;
-    for (int k = 0; k < S.nk; ++k) acc += partial[poff[S.ks0 + k] + i];
-    rho[S.grid_off + i] = acc;
+#pragma unroll 4
+    for (int u = 0; u < nu; ++u) acc += src[(long long)u * nc * S.nr + i];
+    dst[i] = acc;
   }
 }
 
@@ -151,10 +161,16 @@ template <typename R> static void density_t(derek_gpu *h, const void *psi) {
     t.item_list = c.launch_list();
     launch_x_inv<R>(t, 0, c.launch_count(), c.nchunk, c.n[0], disp_min(h, c.n[0]), c.disp_m,
                     (const cplx<R> *)psi, (cplx<R> *)h->d_abuf, h->d_occw, h->stream);
+    launch_density_plane<R>(h->tab, c.d_units, c.nunits, c.n, disp_min(h, c.n[1]), c.disp_m,
+                            (const cplx<R> *)h->d_abuf, h->d_occw, h->d_partial, h->stream);
   }
-  launch_density_plane<R>(h->tab, 0, h->nks, h->max_n[0], h->max_n[1], h->max_n[2], disp_min(h, h->min_n[1]),
-                          disp_min(h, h->min_n[2]), h->max_m_all, (const cplx<R> *)h->d_abuf, h->d_occw,
-                          h->d_partial, h->d_partial_off, h->stream);
+}
+
+// partial grids of every active system into rho (and h->d_mag)
+static void reduce_partials(derek_gpu *h, double *rho, int components) {
+  const int gx = (int)std::min<long long>((h->max_nr + 255) / 256, 152 * 4);
+  derek::note_launch(), k_reduce_partials<<<dim3(gx, h->nsys, components), 256, 0, h->stream>>>(
+      h->d_sys, h->d_partial, h->d_sys_part, h->d_sys_units, rho, h->d_mag, h->total_grid);
 }
 
 int density_items(derek_gpu *h, const void *psi, double *rho) {
@@ -162,9 +178,7 @@ int density_items(derek_gpu *h, const void *psi, double *rho) {
     density_t<double>(h, psi);
   else
     density_t<float>(h, psi);
-  for (int s = 0; s < h->nsys; ++s)
-    derek::note_launch(), k_reduce_partials<<<152, 256, 0, h->stream>>>(h->d_sys, h->d_ks, s, h->d_partial,
-                                                  h->d_partial_off, rho);
+  reduce_partials(h, rho, 1);
   DEREK_CUDA(h, cudaGetLastError());
   return DEREK_OK;
 }
@@ -221,9 +235,9 @@ template <typename R> static void density_spinor_t(derek_gpu *h, const void *psi
     t.item_list = c.d_list;
     launch_x_inv<R>(t, 0, c.count, c.nchunk, c.n[0], c.n[0], c.max_m, (const cplx<R> *)psi,
                     (cplx<R> *)h->d_abuf, h->d_occw, h->stream);
+    launch_density_spinor<R>(h->tab, c.d_units, c.nunits, c.n, (const cplx<R> *)h->d_abuf, h->d_occw,
+                             h->d_partial, h->stream);
   }
-  launch_density_spinor<R>(h->tab, h->nks, h->max_n, (const cplx<R> *)h->d_abuf, h->d_occw,
-                           h->d_partial, h->d_partial_off, h->stream);
 }
 
 int density_spinor_items(derek_gpu *h, const void *psi, double *rho) {
@@ -231,15 +245,7 @@ int density_spinor_items(derek_gpu *h, const void *psi, double *rho) {
     density_spinor_t<double>(h, psi);
   else
     density_spinor_t<float>(h, psi);
-  for (int s = 0; s < h->nsys; ++s) {
-    const SysDev &S = h->sys[s];
-    if (S.nspinor != 2) continue;
-    for (int c = 0; c < 4; ++c)
-      derek::note_launch(),
-          k_reduce_partials<<<152, 256, 0, h->stream>>>(h->d_sys, h->d_ks, s, h->d_partial + c * (long long)S.nr,
-                                                       h->d_partial_off,
-                                                       c == 0 ? rho : h->d_mag + (c - 1) * h->total_grid);
-  }
+  reduce_partials(h, rho, 4);
   DEREK_CUDA(h, cudaGetLastError());
   return DEREK_OK;
 }
@@ -260,6 +266,10 @@ int refresh_vloc32(derek_gpu *h) {
 }  // namespace derek
 
 using namespace derek;
+
+// (k-set, x-plane) pairs below which the density pass splits bands: three
+// blocks per SM
+constexpr long long kDensityPlanes = 3 * 152;
 
 static thread_local std::string g_create_error;
 
@@ -320,7 +330,7 @@ int derek_gpu_destroy(derek_gpu_t *h) {
                   h->d_col_start, h->d_ent_ix, h->d_col_y, h->d_col_z, h->d_col_x0, h->d_rows, h->d_pw_entry, h->d_kin64,     h->d_kin32,
                   h->d_tw64,  h->d_tw32,    h->d_vext,    h->d_vloc,      h->d_vhxc,
                   h->d_vloc32, h->d_rho_in, h->d_rho_out, h->d_exc,       h->d_vxc,
-                  h->d_cgrid, h->d_partial, h->d_partial_off, h->d_X,     h->d_Y,
+                  h->d_cgrid, h->d_partial, h->d_sys_part, h->d_sys_units, h->d_X,     h->d_Y,
                   h->d_Yp,    h->d_HX,      h->d_abuf,    h->d_occw,      h->d_eig,
                   h->d_occ,   h->d_coef,    h->d_cells,   h->d_wells,     h->d_well_off,
                   h->d_hfpart, h->d_hfgrad, h->d_vnc64, h->d_vnc32, h->d_mag, h->d_ks_band,
@@ -329,6 +339,7 @@ int derek_gpu_destroy(derek_gpu_t *h) {
     if (p) cudaFree(p);
   for (auto &c : h->classes) {
     if (c.d_list) cudaFree(c.d_list);
+    if (c.d_units) cudaFree(c.d_units);
     if (c.d_active) cudaFree(c.d_active);
   }
   derek_scf_free(h);
@@ -373,10 +384,8 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
   std::vector<float> kin32;
   std::vector<double> tw64;
   std::map<int, long long> tw_of;  // n -> offset
-  std::vector<long long> partial_off;
 
-  long long grid_off = 0, psi_off = 0, ent_off = 0, col_off = 0, row_off = 0, a_off = 0,
-            part_off = 0;
+  long long grid_off = 0, psi_off = 0, ent_off = 0, col_off = 0, row_off = 0, a_off = 0;
   for (int s = 0; s < nsys; ++s) {
     const derek_sys_desc &d = desc[s];
     if (d.nspinor != 1 && d.nspinor != 2) FAIL(DEREK_ERR_UNSUPPORTED, "nspinor must be 1 or 2");
@@ -416,8 +425,6 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
     for (int i = 0; i < 3; ++i) {
       S.n[i] = nfine[i];
       h->n_std.push_back(nstd[i]);
-      h->max_n[i] = std::max(h->max_n[i], nfine[i]);
-      h->min_n[i] = s == 0 ? nfine[i] : std::min(h->min_n[i], nfine[i]);
       h->max_nmax = std::max(h->max_nmax, nfine[i]);
       FftPlan &p = S.plan[i];
       p.n = nfine[i];
@@ -467,6 +474,7 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
       v.assign(d.vext, d.vext + S.nr);
     else
       build_vext(d.cell, nfine, d.nelec, d.nwells, d.wells, v);
+    h->max_nr = std::max<long long>(h->max_nr, S.nr);
     h->well_off.push_back((int)(h->wells_host.size() / 5));
     if (d.nwells > 0 && d.wells) h->wells_host.insert(h->wells_host.end(), d.wells, d.wells + 5 * d.nwells);
     h->wells_define_vext.push_back(d.vext == nullptr);
@@ -533,7 +541,6 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
       col_x0.push_back(0);
       K.nrow = (int)krows.size();
       h->ks_max_m.push_back(max_m);
-      h->max_m_all = std::max(h->max_m_all, max_m);
       rows.insert(rows.end(), krows.begin(), krows.end());
       for (int i = 0; i < npw; ++i) {
         const int ix = ((sp.mx[i] % nfine[0]) + nfine[0]) % nfine[0];
@@ -549,8 +556,6 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
       row_off += K.nrow;
       psi_off += (long long)nbi * K.npw_pad;
       a_off += (long long)nbi * nfine[0] * K.ncol_pad;
-      partial_off.push_back(part_off);
-      part_off += (d.nspinor == 2 ? 4 : 1) * (long long)S.nr;
       {
         // plane-wave start vectors: the nbi lowest kinetic energies of the
         // k-point (ties by entry index), entries in column order
@@ -622,7 +627,6 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
     CK(cudaMalloc((void **)&h->d_hfpart, (size_t)nsys * 64 * std::max(h->max_wells, 1) * 5 * sizeof(double)));
     CK(cudaMalloc((void **)&h->d_hfgrad, std::max<size_t>(h->wells_host.size(), 1) * sizeof(double)));
   }
-  CK(upload(&h->d_partial_off, partial_off));
   const size_t gbytes = (size_t)grid_off * sizeof(double);
   CK(cudaMalloc((void **)&h->d_vloc, gbytes));
   CK(cudaMemcpy(h->d_vloc, h->d_vext, gbytes, cudaMemcpyDeviceToDevice));
@@ -634,7 +638,6 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
   CK(cudaMalloc((void **)&h->d_exc, gbytes));
   CK(cudaMalloc((void **)&h->d_vxc, gbytes));
   CK(cudaMalloc((void **)&h->d_cgrid, (size_t)grid_off * sizeof(double2)));
-  CK(cudaMalloc((void **)&h->d_partial, (size_t)std::max<long long>(part_off, 1) * sizeof(double)));
   if (h->any_spinor) {
     // nc_pot starts as V_ext on the diagonal (Source/pot.f90:133-166)
     std::vector<double2> vnc((size_t)4 * grid_off, make_double2(0.0, 0.0));
@@ -715,6 +718,36 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
       CK(cudaMalloc((void **)&c.d_active, std::max<size_t>(c.items.size(), 1) * sizeof(int)));
       h->classes.push_back(c);
     }
+    // density units: a k-set's bands in ng interleaved groups where the batch's
+    // (k-set, x-plane) pairs alone would leave SMs without a block, at most one
+    // group per occupied band and 8 in all (a group costs a partial grid)
+    long long planes = 0;
+    for (const auto &K : h->ks) planes += h->sys[K.sys].n[0];
+    std::vector<long long> sys_part(nsys);
+    std::vector<int> sys_units(nsys, 0);
+    std::map<std::array<int, 3>, std::vector<DensityUnit>> units;
+    long long part_off = 0;
+    for (int q = 0; q < h->nks; ++q) {
+      const KSetDev &K = h->ks[q];
+      const SysDev &S = h->sys[K.sys];
+      const int nocc = (int)std::ceil(S.nelec * S.nspinor / 2.0);
+      int ng = (int)std::min<long long>(8, kDensityPlanes / std::max<long long>(planes, 1));
+      ng = std::max(1, std::min(ng, nocc));
+      if (K.kidx == 0) sys_part[K.sys] = part_off;
+      for (int g = 0; g < ng; ++g) {
+        units[{S.n[0], S.n[1], S.n[2]}].push_back(DensityUnit{q, g, ng, part_off});
+        part_off += (S.nspinor == 2 ? 4 : 1) * (long long)S.nr;
+        ++sys_units[K.sys];
+      }
+    }
+    for (auto &c : h->classes) {
+      const auto &u = units[{c.n[0], c.n[1], c.n[2]}];
+      c.nunits = (int)u.size();
+      CK(upload(&c.d_units, u));
+    }
+    CK(upload(&h->d_sys_part, sys_part));
+    CK(upload(&h->d_sys_units, sys_units));
+    CK(cudaMalloc((void **)&h->d_partial, (size_t)std::max<long long>(part_off, 1) * sizeof(double)));
   }
   if (refresh_vloc32(h) != DEREK_OK) FAIL(DEREK_ERR_CUDA, h->last_error);
   int st = derek_scf_alloc(h);

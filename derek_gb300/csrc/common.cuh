@@ -113,6 +113,13 @@ struct KSetDev {
   double kfrac[3];
 };
 
+// One unit of the density pass: bands g, g + ng, ... of a k-set, summed into a
+// partial grid of its own (spinor systems: four grids n, mx, my, mz).
+struct DensityUnit {
+  int ks, g, ng;
+  long long off;           // element offset of the partial grid
+};
+
 // Host-side count of kernel launches issued by the library (every launch
 // site calls note_launch; a CUDA graph replay adds its captured kernel count).
 void note_launch(long long n = 1);

@@ -15,8 +15,6 @@ struct derek_gpu {
   int nsys = 0;
   int nks = 0;
   int nitems = 0;
-  int max_n[3] = {0, 0, 0};
-  int min_n[3] = {0, 0, 0};
   int max_nmax = 0;        // max over all axes and systems
   int max_nchunk = 0;      // column chunks of the largest sphere
   int max_nb = 0;
@@ -75,8 +73,9 @@ struct derek_gpu {
   std::vector<std::vector<double>> start_rho;   // per system: SCF start density (empty = uniform)
   double *d_exc = nullptr, *d_vxc = nullptr;
   double2 *d_cgrid = nullptr;      // complex work grid
-  double *d_partial = nullptr;     // per-k-set density partials
-  long long *d_partial_off = nullptr;
+  double *d_partial = nullptr;     // density partials, one grid (spinor: four) per unit
+  long long *d_sys_part = nullptr; // per system: offset of its first unit's partial grid
+  int *d_sys_units = nullptr;      // per system: units
 
   // ---- device psi-shaped buffers (element type by precision)
   void *d_X = nullptr, *d_Y = nullptr, *d_Yp = nullptr, *d_HX = nullptr;
@@ -123,6 +122,8 @@ struct derek_gpu {
     int nchunk;
     int max_m;     // largest |centred Miller index| (x, y or z) of a sphere entry in the class
     int disp_m;    // row bound the stage kernels are dispatched with (>= max_m; autotuned)
+    derek::DensityUnit *d_units;   // the class's density units
+    int nunits;
     int *d_list;   // nullptr when the class is the contiguous range of all items
     // the class's items of the still-active systems, used by the SCF's H.psi
     // and density passes once many systems have converged (active_count < 0:
@@ -135,7 +136,6 @@ struct derek_gpu {
   };
   std::vector<ItemClass> classes;
   std::vector<int> ks_max_m;    // per k-set: largest |centred Miller index| of its sphere
-  int max_m_all = 0;
 
   // ---- plan choices the autotuner (autotune.cu) may change; the defaults
   // are the untuned plan

@@ -176,20 +176,20 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_x_fwd(Tables t, int item_be
   }
 }
 
-// ---- density: per (k-set, x-plane), loop over bands ------------------------
+// ---- density: per (unit, x-plane), loop over the unit's bands ------------------------
 // FP64 accumulators of one plane, rounded up to an even count so that the
 // complex planes after them start on a 16-byte boundary (a double2 needs it)
 __host__ __device__ constexpr int density_acc_count(int points) { return (points + 1) & ~1; }
 
 template <typename R>
-__global__ void __launch_bounds__(kLineThreads, 2) k_density_plane(Tables t, int ks_begin, const cplx<R> *__restrict__ abuf,
+__global__ void __launch_bounds__(kLineThreads, 2) k_density_plane(Tables t, const DensityUnit *__restrict__ units,
+                                                       const cplx<R> *__restrict__ abuf,
                                                        const double *__restrict__ occ,
-                                                       double *__restrict__ partial,
-                                                       const long long *__restrict__ partial_off) {
+                                                       double *__restrict__ partial) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int ksi = ks_begin + blockIdx.x;
+  const DensityUnit U = units[blockIdx.x];
   const int x = blockIdx.y;
-  const KSetDev &K = t.ks[ksi];
+  const KSetDev &K = t.ks[U.ks];
   const SysDev &S = t.sys[K.sys];
   if (!S.active) return;
   const int n1 = S.n[0], n2 = S.n[1], n3 = S.n[2];
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_density_plane(Tables t, int
   const short *cy = t.col_y + K.col_off;
   const short *cz = t.col_z + K.col_off;
   const short *rows = t.rows + K.row_off;
-  for (int b = 0; b < K.nb; ++b) {
+  for (int b = U.g; b < K.nb; b += U.ng) {
     const double w = occ[K.item0 + b];
     if (w == 0.0) continue;
     __syncthreads();
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_density_plane(Tables t, int
     }
   }
   __syncthreads();
-  double *dst = partial + partial_off[ksi] + (long long)x * n2 * n3;
+  double *dst = partial + U.off + (long long)x * n2 * n3;
   // the sums sit in slot order
   for (int y = threadIdx.x >> 5; y < n2; y += blockDim.x >> 5) {
     const int sy = line_slot_of(S.lp[1], y) * n3;
@@ -287,18 +287,16 @@ void launch_plane(const Tables &t, int item_begin, int nitems, int max_n1, int m
 
 
 template <typename R>
-void launch_density_plane(const Tables &t, int ks_begin, int nks, int max_n1, int max_n2, int max_n3,
-                          int min_n2, int min_n3, int max_m, const cplx<R> *abuf, const double *occ,
-                          double *partial, const long long *partial_off, cudaStream_t st) {
-  if (nks <= 0) return;
+void launch_density_plane(const Tables &t, const DensityUnit *units, int nunits, const int n[3], int min_n2,
+                          int max_m, const cplx<R> *abuf, const double *occ, double *partial, cudaStream_t st) {
+  if (nunits <= 0) return;
   if constexpr (std::is_same<R, float>::value) {
-    if (max_n2 == max_n3 && min_n2 == max_n2 && min_n3 == max_n3 &&
-        launch_density_reg(t, ks_begin, nks, max_n1, max_n2, max_m, abuf, occ, partial, partial_off, st))
+    if (n[1] == n[2] && min_n2 == n[1] && launch_density_reg(t, units, nunits, n[0], n[1], max_m, abuf, occ, partial, st))
       return;
   }
-  const size_t sm = (size_t)density_acc_count(max_n2 * max_n3) * sizeof(double) + smem_plane<R>(max_n2, max_n3);
+  const size_t sm = (size_t)density_acc_count(n[1] * n[2]) * sizeof(double) + smem_plane<R>(n[1], n[2]);
   cudaFuncSetAttribute(k_density_plane<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::note_launch(), k_density_plane<R><<<dim3(nks, max_n1), kLineThreads, sm, st>>>(t, ks_begin, abuf, occ, partial, partial_off);
+  derek::note_launch(), k_density_plane<R><<<dim3(nunits, n[0]), kLineThreads, sm, st>>>(t, units, abuf, occ, partial);
 }
 
 #define DEREK_INST(R)                                                                             \
@@ -309,9 +307,8 @@ void launch_density_plane(const Tables &t, int ks_begin, int nks, int max_n1, in
   template void launch_x_fwd<R>(const Tables &, int, int, int, int, int, int, const cplx<R> *,   \
                                 const cplx<R> *, const cplx<R> *, cplx<R> *, const Axpby *,      \
                                 cudaStream_t);                                                    \
-  template void launch_density_plane<R>(const Tables &, int, int, int, int, int, int, int, int,   \
-                                        const cplx<R> *, const double *, double *,                \
-                                        const long long *, cudaStream_t);
+  template void launch_density_plane<R>(const Tables &, const DensityUnit *, int, const int *, int, int, \
+                                        const cplx<R> *, const double *, double *, cudaStream_t);
 DEREK_INST(float)
 DEREK_INST(double)
 #undef DEREK_INST

@@ -67,9 +67,8 @@ void launch_x_fwd(const Tables &t, int item_begin, int nitems, int max_nchunk, i
                   int min_n1, int max_m, const cplx<R> *abuf, const cplx<R> *psi, const cplx<R> *prev,
                   cplx<R> *out, const Axpby *coef, cudaStream_t st);
 template <typename R>
-void launch_density_plane(const Tables &t, int ks_begin, int nks, int max_n1, int max_n2, int max_n3,
-                          int min_n2, int min_n3, int max_m, const cplx<R> *abuf, const double *occ,
-                          double *partial, const long long *partial_off, cudaStream_t st);
+void launch_density_plane(const Tables &t, const DensityUnit *units, int nunits, const int n[3], int min_n2,
+                          int max_m, const cplx<R> *abuf, const double *occ, double *partial, cudaStream_t st);
 // Non-collinear spinors (spinor.cu).  Band b of a spinor system is items 2b
 // (up) and 2b + 1 (down), so a launch covers an even number of items starting
 // on a pair.  vnc holds the 2x2 potential per grid point as four complex
@@ -81,13 +80,12 @@ void launch_plane_spinor(const Tables &t, int item_begin, int nitems, const int 
 // (spinor_reg.cu); false for any other grid
 bool launch_plane_spinor_reg(const Tables &t, int item_begin, int nitems, const int n[3], int max_m, float2 *abuf,
                              const float2 *vnc, cudaStream_t st);
-// Charge and magnetisation partials per k-set: four planes (n, mx, my, mz)
-// of nr values at partial + partial_off[k-set], from the x-line buffer the
+// Charge and magnetisation partials per unit: four planes (n, mx, my, mz)
+// of nr values at partial + its offset, from the x-line buffer the
 // x_inv pass filled for the items with nonzero weight.
 template <typename R>
-void launch_density_spinor(const Tables &t, int nks, const int max_n[3], const cplx<R> *abuf,
-                           const double *occ, double *partial, const long long *partial_off,
-                           cudaStream_t st);
+void launch_density_spinor(const Tables &t, const DensityUnit *units, int nunits, const int n[3],
+                           const cplx<R> *abuf, const double *occ, double *partial, cudaStream_t st);
 size_t spinor_plane_smem(int n2, int n3, size_t elem);
 
 constexpr int kColChunk = 64;   // columns per x-line chunk (kCC in hpsi4.cu)
@@ -102,9 +100,8 @@ bool launch_xinv_reg(const Tables &t, int item_begin, int nitems, int max_ncol, 
 bool launch_xfwd_reg(const Tables &t, int item_begin, int nitems, int max_ncol, int n, int max_m,
                      const float2 *abuf, const float2 *psi, const float2 *prev, float2 *out,
                      const Axpby *coef, cudaStream_t st);
-bool launch_density_reg(const Tables &t, int ks_begin, int nks, int max_n1, int n, int max_m,
-                        const float2 *abuf, const double *occ, double *partial,
-                        const long long *partial_off, cudaStream_t st);
+bool launch_density_reg(const Tables &t, const DensityUnit *units, int nunits, int n1, int n, int max_m,
+                        const float2 *abuf, const double *occ, double *partial, cudaStream_t st);
 
 // ---- full-grid FFT (grid.cu) -----------------------------------------------
 // In-place unnormalised 3D FFT of one complex FP64 grid per system in

@@ -117,19 +117,19 @@ __global__ void __launch_bounds__(512) k_plane_spinor(Tables t, int item_begin, 
   }
 }
 
-// Density pass per (k-set, x-plane): n, mx, my, mz of the k-set's bands
+// Density pass per (unit, x-plane): n, mx, my, mz of the unit's bands
 // with per-item weights occ (equal on both items of a band), written as four
-// planes of nr values at partial + partial_off[k-set].  Each thread owns the
+// planes of nr values at the unit's partial grids.  Each thread owns the
 // same grid points in every band, so the sums need no synchronisation.
 template <typename R>
-__global__ void __launch_bounds__(512) k_density_spinor(Tables t, const cplx<R> *__restrict__ abuf,
+__global__ void __launch_bounds__(512) k_density_spinor(Tables t, const DensityUnit *__restrict__ units,
+                                                        const cplx<R> *__restrict__ abuf,
                                                         const double *__restrict__ occ,
-                                                        double *__restrict__ partial,
-                                                        const long long *__restrict__ partial_off) {
+                                                        double *__restrict__ partial) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int ksi = blockIdx.x;
+  const DensityUnit U = units[blockIdx.x];
   const int x = blockIdx.y;
-  const KSetDev &K = t.ks[ksi];
+  const KSetDev &K = t.ks[U.ks];
   const SysDev &S = t.sys[K.sys];
   if (!S.active || S.nspinor != 2) return;
   const int n1 = S.n[0], n2 = S.n[1], n3 = S.n[2];
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(512) k_density_spinor(Tables t, const cplx<R> 
   load_lines_tw<R>(twy, twtab<R>(t) + S.lp[1].tw_off, n2);
   load_lines_tw<R>(twz, twtab<R>(t) + S.lp[2].tw_off, n3);
   const long long nr = S.nr;
-  double *dst = partial + partial_off[ksi] + (long long)x * n2 * n3;
+  double *dst = partial + U.off + (long long)x * n2 * n3;
   for (int i = threadIdx.x; i < n2 * n3; i += blockDim.x) {
     dst[i] = 0.0;
     dst[nr + i] = 0.0;
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(512) k_density_spinor(Tables t, const cplx<R> 
     dst[3 * nr + i] = 0.0;
   }
   const long long plane = (long long)n1 * K.ncol_pad;
-  for (int b = 0; b + 1 < K.nb; b += 2) {
+  for (int b = 2 * U.g; b + 1 < K.nb; b += 2 * U.ng) {
     const double w = occ[K.item0 + b];
     if (w == 0.0) continue;
     __syncthreads();   // the previous band's planes are read to the end
@@ -183,20 +183,19 @@ void launch_plane_spinor(const Tables &t, int item_begin, int nitems, const int 
 }
 
 template <typename R>
-void launch_density_spinor(const Tables &t, int nks, const int max_n[3], const cplx<R> *abuf,
-                           const double *occ, double *partial, const long long *partial_off,
-                           cudaStream_t st) {
-  if (nks <= 0) return;
-  const size_t sm = spinor_plane_smem(max_n[1], max_n[2], sizeof(cplx<R>));
+void launch_density_spinor(const Tables &t, const DensityUnit *units, int nunits, const int n[3],
+                           const cplx<R> *abuf, const double *occ, double *partial, cudaStream_t st) {
+  if (nunits <= 0) return;
+  const size_t sm = spinor_plane_smem(n[1], n[2], sizeof(cplx<R>));
   cudaFuncSetAttribute(k_density_spinor<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::note_launch(), k_density_spinor<R><<<dim3(nks, max_n[0]), 512, sm, st>>>(t, abuf, occ, partial, partial_off);
+  derek::note_launch(), k_density_spinor<R><<<dim3(nunits, n[0]), 512, sm, st>>>(t, units, abuf, occ, partial);
 }
 
 #define DEREK_INST(R)                                                                                  \
   template void launch_plane_spinor<R>(const Tables &, int, int, const int *, int, cplx<R> *, const cplx<R> *, \
                                        cudaStream_t);                                                  \
-  template void launch_density_spinor<R>(const Tables &, int, const int *, const cplx<R> *,            \
-                                         const double *, double *, const long long *, cudaStream_t);
+  template void launch_density_spinor<R>(const Tables &, const DensityUnit *, int, const int *,        \
+                                         const cplx<R> *, const double *, double *, cudaStream_t);
 DEREK_INST(float)
 DEREK_INST(double)
 #undef DEREK_INST
