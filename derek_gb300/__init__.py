@@ -209,14 +209,14 @@ class Handle:
         return shape if s.nspinor == 1 else (2,) + shape
 
     def get_wfn(self, sys=0, k=0):
-        psi = np.zeros(self._wfn_shape(sys, k), dtype=np.complex128)
+        psi = np.empty(self._wfn_shape(sys, k), dtype=np.complex128)
         _check(lib.derek_gpu_get_wfn(self._h, sys, k, psi.ctypes.data_as(ctypes.POINTER(ctypes.c_double))),
                self._h, "get_wfn")
         return psi
 
     def pot_apply_wfn(self, sys=0, k=0):
         """H psi of the stored wavefunctions (pot_apply_wfn + kinetic)."""
-        out = np.zeros(self._wfn_shape(sys, k), dtype=np.complex128)
+        out = np.empty(self._wfn_shape(sys, k), dtype=np.complex128)
         _check(lib.derek_gpu_apply_h(self._h, sys, k, out.ctypes.data_as(ctypes.POINTER(ctypes.c_double))),
                self._h, "apply_h")
         return out
@@ -226,7 +226,7 @@ class Handle:
         s = self.systems[sys]
         occ = np.ascontiguousarray(np.asarray(occ, dtype=np.float64).reshape(len(s.kpts), s.nbands))
         nf, _ = self.grid(sys)
-        rho = np.zeros(int(np.prod(nf)))
+        rho = np.empty(int(np.prod(nf)))
         _check(lib.derek_gpu_density(self._h, sys, _dptr(occ), _dptr(rho)), self._h, "density")
         return rho
 
@@ -391,7 +391,7 @@ class Handle:
 
     def density(self, sys=0):
         nf, _ = self.grid(sys)
-        rho = np.zeros(int(np.prod(nf)))
+        rho = np.empty(int(np.prod(nf)))
         _check(lib.derek_gpu_get_density(self._h, sys, _dptr(rho)), self._h, "density")
         return rho
 

@@ -327,7 +327,7 @@ const char *derek_gpu_last_error(derek_gpu_t *h) {
 int derek_gpu_destroy(derek_gpu_t *h) {
   if (!h) return DEREK_ERR_BAD_ARG;
   void *ptrs[] = {h->d_sys,   h->d_ks,      h->d_item_ks, h->d_item_band, h->d_ent_col,
-                  h->d_col_start, h->d_ent_ix, h->d_col_y, h->d_col_z, h->d_col_x0, h->d_rows, h->d_pw_entry, h->d_kin64,     h->d_kin32,
+                  h->d_col_start, h->d_ent_ix, h->d_col_y, h->d_col_z, h->d_col_x0, h->d_rows, h->d_pw_entry, h->d_kin64,     h->d_kin32,    h->d_perm,
                   h->d_tw64,  h->d_tw32,    h->d_vext,    h->d_vloc,      h->d_vhxc,
                   h->d_vloc32, h->d_rho_in, h->d_rho_out, h->d_exc,       h->d_vxc,
                   h->d_cgrid, h->d_partial, h->d_sys_part, h->d_sys_units, h->d_X,     h->d_Y,
@@ -378,7 +378,7 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
   if (h->prec != DEREK_PREC_FP64 && h->prec != DEREK_PREC_MIXED) FAIL(DEREK_ERR_BAD_ARG, "precision");
   h->nsys = nsys;
 
-  std::vector<int> ent_col, col_start;
+  std::vector<int> ent_col, col_start, perm;
   std::vector<short> ent_ix, col_y, col_z, col_x0, rows;
   std::vector<int> pw_entry;
   std::vector<float> kin32;
@@ -522,7 +522,7 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
           const int ix = ((sp.mx[ref] % nfine[0]) + nfine[0]) % nfine[0];
           ent_col.push_back(c);
           ent_ix.push_back((short)ix);
-          h->perm.push_back(ref);
+          perm.push_back(ref);
           h->kin_col.push_back(sp.kinetic[ref]);
           kin32.push_back((float)sp.kinetic[ref]);
           ++e;
@@ -606,6 +606,7 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
   CK(upload(&h->d_rows, rows));
   CK(upload(&h->d_pw_entry, pw_entry));
   CK(upload(&h->d_kin64, h->kin_col));
+  CK(upload(&h->d_perm, perm));
   CK(upload(&h->d_kin32, kin32));
   {
     std::vector<double2> t(tw64.size() / 2);
@@ -666,7 +667,10 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
   CK(cudaMemset(h->d_Y, 0, pbytes));
   CK(cudaMemset(h->d_Yp, 0, pbytes));
   CK(cudaMemset(h->d_HX, 0, pbytes));
-  CK(cudaMalloc(&h->d_abuf, (size_t)std::max<long long>(h->total_abuf, 1) * h->elem_size()));
+  // at least one row of a k-set in the caller's precision (copy_slice)
+  h->abuf_bytes = (size_t)std::max<long long>(h->total_abuf, 1) * h->elem_size();
+  for (const auto &K : h->ks) h->abuf_bytes = std::max(h->abuf_bytes, (size_t)K.npw * sizeof(double2));
+  CK(cudaMalloc(&h->d_abuf, h->abuf_bytes));
   CK(cudaMalloc((void **)&h->d_occw, (size_t)h->nitems * sizeof(double)));
   CK(cudaMalloc((void **)&h->d_eig, (size_t)h->nitems * sizeof(double)));
   CK(cudaMalloc((void **)&h->d_occ, (size_t)h->nitems * sizeof(double)));
@@ -913,47 +917,29 @@ int derek_gpu_get_vloc(derek_gpu_t *h, int s, double *v) {
 // copy between a host complex128 [nspinor][nbr][npw] slice in the
 // reference's G order (coeff(gvec, band, spinor) of one k-point) and the
 // padded, column-ordered device buffer, where band b's spinor s is row
-// nspinor * b + s (only the requested bands; buffer bands stay on the device)
+// nspinor * b + s (only the requested bands; buffer bands stay on the
+// device).  The x-line buffer, free between calls, stages the host rows.
 static int copy_slice(derek_gpu_t *h, int ki, void *dev_base, double *host, bool to_dev) {
   const KSetDev &K = h->ks[ki];
-  const size_t es = h->elem_size();
-  char *dev = (char *)dev_base + (size_t)K.psi_off * es;
-  const int nb = K.nbr;
-  const int nsp = h->sys[K.sys].nspinor;
-  auto host_row = [nb, nsp](int p) { return nsp == 1 ? p : (p % 2) * (nb / 2) + p / 2; };
-  const size_t n = (size_t)nb * K.npw_pad;
-  const int32_t *perm = h->perm.data() + K.ent_off;
-  const bool f64 = h->prec == DEREK_PREC_FP64;
-  std::vector<double> t64(f64 ? 2 * n : 0, 0.0);
-  std::vector<float> t32(f64 ? 0 : 2 * n, 0.0f);
-  if (to_dev) {
-    for (int b = 0; b < nb; ++b)
-      for (int g = 0; g < K.npw; ++g) {
-        const size_t src = 2 * ((size_t)host_row(b) * K.npw + perm[g]);
-        const size_t dst = 2 * ((size_t)b * K.npw_pad + g);
-        if (f64) {
-          t64[dst] = host[src];
-          t64[dst + 1] = host[src + 1];
-        } else {
-          t32[dst] = (float)host[src];
-          t32[dst + 1] = (float)host[src + 1];
-        }
-      }
-    DEREK_CUDA(h, cudaMemcpyAsync(dev, f64 ? (void *)t64.data() : (void *)t32.data(), n * es,
-                                  cudaMemcpyHostToDevice, h->stream));
-    DEREK_CUDA(h, cudaStreamSynchronize(h->stream));
-  } else {
-    DEREK_CUDA(h, cudaMemcpyAsync(f64 ? (void *)t64.data() : (void *)t32.data(), dev, n * es,
-                                  cudaMemcpyDeviceToHost, h->stream));
-    DEREK_CUDA(h, cudaStreamSynchronize(h->stream));
-    for (int b = 0; b < nb; ++b)
-      for (int g = 0; g < K.npw; ++g) {
-        const size_t dst = 2 * ((size_t)host_row(b) * K.npw + perm[g]);
-        const size_t src = 2 * ((size_t)b * K.npw_pad + g);
-        host[dst] = f64 ? t64[src] : (double)t32[src];
-        host[dst + 1] = f64 ? t64[src + 1] : (double)t32[src + 1];
-      }
+  char *dev = (char *)dev_base + (size_t)K.psi_off * h->elem_size();
+  const int nsp = h->sys[K.sys].nspinor, f64 = h->prec == DEREK_PREC_FP64;
+  const int *perm = h->d_perm + K.ent_off;
+  const size_t row = (size_t)K.npw * sizeof(double2);
+  const int chunk = (int)std::min<size_t>(K.nbr, h->abuf_bytes / row);
+  double2 *stage = (double2 *)h->d_abuf;
+  for (int r = 0; r < K.nbr; r += chunk) {
+    const int count = std::min(chunk, K.nbr - r);
+    double *hr = host + 2 * (size_t)r * K.npw;
+    if (to_dev) {
+      DEREK_CUDA(h, cudaMemcpyAsync(stage, hr, count * row, cudaMemcpyHostToDevice, h->stream));
+      launch_wfn_in(f64, stage, perm, K, nsp, r, count, dev, h->stream);
+    } else {
+      launch_wfn_out(f64, dev, perm, K, nsp, r, count, stage, h->stream);
+      DEREK_CUDA(h, cudaMemcpyAsync(hr, stage, count * row, cudaMemcpyDeviceToHost, h->stream));
+    }
   }
+  DEREK_CUDA(h, cudaGetLastError());
+  DEREK_CUDA(h, cudaStreamSynchronize(h->stream));
   return DEREK_OK;
 }
 

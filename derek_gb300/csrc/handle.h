@@ -29,7 +29,6 @@ struct derek_gpu {
   std::vector<int> item_ks, item_band;
   std::vector<int32_t> box_rows, fft_index;  // per sphere entry, reference order
   std::vector<double> kin64;                 // reference order
-  std::vector<int32_t> perm;                 // column-order entry -> reference entry
   std::vector<double> kin_col;               // kinetic energies, column order
   std::vector<double> vext_host;   // per system grid, concatenated
 
@@ -49,6 +48,7 @@ struct derek_gpu {
   int *d_ent_col = nullptr, *d_col_start = nullptr;
   short *d_ent_ix = nullptr, *d_col_y = nullptr, *d_col_z = nullptr, *d_col_x0 = nullptr, *d_rows = nullptr;
   int *d_pw_entry = nullptr;   // per item: entry of its band's start plane wave
+  int *d_perm = nullptr;       // column-order entry -> reference entry
   double *d_kin64 = nullptr;
   float *d_kin32 = nullptr;
   double2 *d_tw64 = nullptr;
@@ -79,7 +79,8 @@ struct derek_gpu {
 
   // ---- device psi-shaped buffers (element type by precision)
   void *d_X = nullptr, *d_Y = nullptr, *d_Yp = nullptr, *d_HX = nullptr;
-  void *d_abuf = nullptr;          // x-line buffer of the H.psi passes
+  void *d_abuf = nullptr;          // x-line buffer of the H.psi passes; stages host wavefunctions
+  size_t abuf_bytes = 0;
   double *d_occw = nullptr;        // per item: w_k f / Omega (density weights)
   double *d_eig = nullptr;         // per item
   double *d_occ = nullptr;         // per item: f in [0, 2]

@@ -109,6 +109,13 @@ bool launch_density_reg(const Tables &t, const DensityUnit *units, int nunits, i
 void launch_fft3d_grid(const Tables &t, int sys_begin, int nsys, int max_n, double2 *data,
                        int sign, cudaStream_t st);
 
+// wavefunction slices of one k-set: `count` of the caller's rows from row0 on,
+// in the caller's layout, to or from the device slice (wfn_io.cu)
+void launch_wfn_in(int fp64, const double2 *src, const int *perm, const KSetDev &K, int nsp, int row0, int count,
+                   void *dst, cudaStream_t st);
+void launch_wfn_out(int fp64, const void *src, const int *perm, const KSetDev &K, int nsp, int row0, int count,
+                    double2 *dst, cudaStream_t st);
+
 void launch_lda(long n, const double *rho, double *exc, double *vxc, cudaStream_t st);
 
 }  // namespace derek
