@@ -394,7 +394,7 @@ extern "C" int derek_gpu_grad_density_loss(derek_gpu_t *h, int s, const double *
                            h->d_opart_off, h->d_Hs, h->d_mat_off, 1, st);
     derek::note_launch(), k_pair_weights<<<h->nks, 256, 0, st>>>(tM, h->d_eig, h->d_occ, h->d_Hs, h->d_mat_off, h->d_C);
     CKA(cudaMemcpyAsync(W.xi, psi, np * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-    launch_rotate<double>(tM, 0, h->nks, h->max_nb, h->max_npw, W.xi, h->d_C, h->d_mat_off, st);
+    launch_rotate<double>(tM, 0, h->nks, h->max_nb, h->max_npw, W.xi, h->d_C, h->d_mat_off, 0, st);
     e = cross_density(psi, W.xi, w_pair, W.dn_out);
     if (e) return e;
     // diagonal V_nn for the Fermi shift

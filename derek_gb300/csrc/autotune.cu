@@ -512,7 +512,7 @@ struct Tuner {
     int best_tc = 1;
     for (int tc = 1; tc >= 0; --tc) {
       h->tune.rotate_tc = tc;
-      const float ms = tm.best(h, 3, [&] { rotate_all(h, h->d_Y, h->d_C); });
+      const float ms = tm.best(h, 3, [&] { rotate_all(h, h->d_Y, h->d_C, 0); });
       if (ms < best) best = ms, best_tc = tc;
     }
     h->tune.rotate_tc = best_tc;

@@ -205,7 +205,7 @@ bool tc_capable(const derek_gpu *h);
 bool use_tc_overlap(const derek_gpu *h);
 bool use_tc_rotate(const derek_gpu *h);
 int overlap_all(derek_gpu *h, const void *A, const void *B, double2 *out, int hermitize);
-int rotate_all(derek_gpu *h, void *X, const double2 *C);
+int rotate_all(derek_gpu *h, void *X, const double2 *C, int upper);   // upper: C upper triangular
 // The host copy of the system table (every system active) back on the
 // device: the SCF masks converged systems off there, the primitives
 // (apply_h, overlap) work on any system.

@@ -65,16 +65,16 @@ int overlap_all(derek_gpu *h, const void *A, const void *B, double2 *out, int he
   return DEREK_OK;
 }
 
-int rotate_all(derek_gpu *h, void *X, const double2 *C) {
+int rotate_all(derek_gpu *h, void *X, const double2 *C, int upper) {
   if (use_tc_rotate(h))
     launch_rotate_tc(h->tab_band, 0, h->nks, h->max_nb_band, h->max_npw_band, (float2 *)X, C, h->d_mat_off,
                      h->d_rot_img, h->d_status, h->stream);
   else if (h->prec == DEREK_PREC_FP64)
     launch_rotate<double>(h->tab_band, 0, h->nks, h->max_nb_band, h->max_npw_band, (double2 *)X, C, h->d_mat_off,
-                          h->stream);
+                          upper, h->stream);
   else
     launch_rotate<float>(h->tab_band, 0, h->nks, h->max_nb_band, h->max_npw_band, (float2 *)X, C, h->d_mat_off,
-                         h->stream);
+                         upper, h->stream);
   return DEREK_OK;
 }
 
@@ -88,7 +88,7 @@ int cholqr_rr(derek_gpu *h) {
   overlap_all(h, X, X, h->d_S, 1);
   launch_cholesky_inv(h->tab_band, 0, h->nks, h->max_nb_band, h->d_S, h->d_C, h->d_mat_off, h->d_scratch,
                       h->d_status, h->stream);
-  rotate_all(h, X, h->d_C);
+  rotate_all(h, X, h->d_C, 1);   // L^-H
   int st = apply_h_items(h, 0, h->nitems, X, nullptr, h->d_HX, nullptr);
   if (st) return st;
   overlap_all(h, X, h->d_HX, h->d_Hs, 1);
@@ -99,7 +99,7 @@ int cholqr_rr(derek_gpu *h) {
   const double jtol = h->prec == DEREK_PREC_FP64 ? 1e-14 : 1e-10;
   launch_jacobi(h->tab_band, 0, h->nks, h->max_nb_band, h->d_Hs, h->d_C, h->d_mat_off, h->d_eig,
                 h->d_scratch, 30, jtol, 0, h->d_sweeps, h->stream, h->tune.jacobi_single);
-  rotate_all(h, X, h->d_C);
+  rotate_all(h, X, h->d_C, 0);
   return DEREK_OK;
 }
 

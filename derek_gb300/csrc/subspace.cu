@@ -14,6 +14,18 @@
 
 namespace derek {
 
+// acc += a b as four fused multiply-adds.  (acc.x += a.x b.x - a.y b.y compiles
+// to a product, a fused multiply-add and an addition: three slots of the pipe
+// per component instead of two.)
+__device__ __forceinline__ double fmadd(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fmadd(float a, float b, float c) { return fmaf(a, b, c); }
+template <typename R> __device__ __forceinline__ void cmac(cplx<R> &acc, cplx<R> a, cplx<R> b) {
+  acc.x = fmadd(a.x, b.x, acc.x);
+  acc.y = fmadd(a.x, b.y, acc.y);
+  acc.x = fmadd(-a.y, b.y, acc.x);
+  acc.y = fmadd(a.y, b.x, acc.y);
+}
+
 // ---------------------------------------------------------------------------
 // Overlap: part[ks][split] = sum_{G in split} conj(A_i(G)) B_j(G)
 //
@@ -113,8 +125,8 @@ __global__ void __launch_bounds__(256) k_overlap_pairs(const Tables t, int ks_be
         for (int u = 0; u < MT; ++u)
 #pragma unroll
           for (int v = 0; v < MT; ++v) {
-            acc[q][u][v].x += a[u].x * b[v].x + a[u].y * b[v].y;
-            acc[q][u][v].y += a[u].x * b[v].y - a[u].y * b[v].x;
+            // conj(a) b: conjugate of a on the left factor
+            cmac<R>(acc[q][u][v], mk<R>(a[u].x, -a[u].y), b[v]);
           }
       }
     }
@@ -194,65 +206,135 @@ __global__ void __launch_bounds__(256) k_overlap_reduce(const Tables t, int ks_b
 }
 
 // ---------------------------------------------------------------------------
-// Rotation: X[:, j] <- sum_i X[:, i] C[i][j], in place per G tile
+// Rotation: X[:, j] <- sum_i X[:, i] C[i][j], in place per G tile.  upper: C is
+// upper triangular (the Cholesky factor L^-H), rows i > j are left out.
+// A lane holds a G, a warp a set of output bands j, so C is read as a
+// broadcast.  JQ is the number of bands per thread the widest subspace needs:
+// with room for 128 bands whatever the subspace, predicated-off multiply-adds
+// of the missing bands cost as much of the pipe as real ones.
 // ---------------------------------------------------------------------------
-constexpr int RG = 32;   // G columns per block
-constexpr int RI = 32;   // rows of C staged per chunk
-constexpr int RJ = 16;   // max output bands per thread (nb <= 8 * RJ = 128)
+constexpr int RG = 32;      // G columns per tile
+constexpr int RWARPS = 8;
+constexpr int RROWS = 8;    // rows of C staged at a time (FP64), skip unit of upper
 
-template <typename R>
-__global__ void __launch_bounds__(256) k_rotate(const Tables t, int ks_begin, cplx<R> *__restrict__ X,
-                                                const double2 *__restrict__ C,
-                                                const long long *__restrict__ mat_off) {
+// FP64: bound by the FP64 pipe.  The whole X tile sits in shared memory, C
+// passes through it in chunks of RROWS rows; warp w holds bands w, w + 8, ...
+// Measured, 84 bands x 17,529 on 4 k-points: 8.6 -> 3.3 ms full, 1.8 ms upper
+// (pipe time 3.2 and 1.6 ms).
+template <int JQ>
+__global__ void __launch_bounds__(256, 2) k_rotate64(const Tables t, int ks_begin, double2 *__restrict__ X,
+                                                     const double2 *__restrict__ C,
+                                                     const long long *__restrict__ mat_off, int upper) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ksi = ks_begin + blockIdx.y;
   const KSetDev &K = t.ks[ksi];
   if (!t.sys[K.sys].active) return;
-  const int g0 = blockIdx.x * RG;
-  if (g0 >= K.npw) return;
-  const int nb = K.nb;
-  cplx<R> *Xs = reinterpret_cast<cplx<R> *>(smem_raw);   // [RI][RG]
-  cplx<R> *Cs = Xs + RI * RG;                            // [RI][nb]
-  const int g = threadIdx.x % RG, jg = threadIdx.x / RG;  // 8 j-groups
-  cplx<R> acc[RJ];
-#pragma unroll
-  for (int q = 0; q < RJ; ++q) acc[q] = mk<R>(0, 0);
-  cplx<R> *Xb = X + K.psi_off;
+  const int g0 = blockIdx.x * RG, npw = K.npw, nb = K.nb;
+  if (g0 >= npw) return;
+  double2 *Xs = reinterpret_cast<double2 *>(smem_raw);   // [nb][RG]
+  double2 *Cs = Xs + nb * RG;                            // [RROWS][nb]
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double2 *Xb = X + K.psi_off;
   const double2 *Cb = C + mat_off[ksi];
-  for (int i0 = 0; i0 < nb; i0 += RI) {
-    const int ni = min(RI, nb - i0);
-    for (int e = threadIdx.x; e < RI * RG; e += blockDim.x) {
-      const int r = e / RG, c = e % RG;
-      const int gg = g0 + c;
-      Xs[e] = (r < ni && gg < K.npw) ? Xb[(long long)(i0 + r) * K.npw_pad + gg] : mk<R>(0, 0);
-    }
-    for (int e = threadIdx.x; e < ni * nb; e += blockDim.x) {
-      const int r = e / nb, c = e % nb;
-      const double2 v = Cb[(long long)(i0 + r) * nb + c];
-      Cs[r * nb + c] = mk<R>((R)v.x, (R)v.y);
-    }
-    __syncthreads();
-    for (int r = 0; r < ni; ++r) {
-      const cplx<R> x = Xs[r * RG + g];
+  for (int r = w; r < nb; r += RWARPS)
+    Xs[r * RG + lane] = g0 + lane < npw ? Xb[(long long)r * K.npw_pad + g0 + lane] : make_double2(0.0, 0.0);
+  double2 acc[JQ];
 #pragma unroll
-      for (int q = 0; q < RJ; ++q) {
-        const int j = jg + 8 * q;
-        if (j < nb) {
-          const cplx<R> c = Cs[r * nb + j];
-          acc[q].x += x.x * c.x - x.y * c.y;
-          acc[q].y += x.x * c.y + x.y * c.x;
-        }
+  for (int q = 0; q < JQ; ++q) acc[q] = make_double2(0.0, 0.0);
+  for (int r0 = 0; r0 < nb; r0 += RROWS) {
+    const int nr = min(RROWS, nb - r0);
+    for (int e = threadIdx.x; e < nr * nb; e += blockDim.x) Cs[e] = Cb[(long long)r0 * nb + e];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < JQ; ++q) {
+      const int j = w + RWARPS * q;
+      if (j >= nb || (upper && j < r0)) continue;
+      for (int r = 0; r < nr; ++r) {
+        const double2 x = Xs[(r0 + r) * RG + lane], c = Cs[r * nb + j];
+        cmac<double>(acc[q], x, c);
       }
     }
     __syncthreads();
   }
-  const int gg = g0 + g;
-  if (gg < K.npw) {
+  if (g0 + lane < npw) {
 #pragma unroll
-    for (int q = 0; q < RJ; ++q) {
-      const int j = jg + 8 * q;
-      if (j < nb) Xb[(long long)j * K.npw_pad + gg] = acc[q];
+    for (int q = 0; q < JQ; ++q) {
+      const int j = w + RWARPS * q;
+      if (j < nb) Xb[(long long)j * K.npw_pad + g0 + lane] = acc[q];
     }
+  }
+}
+
+// FP32, bound by shared-memory loads and multiply-adds alike: C is converted once per block into shared memory (FP64-to-FP32
+// conversions run on the FP64 pipe; per 32 columns they took as long as the
+// product itself) and the block walks G tiles of 64.  A thread holds two G and
+// the band pairs 2 (w + 8 q) + {0, 1}: one 16-byte broadcast of C per four
+// complex products.
+template <int JQ>
+__global__ void __launch_bounds__(256, 2) k_rotate32(const Tables t, int ks_begin, float2 *__restrict__ X,
+                                                     const double2 *__restrict__ C,
+                                                     const long long *__restrict__ mat_off, int upper) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int ksi = ks_begin + blockIdx.y;
+  const KSetDev &K = t.ks[ksi];
+  if (!t.sys[K.sys].active) return;
+  constexpr int TG = 2 * RG;
+  const int npw = K.npw, nb = K.nb, ldc = (nb + 1) & ~1;
+  if ((int)blockIdx.x * TG >= npw) return;
+  float2 *Cs = reinterpret_cast<float2 *>(smem_raw);   // [nb][ldc]
+  float2 *Xs = Cs + nb * ldc;                          // [nb][TG]
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  float2 *Xb = X + K.psi_off;
+  const double2 *Cb = C + mat_off[ksi];
+  for (int r = w; r < nb; r += RWARPS)
+    for (int c = lane; c < ldc; c += 32) {
+      const double2 v = c < nb ? Cb[(long long)r * nb + c] : make_double2(0.0, 0.0);
+      Cs[r * ldc + c] = make_float2((float)v.x, (float)v.y);
+    }
+  for (int g0 = blockIdx.x * TG; g0 < npw; g0 += gridDim.x * TG) {
+    __syncthreads();   // C staged; the previous tile's reads done
+    for (int r = w; r < nb; r += RWARPS)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int g = g0 + lane + 32 * u;
+        Xs[r * TG + lane + 32 * u] = g < npw ? Xb[(long long)r * K.npw_pad + g] : make_float2(0.f, 0.f);
+      }
+    __syncthreads();
+    float2 acc[JQ][2][2];
+#pragma unroll
+    for (int q = 0; q < JQ; ++q)
+#pragma unroll
+      for (int v = 0; v < 2; ++v)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) acc[q][v][u] = make_float2(0.f, 0.f);
+    for (int r0 = 0; r0 < nb; r0 += RROWS) {
+      const int r1 = min(nb, r0 + RROWS);
+      // the first pair this chunk of rows reaches
+      const int q0 = upper ? max(0, (r0 / 2 - w + RWARPS - 1) / RWARPS) : 0;
+      for (int r = r0; r < r1; ++r) {
+        const float2 x0 = Xs[r * TG + lane], x1 = Xs[r * TG + lane + 32];
+#pragma unroll
+        for (int q = 0; q < JQ; ++q) {
+          const int j = 2 * (w + RWARPS * q);
+          if (j >= nb || q < q0) continue;
+          const float4 c = *reinterpret_cast<const float4 *>(&Cs[r * ldc + j]);
+          const float2 ca = make_float2(c.x, c.y), cb = make_float2(c.z, c.w);
+          cmac<float>(acc[q][0][0], x0, ca);
+          cmac<float>(acc[q][0][1], x1, ca);
+          cmac<float>(acc[q][1][0], x0, cb);
+          cmac<float>(acc[q][1][1], x1, cb);
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < JQ; ++q)
+#pragma unroll
+      for (int v = 0; v < 2; ++v)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int j = 2 * (w + RWARPS * q) + v, g = g0 + lane + 32 * u;
+          if (j < nb && g < npw) Xb[(long long)j * K.npw_pad + g] = acc[q][v][u];
+        }
   }
 }
 
@@ -840,12 +922,41 @@ void launch_overlap_reduce(const Tables &t, int ks_begin, int nks, int max_nb, c
 
 template <typename R>
 void launch_rotate(const Tables &t, int ks_begin, int nks, int max_nb, int max_npw, cplx<R> *X,
-                   const double2 *C, const long long *mat_off, cudaStream_t st) {
+                   const double2 *C, const long long *mat_off, int upper, cudaStream_t st) {
   if (nks <= 0) return;
-  const size_t sm = (RI * RG + (size_t)RI * max_nb) * sizeof(cplx<R>);
-  cudaFuncSetAttribute(k_rotate<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  dim3 grid((max_npw + RG - 1) / RG, nks);
-  derek::note_launch(), k_rotate<R><<<grid, 256, sm, st>>>(t, ks_begin, X, C, mat_off);
+  constexpr bool F64 = std::is_same<R, double>::value;
+  const int ldc = (max_nb + 1) & ~1;
+  const size_t sm = F64 ? (size_t)max_nb * (RG + RROWS) * sizeof(cplx<R>)
+                        : (size_t)max_nb * (ldc + 2 * RG) * sizeof(cplx<R>);
+  const int tiles = (max_npw + (F64 ? RG : 2 * RG) - 1) / (F64 ? RG : 2 * RG);
+  // FP32 blocks keep their converted C over several tiles once that leaves
+  // four blocks per SM
+  const int gx = F64 ? tiles : std::min(tiles, std::max(1, (4 * sm_count() + nks - 1) / nks));
+  auto go = [&](auto kern) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    derek::note_launch(), kern<<<dim3(gx, nks), 256, sm, st>>>(t, ks_begin, X, C, mat_off, upper);
+  };
+  if constexpr (F64) {
+    switch ((max_nb + RWARPS - 1) / RWARPS) {
+      case 1: go(k_rotate64<1>); break;
+      case 2: go(k_rotate64<2>); break;
+      case 3: go(k_rotate64<3>); break;
+      case 4: go(k_rotate64<4>); break;
+      case 5: case 6: go(k_rotate64<6>); break;
+      case 7: case 8: go(k_rotate64<8>); break;
+      case 9: case 10: case 11: case 12: go(k_rotate64<12>); break;
+      default: go(k_rotate64<16>); break;
+    }
+  } else {
+    switch ((max_nb + 2 * RWARPS - 1) / (2 * RWARPS)) {
+      case 1: go(k_rotate32<1>); break;
+      case 2: go(k_rotate32<2>); break;
+      case 3: go(k_rotate32<3>); break;
+      case 4: go(k_rotate32<4>); break;
+      case 5: case 6: go(k_rotate32<6>); break;
+      default: go(k_rotate32<8>); break;
+    }
+  }
 }
 
 bool cholesky_fits_smem(int max_nb) { return 2 * (size_t)max_nb * max_nb * 16 <= 200 * 1024; }
@@ -910,7 +1021,7 @@ void launch_jacobi(const Tables &t, int ks_begin, int nks, int max_nb, const dou
                                   const cplx<R> *, double2 *, const long long *, double2 *,   \
                                   const long long *, int, cudaStream_t);                      \
   template void launch_rotate<R>(const Tables &, int, int, int, int, cplx<R> *,               \
-                                 const double2 *, const long long *, cudaStream_t);
+                                 const double2 *, const long long *, int, cudaStream_t);
 DEREK_INST(float)
 DEREK_INST(double)
 #undef DEREK_INST

@@ -77,3 +77,21 @@ def test_spinor_register_planes(oracle, n, rows):
         h.set_wfn(psi)
         got = h.pot_apply_wfn()
     assert rel_err(got, oracle.apply_h_spinor(s, kb, nc, psi)) < 2e-5
+
+
+# every count of bands per thread of the rotations, odd ones among them, and a
+# last G tile that is partly filled: band energies (the lower half, well inside
+# the subspace) against the dense Hamiltonian, bounds as tests/test_gpu_nscf.py
+@pytest.mark.parametrize("precision,eig_tol,tol", [(0, 1e-10, 1e-8), (1, 5e-6, 2e-5)])
+@pytest.mark.parametrize("nb", [1, 7, 8, 9, 17, 25, 33, 49, 64, 65, 97, 124])
+def test_rotations_at_every_band_count(oracle, nb, precision, eig_tol, tol):
+    import derek_gb300 as dg
+    from test_gpu_nscf import dense_eigenvalues
+    from test_gpu_primitives import make_pair
+    s, spec = make_pair(oracle, L=9.0, ecut=5.0, nb=nb, nelec=1.0, seed=nb)
+    nconv = (nb + 1) // 2
+    with dg.Handle(spec, precision=precision, buffer_bands=4, use_tensor_cores=0, init_vectors=1) as h:
+        h.set_vloc(s.vext)
+        (eig,), _ = h.nscf(max_iter=300, eig_tol=eig_tol, nconv=nconv)
+    ref = dense_eigenvalues(oracle, s, 0, s.vext, nconv)
+    assert np.max(np.abs(eig[0, :nconv] - ref)) < tol
