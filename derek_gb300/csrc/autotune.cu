@@ -536,7 +536,7 @@ struct Tuner {
     for (int single = 0; single <= 1; ++single) {
       const float ms = tm.best(h, 2, [&] {
         launch_jacobi(h->tab_band, 0, h->nks, h->max_nb_band, h->d_Hs, h->d_C, h->d_mat_off, h->d_eig,
-                      h->d_scratch, 30, h->prec == DEREK_PREC_FP64 ? 1e-14 : 1e-10, 0, h->d_sweeps, h->stream,
+                      h->d_scratch, 30, h->prec == DEREK_PREC_FP64 ? 1e-14 : 1e-10, h->d_sweeps, h->stream,
                       single);
       });
       if (ms < best) best = ms, best_single = single;

@@ -98,7 +98,7 @@ int cholqr_rr(derek_gpu *h) {
   // saving about one of the four sweeps near convergence.
   const double jtol = h->prec == DEREK_PREC_FP64 ? 1e-14 : 1e-10;
   launch_jacobi(h->tab_band, 0, h->nks, h->max_nb_band, h->d_Hs, h->d_C, h->d_mat_off, h->d_eig,
-                h->d_scratch, 30, jtol, 0, h->d_sweeps, h->stream, h->tune.jacobi_single);
+                h->d_scratch, 30, jtol, h->d_sweeps, h->stream, h->tune.jacobi_single);
   rotate_all(h, X, h->d_C, 0);
   return DEREK_OK;
 }

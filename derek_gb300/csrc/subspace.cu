@@ -38,17 +38,19 @@ template <typename R> __device__ __forceinline__ void cmac(cplx<R> &acc, cplx<R>
 // one is its exact conjugate).  Every block stages OKC coefficients of all
 // bands.  The split along G is as fine as it takes to give every SM blocks
 // (launch_overlap).  Measured, FP64: 12 bands x 1,510 plane waves 716 -> 12 us
-// (A = B) and 15 us; 84 bands x 17,529 on 4 k-points 8.2 -> 2.8 ms (A = B) and
-// 5.5 ms (1.0 and 2.0 x 10^9 multiply-adds at the pipe's rate: 1.6 and 3.2 ms).
+// (A = B) and 15 us; 84 bands x 17,529 on 4 k-points 8.2 -> 1.7 ms (A = B) and
+// 3.7 ms (1.0 and 2.0 x 10^9 multiply-adds at the pipe's rate: 1.6 and 3.2 ms).
 // ---------------------------------------------------------------------------
 template <typename R> struct OverlapShape;
 // FP64: one pair per tile, its four fused multiply-adds hide both loads
 template <> struct OverlapShape<double> {
   static constexpr int MT = 1, OKC = 16, PMAX = 8;
 };
-// FP32: 2 x 2 pairs, half the shared loads per multiply-add
+// FP32: 2 x 2 pairs, half the shared loads per multiply-add; short chunks, whose
+// sums are rounded on their own (an SCF's free energy at its FP32 noise floor
+// moves by 1.9e-7 Ha per iteration, 3.8e-7 with one running sum)
 template <> struct OverlapShape<float> {
-  static constexpr int MT = 2, OKC = 32, PMAX = 4;
+  static constexpr int MT = 2, OKC = 16, PMAX = 4;
 };
 
 template <typename R, int P, bool SAME>
@@ -110,6 +112,15 @@ __global__ void __launch_bounds__(256) k_overlap_pairs(const Tables t, int ks_be
       if (!SAME) Bs[r * LD + c] = in ? Bb[(long long)r * K.npw_pad + g] : mk<R>(0, 0);
     }
     __syncthreads();
+    // FP32 sums in two levels, the chunk's products first: the rounding of a
+    // long running sum is what the Ritz values' noise comes from
+    cplx<R> sum[P][MT][MT];
+#pragma unroll
+    for (int q = 0; q < P; ++q)
+#pragma unroll
+      for (int u = 0; u < MT; ++u)
+#pragma unroll
+        for (int v = 0; v < MT; ++v) sum[q][u][v] = std::is_same<R, float>::value ? mk<R>(0, 0) : acc[q][u][v];
 #pragma unroll 2
     for (int c = 0; c < OKC; ++c) {
 #pragma unroll
@@ -126,10 +137,17 @@ __global__ void __launch_bounds__(256) k_overlap_pairs(const Tables t, int ks_be
 #pragma unroll
           for (int v = 0; v < MT; ++v) {
             // conj(a) b: conjugate of a on the left factor
-            cmac<R>(acc[q][u][v], mk<R>(a[u].x, -a[u].y), b[v]);
+            cmac<R>(sum[q][u][v], mk<R>(a[u].x, -a[u].y), b[v]);
           }
       }
     }
+#pragma unroll
+    for (int q = 0; q < P; ++q)
+#pragma unroll
+      for (int u = 0; u < MT; ++u)
+#pragma unroll
+        for (int v = 0; v < MT; ++v)
+          acc[q][u][v] = std::is_same<R, float>::value ? cadd<R>(acc[q][u][v], sum[q][u][v]) : sum[q][u][v];
     __syncthreads();
   }
   double2 *dst = part + part_off[ksi] + (long long)blockIdx.y * nb * nb;
@@ -434,14 +452,391 @@ __global__ void __launch_bounds__(256) k_cholesky_inv(const Tables t, int ks_beg
 // Entry (i, j) of U^H A U depends only on the 2x2 block of A at the pairs
 // holding i and j, so a round is one pass over the blocks (a <= b) of pairs:
 // A'_ab = U_a^H A_ab U_b, with A'_ba = A'_ab^H written by the same thread.
-// That touches half of A, with all arithmetic on A in FP64.  The
-// eigenvectors accumulate in VT (FP64, or FP32 on the mixed-precision path,
-// whose wavefunctions are FP32), stored one eigenvector per row so that a
-// warp updates consecutive addresses.  Eigenvalues ascending go to
-// eig[item0 + j]; eigenvectors (columns) to C.
+// All arithmetic on A and on the eigenvectors, stored one per row, is FP64.
+// Eigenvalues ascending go to eig[item0 + j]; eigenvectors (columns) to C.
+//
+// Bound by FP64 issue: an FP64 operation of one warp takes 64 clocks of its
+// quarter of the SM, dependent or not, so what counts is operations per warp
+// on the fullest quarter.
+//   Rotations: the angle and the phase come from FP32 (their error leaves
+//   1e-7 of an off-diagonal element for the next sweep, which squares it), and
+//   (c, s) and the phase are then brought to unit length in FP64 by two terms
+//   of 1/sqrt(1 + d), d ~ 1e-7.  12 FP64 operations instead of two reciprocal
+//   roots, a root and a division in a chain of ~2,700 clocks.
+//   Blocks: one per thread (LPB = 1) or, where a CTA has few, one element per
+//   lane (LPB = 4).
+//   A cluster of CS CTAs shares a k-set: each CTA keeps a full copy of A,
+//   computes every rotation (equal copies, equal decisions), updates its share
+//   of the blocks in all copies through distributed shared memory, and its
+//   slice of the eigenvector rows.
+// Two cluster barriers a round, both split so that work covers them: B1, every
+// CTA has read this round's pivots, before remote copies are written (the
+// first block is computed between arrival and wait); B2, every block is
+// written, with the eigenvector update in between.
+// Measured per solve, mean over an SCF, against two CTAs with exact angles: n =
+// 12, 178 -> 98 us; n = 24, 8 k-sets, 560 -> 340 us, 40 k-sets 542 -> 363 us; n =
+// 84, 4 k-sets, 9.6 -> 4.4 ms; 64 k-sets 7.8 ms either way (two CTAs, all of it
+// FP64 issue).
 // ---------------------------------------------------------------------------
+__host__ __device__ constexpr size_t jacobi_round_bytes(size_t np) {
+  return (np * (sizeof(double2) + 2 * sizeof(double) + 3 * sizeof(int)) + 15) / 16 * 16;
+}
+struct JacobiTables {   // of one round, in shared memory
+  double2 *ph;
+  double *c, *s;
+  int *pp, *pq, *act;
+};
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
 // pair k of round r in the circle schedule over ne positions (position 0
 // fixed, the others advance one place per round)
+__device__ __forceinline__ void rr_pair(int k, int r, int ne, int &p, int &q) {
+  const int m = ne - 1;
+  int a = k - 1 + r, b = ne - 2 - k + r;
+  if (a >= m) a -= m;
+  if (b >= m) b -= m;
+  a = k == 0 ? 0 : 1 + a;
+  b += 1;
+  p = min(a, b);
+  q = max(a, b);
+}
+
+// neg ? -x : x on the sign bit (a negation by itself is an FP64 operation)
+__device__ __forceinline__ double flip(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
+}
+
+// x + y i scaled to unit length, x^2 + y^2 = 1 + d with |d| ~ 1e-7
+__device__ __forceinline__ void unit_length(double &x, double &y) {
+  const double d = fma(x, x, fma(y, y, -1.0));
+  const double k = fma(d, fma(d, 0.375, -0.5), 1.0);
+  x *= k;
+  y *= k;
+}
+
+template <int CS, int LPB>
+__global__ void __launch_bounds__(256) k_jacobi(const Tables t, int ks_begin, const double2 *__restrict__ Hs,
+                                                double2 *__restrict__ Cout, const long long *__restrict__ mat_off,
+                                                double *__restrict__ eig, int max_sweeps, double tol,
+                                                int *__restrict__ sweeps_out) {
+  namespace cg = cooperative_groups;
+  constexpr int NT = 256;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int crank = blockIdx.x % CS;
+  const int ksi = ks_begin + blockIdx.x / CS;
+  const KSetDev &K = t.ks[ksi];
+  if (!t.sys[K.sys].active) return;   // the whole cluster leaves together
+  const int tid = threadIdx.x;
+  const int n = K.nb;
+  const int ne = n + (n & 1);   // even count for the tournament; index n is a dummy
+  const int np = ne / 2;
+  const int nblk = np * (np + 1) / 2;
+  const int hv = (n + CS - 1) / CS;   // eigenvector rows of a CTA
+  const int v0 = min(n, crank * hv), nv = min(n, v0 + hv) - v0;
+  double2 *A = reinterpret_cast<double2 *>(smem_raw);
+  double2 *Vt = A + n * n;                  // [n][hv]: eigenvector i, rows v0 ...
+  unsigned char *sp = reinterpret_cast<unsigned char *>(Vt + n * hv);
+  // two rounds' tables: a round's eigenvector update overlaps the next round's
+  // rotations
+  auto tables = [sp, np](int i) {
+    JacobiTables T;
+    T.ph = reinterpret_cast<double2 *>(sp + i * jacobi_round_bytes(np));
+    T.c = reinterpret_cast<double *>(T.ph + np);
+    T.s = T.c + np;
+    T.pp = reinterpret_cast<int *>(T.s + np);
+    T.pq = T.pp + np;
+    T.act = T.pq + np;
+    return T;
+  };
+  short2 *blk = reinterpret_cast<short2 *>(sp + 2 * jacobi_round_bytes(np));   // [nblk]: (a, b), a <= b
+  __shared__ float red[2][NT / 32];
+  double2 *copy[CS];   // A of every CTA, the own one first
+  copy[0] = A;
+  if constexpr (CS > 1) {
+    cg::cluster_group cluster = cg::this_cluster();
+#pragma unroll
+    for (int r = 1; r < CS; ++r) copy[r] = cluster.map_shared_rank(A, (crank + r) % CS);
+  }
+  const double2 *Hb = Hs + mat_off[ksi];
+  for (int e = tid; e < n * n; e += NT) A[e] = Hb[e];
+  for (int e = tid; e < n * hv; e += NT) Vt[e] = make_double2(e / hv == v0 + e % hv ? 1.0 : 0.0, 0.0);
+  for (int w = tid; w < nblk; w += NT) {
+    // w -> (a, b) with a <= b, rows of the upper triangle in order
+    int a = 0, rem = w;
+    while (rem >= np - a) {
+      rem -= np - a;
+      ++a;
+    }
+    blk[w] = make_short2((short)a, (short)(a + rem));
+  }
+  if constexpr (CS > 1) {   // every CTA running and initialised before a remote write
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  // A lives in its upper triangle: half the stores to the other copies, whose
+  // 16-byte packets bound large clusters (5.6 -> 4.4 ms at 84 bands, CS = 8)
+  auto get = [&](int r, int c) {
+    const double2 v = A[min(r, c) * n + max(r, c)];
+    return make_double2(v.x, flip(v.y, r > c));
+  };
+  auto put = [&](int r, int c, double2 v) {
+    const int idx = min(r, c) * n + max(r, c);
+    const double2 w = make_double2(v.x, r == c ? 0.0 : flip(v.y, r > c));
+#pragma unroll
+    for (int k = 0; k < CS; ++k) copy[k][idx] = w;
+  };
+  // FP32 arithmetic runs on entries divided by the largest one
+  float big = 0.f;
+  for (int e = tid; e < n * n; e += NT) big = fmaxf(big, fmaxf(fabsf((float)A[e].x), fabsf((float)A[e].y)));
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, w));
+  if ((tid & 31) == 0) red[0][tid >> 5] = big;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < NT / 32; ++w) big = fmaxf(big, red[0][w]);
+  const float scale = big > 0.f ? 1.f / big : 1.f;
+  __syncthreads();
+  int sweep = 0;
+  for (; sweep < max_sweeps; ++sweep) {
+    // convergence: sum of |offdiag|^2 against sum of |A|^2; FP32 sums decide as
+    // well as FP64 ones
+    float off = 0.f, dia = 0.f;
+    for (int e = tid; e < n * n; e += NT) {
+      const float x = (float)A[e].x * scale, y = (float)A[e].y * scale;
+      const int i = e / n, j = e - i * n;
+      if (i == j)
+        dia = fmaf(x, x, dia);
+      else if (i < j)
+        off = fmaf(x, x, fmaf(y, y, off));
+    }
+    off *= 2.f;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+      off += __shfl_xor_sync(0xffffffffu, off, w);
+      dia += __shfl_xor_sync(0xffffffffu, dia, w);
+    }
+    if ((tid & 31) == 0) {
+      red[0][tid >> 5] = off;
+      red[1][tid >> 5] = dia;
+    }
+    __syncthreads();
+    off = dia = 0.f;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+      off += red[0][w];
+      dia += red[1][w];
+    }
+    const float tot = off + dia, ftol = (float)tol;
+    __syncthreads();
+    if (!(off > ftol * ftol * tot)) break;
+    // rotations of elements below tol ||A||_F / (4 n) cannot matter for the
+    // test and are skipped
+    const float skip = ftol / (4.f * n), skip2 = skip * skip * tot;
+    for (int round = 0; round < ne - 1; ++round) {
+      const JacobiTables T = tables(round & 1);
+      // threads 0 .. np-1: phases; threads 128 ..: (c, s) of the same pairs, on
+      // warps of other quarters of the SM
+      const int half = tid >> 7, k = tid & 127;
+      if (k < np) {
+        int p, q;
+        rr_pair(k, round, ne, p, q);
+        double u = 1.0, v = 0.0;
+        int on = 0;
+        if (q < n) {
+          const double2 b = A[p * n + q];
+          const float bx = (float)b.x * scale, by = (float)b.y * scale;
+          const float e2 = bx * bx + by * by;
+          on = e2 > skip2;
+          if (on) {
+            const float ie = rsqrtf(e2);
+            float fu = bx * ie, fv = by * ie;
+            if (half) {
+              const float d = (float)(A[q * n + q].x - A[p * n + p].x) * scale;
+              const float tau = d * (0.5f * ie);
+              const float tt = copysignf(1.f, tau) / (fabsf(tau) + sqrtf(fmaf(tau, tau, 1.f)));
+              fu = rsqrtf(fmaf(tt, tt, 1.f));
+              fv = tt * fu;
+            }
+            u = fu;
+            v = fv;
+            unit_length(u, v);
+          }
+        }
+        if (half) {
+          T.c[k] = u;
+          T.s[k] = v;
+          T.pp[k] = p;
+          T.pq[k] = q;
+        } else {
+          T.ph[k] = make_double2(u, v);
+          T.act[k] = on;
+        }
+      }
+      __syncthreads();
+      if constexpr (CS > 1) cluster_arrive();   // B1: this CTA has read its pivots
+      bool waited = CS == 1;
+      // blocks of A: left by U_a^H (new row p = c A_p - s ph A_q, new row
+      // q = s A_p + c ph A_q), right by U_b (new col p = c X_p - s conj(ph) X_q,
+      // new col q = s X_p + c conj(ph) X_q)
+      if constexpr (LPB == 4) {
+        const int i = (tid >> 1) & 1, j = tid & 1;
+        const int per = (nblk * 4 + CS - 1) / CS;   // items of a CTA
+        for (int base = 0; base < per; base += NT) {
+          const int w = (base + tid) / 4 * CS + crank;
+          const bool in = w < nblk;
+          const short2 ab = in ? blk[w] : make_short2(0, 0);
+          const int ia = ab.x, ib = ab.y;
+          const bool on = in && (T.act[ia] | T.act[ib]);
+          const int row = i ? T.pq[ia] : T.pp[ia], col = j ? T.pq[ib] : T.pp[ib];
+          const bool ok = on && row < n && col < n;
+          double2 x = ok ? get(row, col) : make_double2(0.0, 0.0);
+          double2 y;
+          {
+            y.x = __shfl_xor_sync(0xffffffffu, x.x, 2);
+            y.y = __shfl_xor_sync(0xffffffffu, x.y, 2);
+            const double2 ph = T.ph[ia];
+            const double2 z = zmul(ph, i ? x : y);
+            const double2 o = i ? y : x;
+            const double c = T.c[ia], sn = T.s[ia];
+            const double al = i ? sn : c, be = flip(i ? c : sn, !i);
+            x = make_double2(fma(be, z.x, al * o.x), fma(be, z.y, al * o.y));
+          }
+          {
+            y.x = __shfl_xor_sync(0xffffffffu, x.x, 1);
+            y.y = __shfl_xor_sync(0xffffffffu, x.y, 1);
+            const double2 ph = T.ph[ib];
+            const double2 z = zmul(make_double2(ph.x, -ph.y), j ? x : y);
+            const double2 o = j ? y : x;
+            const double c = T.c[ib], sn = T.s[ib];
+            const double al = j ? sn : c, be = flip(j ? c : sn, !j);
+            x = make_double2(fma(be, z.x, al * o.x), fma(be, z.y, al * o.y));
+          }
+          if constexpr (CS > 1) {
+            if (!waited) {
+              __syncwarp();
+              cluster_wait();
+              waited = true;
+            }
+          }
+          if (ok && (ia != ib || j >= i)) put(row, col, x);
+        }
+      } else {
+        for (int base = 0; base < nblk; base += CS * NT) {
+          const int w = base + tid * CS + crank;
+          const bool in = w < nblk;
+          const short2 ab = in ? blk[w] : make_short2(0, 0);
+          const int ia = ab.x, ib = ab.y;
+          const int on_a = in ? T.act[ia] : 0, on_b = in ? T.act[ib] : 0;
+          const int pa = T.pp[ia], qa = T.pq[ia], pb = T.pp[ib], qb = T.pq[ib];
+          const bool qa_ok = qa < n, qb_ok = qb < n;
+          const double2 z = make_double2(0.0, 0.0);
+          double2 x00 = z, x01 = z, x10 = z, x11 = z;
+          if (on_a | on_b) {
+            x00 = get(pa, pb);
+            if (qb_ok) x01 = get(pa, qb);
+            if (qa_ok) x10 = get(qa, pb);
+            if (qa_ok && qb_ok) x11 = get(qa, qb);
+          }
+          if (on_a) {
+            const double c = T.c[ia], sn = T.s[ia];
+            const double2 ph = T.ph[ia];
+            const double2 t0 = zmul(ph, x10), t1 = zmul(ph, x11);
+            const double2 n00 = make_double2(fma(-sn, t0.x, c * x00.x), fma(-sn, t0.y, c * x00.y));
+            const double2 n01 = make_double2(fma(-sn, t1.x, c * x01.x), fma(-sn, t1.y, c * x01.y));
+            x10 = make_double2(fma(c, t0.x, sn * x00.x), fma(c, t0.y, sn * x00.y));
+            x11 = make_double2(fma(c, t1.x, sn * x01.x), fma(c, t1.y, sn * x01.y));
+            x00 = n00;
+            x01 = n01;
+          }
+          if (on_b) {
+            const double c = T.c[ib], sn = T.s[ib];
+            const double2 ph = T.ph[ib], phc = make_double2(ph.x, -ph.y);
+            const double2 t0 = zmul(phc, x01), t1 = zmul(phc, x11);
+            const double2 n00 = make_double2(fma(-sn, t0.x, c * x00.x), fma(-sn, t0.y, c * x00.y));
+            const double2 n10 = make_double2(fma(-sn, t1.x, c * x10.x), fma(-sn, t1.y, c * x10.y));
+            x01 = make_double2(fma(c, t0.x, sn * x00.x), fma(c, t0.y, sn * x00.y));
+            x11 = make_double2(fma(c, t1.x, sn * x10.x), fma(c, t1.y, sn * x10.y));
+            x00 = n00;
+            x10 = n10;
+          }
+          if constexpr (CS > 1) {
+            if (!waited) {
+              __syncwarp();
+              cluster_wait();
+              waited = true;
+            }
+          }
+          if (!(on_a | on_b)) continue;
+          put(pa, pb, x00);
+          if (qb_ok) put(pa, qb, x01);
+          if (qa_ok && ia != ib) put(qa, pb, x10);   // a pair's own block: the mirror of x01
+          if (qa_ok && qb_ok) put(qa, qb, x11);
+        }
+      }
+      if constexpr (CS > 1) {
+        if (!waited) cluster_wait();
+        __syncwarp();
+        cluster_arrive();   // B2: this CTA's blocks are written everywhere
+      }
+      // eigenvectors: Vt[col][row], new col p = c X_p - s conj(ph) X_q,
+      // new col q = s X_p + c conj(ph) X_q; last threads first, the blocks
+      // fill the first ones
+      for (int w = NT - 1 - tid; w < np * nv; w += NT) {
+        const int kk = w / nv, row = w - kk * nv;
+        if (!T.act[kk]) continue;
+        const double c = T.c[kk], sn = T.s[kk];
+        const double2 ph = T.ph[kk];
+        double2 &xp = Vt[T.pp[kk] * hv + row];
+        double2 &xq = Vt[T.pq[kk] * hv + row];
+        const double2 a = xp, tq = zmul(make_double2(ph.x, -ph.y), xq);
+        xp = make_double2(fma(-sn, tq.x, c * a.x), fma(-sn, tq.y, c * a.y));
+        xq = make_double2(fma(c, tq.x, sn * a.x), fma(c, tq.y, sn * a.y));
+      }
+      if constexpr (CS > 1) {
+        __syncwarp();
+        cluster_wait();
+      } else {
+        __syncthreads();
+      }
+    }
+    __syncthreads();   // the eigenvector update of the last round
+  }
+  if (tid == 0 && crank == 0 && sweeps_out) sweeps_out[ksi] = sweep;
+  // ascending order by rank (ties by index) on order-preserving integer keys
+  long long *key = reinterpret_cast<long long *>(tables(0).ph);
+  int *rank = reinterpret_cast<int *>(tables(1).ph);
+  __syncthreads();
+  for (int i = tid; i < n; i += NT) {
+    const long long v = __double_as_longlong(A[i * n + i].x);
+    key[i] = v < 0 ? ~v ^ (long long)0x8000000000000000ull : v;
+  }
+  __syncthreads();
+  for (int i = tid; i < n; i += NT) {
+    const long long vi = key[i];
+    int r = 0;
+    for (int j = 0; j < n; ++j) r += key[j] < vi || (key[j] == vi && j < i);
+    rank[i] = r;
+    if (crank == 0) eig[K.item0 + r] = A[i * n + i].x;
+  }
+  __syncthreads();
+  double2 *Cb = Cout + mat_off[ksi];
+  for (int e = tid; e < n * nv; e += NT) {
+    const int r = e / n, i = e - r * n;
+    Cb[(v0 + r) * n + rank[i]] = Vt[i * hv + r];
+  }
+  if constexpr (CS > 1) {   // no CTA leaves while a partner could still address it
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+  }
+}
+
+// The same solve with A and the eigenvectors in global scratch, for subspaces
+// whose A does not fit the shared memory (from about 116 bands).
 // Rotation that zeroes the Hermitian 2x2 block [[a, b], [conj(b), d]]: the
 // phase ph = b / |b|, then the real symmetric rotation (c, s) of
 // [[a, |b|], [|b|, d]] with t = sign(tau) / (|tau| + sqrt(1 + tau^2)),
@@ -462,24 +857,14 @@ __device__ __forceinline__ bool jacobi_rotation(double a, double d, double2 b, d
   return true;
 }
 
-__device__ __forceinline__ void rr_pair(int k, int r, int ne, int &p, int &q) {
-  const int m = ne - 1;
-  const int a = k == 0 ? 0 : 1 + (k - 1 + r) % m;
-  const int b = 1 + (ne - 2 - k + r) % m;
-  p = min(a, b);
-  q = max(a, b);
-}
 
-template <typename VT>
-__global__ void __launch_bounds__(256) k_jacobi(const Tables t, int ks_begin,
+__global__ void __launch_bounds__(256) k_jacobi_global(const Tables t, int ks_begin,
                                                 const double2 *__restrict__ Hs,
                                                 double2 *__restrict__ Cout,
                                                 const long long *__restrict__ mat_off,
                                                 double *__restrict__ eig,
                                                 double2 *__restrict__ scratch, int max_sweeps,
-                                                double tol, int a_in_smem, int v_in_smem,
-                                                int *__restrict__ sweeps_out) {
-  using V2 = cplx<VT>;
+                                                double tol, int *__restrict__ sweeps_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ksi = ks_begin + blockIdx.x;
   const KSetDev &K = t.ks[ksi];
@@ -488,12 +873,8 @@ __global__ void __launch_bounds__(256) k_jacobi(const Tables t, int ks_begin,
   const int ne = n + (n & 1);  // even count for the tournament; index n is a dummy
   const int np = ne / 2;
   const int nblk = np * (np + 1) / 2;
-  unsigned char *sp = smem_raw;
-  double2 *A = a_in_smem ? reinterpret_cast<double2 *>(sp) : scratch + 2 * mat_off[ksi] + (long long)n * n;
-  if (a_in_smem) sp += (size_t)n * n * sizeof(double2);
-  V2 *Vt = v_in_smem ? reinterpret_cast<V2 *>(sp) : reinterpret_cast<V2 *>(scratch + 2 * mat_off[ksi]);
-  if (v_in_smem) sp += ((size_t)n * n * sizeof(V2) + 15) / 16 * 16;
-  double2 *rph = reinterpret_cast<double2 *>(sp);  // [np]
+  double2 *Vt = scratch + 2 * mat_off[ksi], *A = Vt + (long long)n * n;
+  double2 *rph = reinterpret_cast<double2 *>(smem_raw);  // [np]
   double *rc = reinterpret_cast<double *>(rph + np);
   double *rs = rc + np;
   int *pp = reinterpret_cast<int *>(rs + np);
@@ -506,10 +887,7 @@ __global__ void __launch_bounds__(256) k_jacobi(const Tables t, int ks_begin,
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
     A[e] = Hb[e];
     const int i = e / n, j = e % n;
-    V2 one;
-    one.x = (VT)(i == j ? 1 : 0);
-    one.y = (VT)0;
-    Vt[e] = one;
+    Vt[e] = make_double2(i == j ? 1.0 : 0.0, 0.0);
   }
   for (int w = threadIdx.x; w < nblk; w += blockDim.x) {
     // w -> (a, b) with a <= b, rows of the upper triangle in order
@@ -629,12 +1007,12 @@ __global__ void __launch_bounds__(256) k_jacobi(const Tables t, int ks_begin,
       for (int w = threadIdx.x; w < np * n; w += blockDim.x) {
         const int k = w / n, row = w - (w / n) * n;
         if (!act[k]) continue;
-        const VT c = (VT)rc[k], s = (VT)rs[k];
-        const VT phx = (VT)rph[k].x, phy = (VT)-rph[k].y;
-        V2 &xp = Vt[pp[k] * n + row];
-        V2 &xq = Vt[pq[k] * n + row];
-        const V2 a = xp, b = xq;
-        const VT tx = phx * b.x - phy * b.y, ty = phx * b.y + phy * b.x;
+        const double c = rc[k], s = rs[k];
+        const double phx = rph[k].x, phy = -rph[k].y;
+        double2 &xp = Vt[pp[k] * n + row];
+        double2 &xq = Vt[pq[k] * n + row];
+        const double2 a = xp, b = xq;
+        const double tx = phx * b.x - phy * b.y, ty = phx * b.y + phy * b.x;
         xp.x = c * a.x - s * tx;
         xp.y = c * a.y - s * ty;
         xq.x = s * a.x + c * tx;
@@ -655,210 +1033,9 @@ __global__ void __launch_bounds__(256) k_jacobi(const Tables t, int ks_begin,
     for (int j = 0; j < n; ++j) rank += (ev[j] < vi) || (ev[j] == vi && j < i);
     eig[K.item0 + rank] = vi;
     for (int r = 0; r < n; ++r) {
-      const V2 v = Vt[i * n + r];
-      Cb[r * n + rank] = make_double2((double)v.x, (double)v.y);
+      Cb[r * n + rank] = Vt[i * n + r];
     }
   }
-}
-
-// ---------------------------------------------------------------------------
-// The same Jacobi eigensolver on a cluster of two CTAs per k-set, so the FP64
-// work of a round is split over two SMs.  Each CTA keeps a full copy of A and
-// computes every rotation (the two copies are equal, so both take the same
-// decisions); it updates half of the 2x2 blocks of a round and writes each
-// result into its own A and, through distributed shared memory, into its
-// partner's, then updates its half of the eigenvector rows.  One cluster
-// barrier per round makes the partner's writes visible before the next
-// round reads A.
-// ---------------------------------------------------------------------------
-template <typename VT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256)
-    k_jacobi_pair(const Tables t, int ks_begin, const double2 *__restrict__ Hs,
-                  double2 *__restrict__ Cout, const long long *__restrict__ mat_off,
-                  double *__restrict__ eig, int max_sweeps, double tol, int *__restrict__ sweeps_out) {
-  using V2 = cplx<VT>;
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int crank = (int)cluster.block_rank();
-  const int ksi = ks_begin + blockIdx.x / 2;
-  const KSetDev &K = t.ks[ksi];
-  if (!t.sys[K.sys].active) return;   // both CTAs of the cluster leave together
-  const int n = K.nb;
-  const int ne = n + (n & 1);
-  const int np = ne / 2;
-  const int nblk = np * (np + 1) / 2;
-  const int hv = (n + 1) / 2;                  // eigenvector rows per CTA
-  const int r0 = crank * hv, r1 = min(n, r0 + hv);
-  unsigned char *sp = smem_raw;
-  double2 *A = reinterpret_cast<double2 *>(sp);
-  sp += (size_t)n * n * sizeof(double2);
-  V2 *Vt = reinterpret_cast<V2 *>(sp);          // [n][hv]: eigenvector i, rows r0..r1
-  sp += ((size_t)n * hv * sizeof(V2) + 15) / 16 * 16;
-  double2 *rph = reinterpret_cast<double2 *>(sp);
-  double *rc = reinterpret_cast<double *>(rph + np);
-  double *rs = rc + np;
-  int *pp = reinterpret_cast<int *>(rs + np);
-  int *pq = pp + np;
-  int *act = pq + np;
-  short2 *blk = reinterpret_cast<short2 *>(act + np);
-  __shared__ double red[256];
-  __shared__ double red2[256];
-  double2 *Ap = cluster.map_shared_rank(A, crank ^ 1);   // the partner's copy of A
-  const double2 *Hb = Hs + mat_off[ksi];
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) A[e] = Hb[e];
-  for (int e = threadIdx.x; e < n * hv; e += blockDim.x) {
-    const int i = e / hv, r = r0 + e % hv;
-    V2 one;
-    one.x = (VT)(i == r ? 1 : 0);
-    one.y = (VT)0;
-    Vt[e] = one;
-  }
-  for (int w = threadIdx.x; w < nblk; w += blockDim.x) {
-    int a = 0, rem = w;
-    while (rem >= np - a) {
-      rem -= np - a;
-      ++a;
-    }
-    blk[w] = make_short2((short)a, (short)(a + rem));
-  }
-  cluster.sync();   // both CTAs running and initialised before any remote write
-  int sweep = 0;
-  for (; sweep < max_sweeps; ++sweep) {
-    double off = 0, tot = 0;
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-      const double m2 = A[e].x * A[e].x + A[e].y * A[e].y;
-      tot += m2;
-      if (e / n != e % n) off += m2;
-    }
-    red[threadIdx.x] = off;
-    red2[threadIdx.x] = tot;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-      if (threadIdx.x < s) {
-        red[threadIdx.x] += red[threadIdx.x + s];
-        red2[threadIdx.x] += red2[threadIdx.x + s];
-      }
-      __syncthreads();
-    }
-    const bool done = red[0] <= tol * tol * red2[0];
-    const double skip = tol * sqrt(red2[0]) / (4.0 * n);
-    __syncthreads();
-    if (done) break;
-    for (int round = 0; round < ne - 1; ++round) {
-      for (int k = threadIdx.x; k < np; k += blockDim.x) {
-        int p, q;
-        rr_pair(k, round, ne, p, q);
-        pp[k] = p;
-        pq[k] = q;
-        double c = 1.0, s = 0.0;
-        double2 ph = make_double2(1.0, 0.0);
-        int on = 0;
-        if (q < n) {
-          on = jacobi_rotation(A[p * n + p].x, A[q * n + q].x, A[p * n + q], skip, c, s, ph) ? 1 : 0;
-        }
-        rc[k] = c;
-        rs[k] = s;
-        rph[k] = ph;
-        act[k] = on;
-      }
-      __syncthreads();
-      for (int w = crank + 2 * (int)threadIdx.x; w < nblk; w += 2 * blockDim.x) {
-        const short2 ab = blk[w];
-        const int ia = ab.x, ib = ab.y;
-        const int on_a = act[ia], on_b = act[ib];
-        if (!on_a && !on_b) continue;
-        const int pa = pp[ia], qa = pq[ia], pb = pp[ib], qb = pq[ib];
-        const bool qa_ok = qa < n, qb_ok = qb < n;
-        const double2 z = make_double2(0.0, 0.0);
-        double2 x00 = A[pa * n + pb];
-        double2 x01 = qb_ok ? A[pa * n + qb] : z;
-        double2 x10 = qa_ok ? A[qa * n + pb] : z;
-        double2 x11 = (qa_ok && qb_ok) ? A[qa * n + qb] : z;
-        if (on_a) {
-          const double c = rc[ia], s = rs[ia];
-          const double2 ph = rph[ia];
-          const double2 t0 = zmul(ph, x10), t1 = zmul(ph, x11);
-          const double2 n00 = make_double2(c * x00.x - s * t0.x, c * x00.y - s * t0.y);
-          const double2 n01 = make_double2(c * x01.x - s * t1.x, c * x01.y - s * t1.y);
-          x10 = make_double2(s * x00.x + c * t0.x, s * x00.y + c * t0.y);
-          x11 = make_double2(s * x01.x + c * t1.x, s * x01.y + c * t1.y);
-          x00 = n00;
-          x01 = n01;
-        }
-        if (on_b) {
-          const double c = rc[ib], s = rs[ib];
-          const double2 phc = make_double2(rph[ib].x, -rph[ib].y);
-          const double2 t0 = zmul(phc, x01), t1 = zmul(phc, x11);
-          const double2 n00 = make_double2(c * x00.x - s * t0.x, c * x00.y - s * t0.y);
-          const double2 n10 = make_double2(c * x10.x - s * t1.x, c * x10.y - s * t1.y);
-          x01 = make_double2(s * x00.x + c * t0.x, s * x00.y + c * t0.y);
-          x11 = make_double2(s * x10.x + c * t1.x, s * x10.y + c * t1.y);
-          x00 = n00;
-          x10 = n10;
-        }
-        // each entry goes to both copies of A
-        auto put = [&](int idx, double2 v) {
-          A[idx] = v;
-          Ap[idx] = v;
-        };
-        if (ia == ib) {
-          put(pa * n + pa, make_double2(x00.x, 0.0));
-          put(qa * n + qa, make_double2(x11.x, 0.0));
-          put(pa * n + qa, z);
-          put(qa * n + pa, z);
-          continue;
-        }
-        put(pa * n + pb, x00);
-        put(pb * n + pa, make_double2(x00.x, -x00.y));
-        if (qb_ok) {
-          put(pa * n + qb, x01);
-          put(qb * n + pa, make_double2(x01.x, -x01.y));
-        }
-        if (qa_ok) {
-          put(qa * n + pb, x10);
-          put(pb * n + qa, make_double2(x10.x, -x10.y));
-        }
-        if (qa_ok && qb_ok) {
-          put(qa * n + qb, x11);
-          put(qb * n + qa, make_double2(x11.x, -x11.y));
-        }
-      }
-      // eigenvector rows r0..r1 of this CTA
-      const int nr = r1 - r0;
-      for (int w = threadIdx.x; w < np * nr; w += blockDim.x) {
-        const int k = w / nr, row = w - (w / nr) * nr;
-        if (!act[k]) continue;
-        const VT c = (VT)rc[k], s = (VT)rs[k];
-        const VT phx = (VT)rph[k].x, phy = (VT)-rph[k].y;
-        V2 &xp = Vt[pp[k] * hv + row];
-        V2 &xq = Vt[pq[k] * hv + row];
-        const V2 a = xp, b = xq;
-        const VT tx = phx * b.x - phy * b.y, ty = phx * b.y + phy * b.x;
-        xp.x = c * a.x - s * tx;
-        xp.y = c * a.y - s * ty;
-        xq.x = s * a.x + c * tx;
-        xq.y = s * a.y + c * ty;
-      }
-      cluster.sync();   // both halves of the round written into both copies of A
-    }
-  }
-  if (threadIdx.x == 0 && crank == 0 && sweeps_out) sweeps_out[ksi] = sweep;
-  double *ev = rc;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) ev[i] = A[i * n + i].x;
-  __syncthreads();
-  double2 *Cb = Cout + mat_off[ksi];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double vi = ev[i];
-    int rank = 0;
-    for (int j = 0; j < n; ++j) rank += (ev[j] < vi) || (ev[j] == vi && j < i);
-    if (crank == 0) eig[K.item0 + rank] = vi;
-    for (int r = r0; r < r1; ++r) {
-      const V2 v = Vt[i * hv + (r - r0)];
-      Cb[r * n + rank] = make_double2((double)v.x, (double)v.y);
-    }
-  }
-  cluster.sync();   // neither CTA leaves while its partner could still address it
 }
 
 // ---------------------------------------------------------------------------
@@ -970,49 +1147,73 @@ void launch_cholesky_inv(const Tables &t, int ks_begin, int nks, int max_nb, con
   derek::note_launch(), k_cholesky_inv<<<nks, 256, sm, st>>>(t, ks_begin, S, C, mat_off, scratch, status, use_smem);
 }
 
-// shared memory of the Jacobi kernel: A (FP64) when it fits, the eigenvector
-// matrix when it also fits, and the pair and block tables
+// tables of the Jacobi kernels: two rounds' rotations and the block list
 static size_t jacobi_tables(int max_nb) {
   const size_t np = (size_t)(max_nb + 1) / 2;
-  return np * (sizeof(double2) + 2 * sizeof(double) + 3 * sizeof(int)) + np * (np + 1) / 2 * 4 + 64;
+  return 2 * jacobi_round_bytes(np) + np * (np + 1) / 2 * sizeof(short2);
 }
-constexpr size_t kJacobiSmem = 227 * 1024 - 4096;   // static reduction arrays take 4 KB
+static size_t jacobi_smem(int max_nb, int cs) {
+  const size_t hv = (size_t)(max_nb + cs - 1) / cs;
+  return (size_t)max_nb * (max_nb + hv) * sizeof(double2) + jacobi_tables(max_nb);
+}
+constexpr size_t kJacobiSmem = 227 * 1024 - 1024;   // beside the static reduction arrays
+
+template <int CS, int LPB, typename... Args>
+static void jacobi_go(int nks, size_t sm, cudaStream_t st, Args... args) {
+  auto kern = k_jacobi<CS, LPB>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(CS * nks);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CS;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = CS > 1 ? 1 : 0;
+  derek::note_launch();
+  cudaLaunchKernelEx(&cfg, kern, args...);
+}
 
 void launch_jacobi(const Tables &t, int ks_begin, int nks, int max_nb, const double2 *Hs,
                    double2 *C, const long long *mat_off, double *eig, double2 *scratch,
-                   int max_sweeps, double tol, int fp32_vectors, int *sweeps_out, cudaStream_t st,
-                   int single) {
+                   int max_sweeps, double tol, int *sweeps_out, cudaStream_t st, int single) {
   if (nks <= 0) return;
-  const size_t nn = (size_t)max_nb * max_nb;
-  const size_t tab = jacobi_tables(max_nb);
-  const size_t vbytes = (nn * (fp32_vectors ? sizeof(float2) : sizeof(double2)) + 15) / 16 * 16;
-  const int a_smem = nn * sizeof(double2) + tab <= kJacobiSmem;
-  const int v_smem = a_smem && nn * sizeof(double2) + vbytes + tab <= kJacobiSmem;
-  const size_t sm = (a_smem ? nn * sizeof(double2) : 0) + (v_smem ? vbytes : 0) + tab;
-  // two CTAs per k-set when A and half of the eigenvector rows fit
-  const size_t hv = (size_t)(max_nb + 1) / 2;
-  const size_t vhalf = ((size_t)max_nb * hv * (fp32_vectors ? sizeof(float2) : sizeof(double2)) + 15) / 16 * 16;
-  const size_t sm_pair = nn * sizeof(double2) + vhalf + tab;
-  if (!single && sm_pair <= kJacobiSmem) {
-    if (fp32_vectors) {
-      cudaFuncSetAttribute(k_jacobi_pair<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_pair);
-      derek::note_launch(), k_jacobi_pair<float><<<2 * nks, 256, sm_pair, st>>>(t, ks_begin, Hs, C, mat_off, eig,
-                                                                             max_sweeps, tol, sweeps_out);
-    } else {
-      cudaFuncSetAttribute(k_jacobi_pair<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_pair);
-      derek::note_launch(), k_jacobi_pair<double><<<2 * nks, 256, sm_pair, st>>>(t, ks_begin, Hs, C, mat_off, eig,
-                                                                              max_sweeps, tol, sweeps_out);
-    }
+  const int np = (max_nb + 1) / 2, nblk = np * (np + 1) / 2;
+  // CTAs per k-set: as many as leave each its own SM (128 of them: clusters
+  // do not fill every SM) and 16 blocks of a round; at least as many as make
+  // A and a slice of the eigenvectors fit
+  int cs = 1;
+  while (!single && cs < 8 && 2 * cs * nks <= 128 && nblk >= 32 * cs) cs *= 2;
+  while (cs < 8 && jacobi_smem(max_nb, cs) > kJacobiSmem) cs *= 2;
+  const size_t sm = jacobi_smem(max_nb, cs);
+  if (sm > kJacobiSmem) {
+    const size_t tab = jacobi_tables(max_nb);
+    derek::note_launch(), k_jacobi_global<<<nks, 256, tab, st>>>(t, ks_begin, Hs, C, mat_off, eig, scratch, max_sweeps,
+                                                                 tol, sweeps_out);
     return;
   }
-  if (fp32_vectors) {
-    cudaFuncSetAttribute(k_jacobi<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    derek::note_launch(), k_jacobi<float><<<nks, 256, sm, st>>>(t, ks_begin, Hs, C, mat_off, eig, scratch, max_sweeps,
-                                                                tol, a_smem, v_smem, sweeps_out);
-  } else {
-    cudaFuncSetAttribute(k_jacobi<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    derek::note_launch(), k_jacobi<double><<<nks, 256, sm, st>>>(t, ks_begin, Hs, C, mat_off, eig, scratch, max_sweeps,
-                                                                 tol, a_smem, v_smem, sweeps_out);
+  // one element per lane (16 FP64 operations) or one block per thread (48):
+  // whichever leaves the fullest quarter of the SM fewer
+  auto quarter = [&](int lanes) { return ((lanes + 31) / 32 + 3) / 4; };
+  const bool fine = quarter((4 * nblk + cs - 1) / cs) * 16 < quarter((nblk + cs - 1) / cs) * 48;
+  auto go = [&](auto csc, auto lc) {
+    jacobi_go<decltype(csc)::value, decltype(lc)::value>(nks, sm, st, t, ks_begin, Hs, C, mat_off, eig, max_sweeps, tol,
+                                                        sweeps_out);
+  };
+  auto pick = [&](auto csc) {
+    if (fine)
+      go(csc, std::integral_constant<int, 4>{});
+    else
+      go(csc, std::integral_constant<int, 1>{});
+  };
+  switch (cs) {
+    case 1: pick(std::integral_constant<int, 1>{}); break;
+    case 2: pick(std::integral_constant<int, 2>{}); break;
+    case 4: pick(std::integral_constant<int, 4>{}); break;
+    default: pick(std::integral_constant<int, 8>{}); break;
   }
 }
 

@@ -46,12 +46,10 @@ bool cholesky_fits_smem(int max_nb);
 void launch_cholesky_inv(const Tables &t, int ks_begin, int nks, int max_nb, const double2 *S,
                          double2 *C, const long long *mat_off, double2 *scratch, int *status,
                          cudaStream_t st);
-// fp32_vectors: accumulate the eigenvectors in FP32 (A stays FP64); single:
-// one CTA per k-set even where the two-CTA cluster kernel fits
+// single: one CTA per k-set wherever A and the eigenvectors fit one
 void launch_jacobi(const Tables &t, int ks_begin, int nks, int max_nb, const double2 *Hs,
                    double2 *C, const long long *mat_off, double *eig, double2 *scratch,
-                   int max_sweeps, double tol, int fp32_vectors, int *sweeps_out, cudaStream_t st,
-                   int single = 0);
+                   int max_sweeps, double tol, int *sweeps_out, cudaStream_t st, int single = 0);
 
 // Per-system SCF scalars kept on the device.
 constexpr int kMaxHist = 16;

@@ -95,3 +95,29 @@ def test_rotations_at_every_band_count(oracle, nb, precision, eig_tol, tol):
         (eig,), _ = h.nscf(max_iter=300, eig_tol=eig_tol, nconv=nconv)
     ref = dense_eigenvalues(oracle, s, 0, s.vext, nconv)
     assert np.max(np.abs(eig[0, :nconv] - ref)) < tol
+
+
+# Jacobi solves on one CTA and on clusters of 2, 4 and 8, one element per lane and
+# one block per thread, odd counts, subspaces in shared memory and in global
+# scratch: the Ritz vectors diagonalise the projected Hamiltonian
+@pytest.mark.parametrize("nb,nk", [(2, 1), (5, 3), (16, 1), (23, 2), (23, 40), (44, 1), (44, 70), (84, 1), (85, 20),
+                                   (115, 2), (128, 1)])
+def test_jacobi_solves(oracle, nb, nk):
+    import derek_gb300 as dg
+    from test_gpu_primitives import make_pair
+    kpts = [(0.1 + 0.005 * i, 0.2, -0.3 + 0.004 * i) for i in range(nk)]
+    s, spec = make_pair(oracle, L=8.0, ecut=4.0, nb=nb, nelec=1.0, kpts=kpts, seed=nb)
+    with dg.Handle(spec, precision=0, buffer_bands=0, init_vectors=1, use_tensor_cores=0) as h:
+        h.set_vloc(s.vext)
+        try:
+            h.nscf(max_iter=2, eig_tol=1e-12)
+        except dg.DerekError:
+            pass   # two iterations do not converge; the Ritz pairs are exact in their subspace
+        eig = h.eigenvalues()
+        for k in sorted({0, nk - 1}):
+            psi = h.get_wfn(0, k)
+            hpsi = h.pot_apply_wfn(0, k)
+            hs = psi.conj() @ hpsi.T
+            # Ritz vectors diagonalise H: rounding times ||H|| ~ 20 Ha
+            assert np.max(np.abs(hs - np.diag(eig[k]))) < 1e-10
+            assert np.all(np.diff(eig[k]) >= 0)
