@@ -34,6 +34,52 @@ template <typename R> __host__ __device__ __forceinline__ cplx<R> cmulc(cplx<R> 
 template <typename R> __host__ __device__ __forceinline__ cplx<R> cscale(cplx<R> a, R s) {
   return mk<R>(a.x * s, a.y * s);
 }
+// a s + b (real s), fused
+template <typename R> __device__ __forceinline__ cplx<R> caxpy(cplx<R> a, R s, cplx<R> b);
+template <> __device__ __forceinline__ double2 caxpy<double>(double2 a, double s, double2 b) {
+  return make_double2(fma(a.x, s, b.x), fma(a.y, s, b.y));
+}
+// SIGN i (a - b)
+template <typename R, int SIGN> __device__ __forceinline__ cplx<R> csub_si(cplx<R> a, cplx<R> b) {
+  return SIGN > 0 ? mk<R>(b.y - a.y, a.x - b.x) : mk<R>(a.y - b.y, b.x - a.x);
+}
+
+// Complex FP32 additions and real multiples as packed pairs: one issue slot
+// instead of two (the multiply-add pipe's rate is the same).  The register-line
+// transforms are bound by issue, and their values sit in aligned register pairs
+// anyway.  Each half rounds as the scalar operation does.  Multiplications by
+// +-i swap the halves, so they stay two scalar operations (csub_si).
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ unsigned long long pack2(float2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+template <> __device__ __forceinline__ float2 cadd<float>(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+  return unpack2(r);
+}
+template <> __device__ __forceinline__ float2 csub<float>(float2 a, float2 b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+  return unpack2(r);
+}
+#endif
+template <> __device__ __forceinline__ float2 caxpy<float>(float2 a, float s, float2 b) {
+#ifdef __CUDA_ARCH__
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(make_float2(s, s))), "l"(pack2(b)));
+  return unpack2(r);
+#else
+  return make_float2(a.x * s + b.x, a.y * s + b.y);
+#endif
+}
 
 constexpr int kMaxRadices = 8;
 constexpr int kMaxDim = 128;       // largest FFT length along one axis

@@ -272,12 +272,12 @@ template <typename R_, int SIGN> __device__ __forceinline__ cplx<R_> mul_si(cplx
 template <typename R_, int SIGN> struct Dft<R_, 3, SIGN> {
   __device__ __forceinline__ static void run(cplx<R_> *v) {
     const R_ h = (R_)0.86602540378443864676;  // sqrt(3)/2
-    cplx<R_> t1 = cadd<R_>(v[1], v[2]);
-    cplx<R_> t2 = cscale<R_>(mul_si<R_, SIGN>(csub<R_>(v[1], v[2])), h);
-    cplx<R_> m = mk<R_>(v[0].x - (R_)0.5 * t1.x, v[0].y - (R_)0.5 * t1.y);
+    const cplx<R_> t1 = cadd<R_>(v[1], v[2]);
+    const cplx<R_> t2 = csub_si<R_, SIGN>(v[1], v[2]);
+    const cplx<R_> m = caxpy<R_>(t1, (R_)-0.5, v[0]);
     v[0] = cadd<R_>(v[0], t1);
-    v[1] = cadd<R_>(m, t2);
-    v[2] = csub<R_>(m, t2);
+    v[1] = caxpy<R_>(t2, h, m);
+    v[2] = caxpy<R_>(t2, -h, m);
   }
 };
 
@@ -286,7 +286,7 @@ template <typename R_, int SIGN> struct Dft<R_, 4, SIGN> {
     cplx<R_> a = cadd<R_>(v[0], v[2]);
     cplx<R_> b = csub<R_>(v[0], v[2]);
     cplx<R_> c = cadd<R_>(v[1], v[3]);
-    cplx<R_> d = mul_si<R_, SIGN>(csub<R_>(v[1], v[3]));
+    cplx<R_> d = csub_si<R_, SIGN>(v[1], v[3]);
     v[0] = cadd<R_>(a, c);
     v[2] = csub<R_>(a, c);
     v[1] = cadd<R_>(b, d);
@@ -308,12 +308,12 @@ template <typename R_, int SIGN> struct Dft<R_, 8, SIGN> {
     const cplx<R_> o3 = SIGN > 0 ? mk<R_>(-o[3].x - o[3].y, o[3].x - o[3].y) : mk<R_>(o[3].y - o[3].x, -o[3].x - o[3].y);
     v[0] = cadd<R_>(e[0], o[0]);
     v[4] = csub<R_>(e[0], o[0]);
-    v[1] = mk<R_>(e[1].x + r * o1.x, e[1].y + r * o1.y);
-    v[5] = mk<R_>(e[1].x - r * o1.x, e[1].y - r * o1.y);
-    v[2] = cadd<R_>(e[2], o2);
-    v[6] = csub<R_>(e[2], o2);
-    v[3] = mk<R_>(e[3].x + r * o3.x, e[3].y + r * o3.y);
-    v[7] = mk<R_>(e[3].x - r * o3.x, e[3].y - r * o3.y);
+    v[1] = caxpy<R_>(o1, r, e[1]);
+    v[5] = caxpy<R_>(o1, -r, e[1]);
+    v[2] = mk<R_>(e[2].x + o2.x, e[2].y + o2.y);
+    v[6] = mk<R_>(e[2].x - o2.x, e[2].y - o2.y);
+    v[3] = caxpy<R_>(o3, r, e[3]);
+    v[7] = caxpy<R_>(o3, -r, e[3]);
   }
 };
 

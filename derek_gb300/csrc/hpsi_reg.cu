@@ -2,7 +2,7 @@
 // registers (regfft.cuh).
 //
 // A block works on XP consecutive x-planes: of one k-set, band after band
-// (density), or of a sequence of items (apply H, one block per SM keeping its
+// (density), or of a sequence of items (apply H, resident blocks keeping their
 // group of x-planes and its V(r) planes).  Each plane sits in shared memory
 // as the rows of centred Miller
 // index my in [-RY, RY] (row my + RY), PZ elements per row: the rows a
@@ -25,7 +25,7 @@
 namespace derek {
 
 // ---- H.psi (y,z) pass ----------------------------------------------------------
-// Block b keeps x-group g = b mod ng and walks the items r, r + R, ... with
+// One or two resident blocks per SM.  Block b keeps x-group g = b mod ng and walks the items r, r + R, ... with
 // r = b div ng, R = gridDim.x / ng.  Its V(r) planes stay in shared memory
 // while consecutive items belong to the same system.  While the forward z
 // transforms of a tile run (most threads idle), the threads without a z line
@@ -83,7 +83,7 @@ __device__ __forceinline__ void stage_offsets(const Tables &t, int item_begin, i
 constexpr int kPrefetchValues = 32;
 
 template <int N, int RY, int XP, int NT>
-__global__ void __launch_bounds__(NT, 1) k_plane_persist(Tables t, int item_begin, int nitems, int ng,
+__global__ void __launch_bounds__(NT, kThreadsMax / NT) k_plane_persist(Tables t, int item_begin, int nitems, int ng,
                                                          float2 *__restrict__ abuf,
                                                          const float *__restrict__ vloc) {
   using Lay = RowsLayout<N, RY>;
@@ -299,15 +299,21 @@ static void plane_persist_go(const Tables &t, int item_begin, int nitems, int ma
   using Lay = RowsLayout<N, RY>;
   constexpr size_t OFFS = 2 * (size_t)(Lay::NRW * Lay::NRW + Lay::NRW) * sizeof(short);
   constexpr int PLANE = Lay::PP * 8 + Lay::VP * 4;
-  constexpr int BYS = (int)((kSmemMax - 256 - OFFS) / PLANE);
-  constexpr int XP0 = BYS < kThreadsMax / N ? BYS : kThreadsMax / N;
+  // Two blocks of 192 threads per SM up to N = 48, whose barriers overlap; one
+  // of 384 above, where 192 threads hold two or three planes and leave lanes
+  // idle.  One launch, two blocks against one: N = 32 8.6 / 10.9 us (12 items),
+  // 48 245 / 274 us (960 items), 54 346 / 264, 64 547 / 516, 72 6.4 / 5.1 ms.
+  constexpr int CAP = N <= 48 ? kThreadsMax / 2 : kThreadsMax;
+  constexpr int BPS = kThreadsMax / CAP;
+  constexpr int BYS = (int)((kSmemMax / BPS - 1280 - OFFS) / PLANE);
+  constexpr int XP0 = BYS < CAP / N ? BYS : CAP / N;
   constexpr int XP = XP0 < 1 ? 1 : XP0;
   constexpr int NT = (N * XP + 31) / 32 * 32;
   const size_t smem = (size_t)XP * PLANE + OFFS + 16;
   auto kern = k_plane_persist<N, RY, XP, NT>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const int ng = (max_n1 + XP - 1) / XP;
-  int R = sm_count() / ng;
+  int R = kThreadsMax / NT * sm_count() / ng;
   if (R < 1) R = 1;
   if (R > nitems) R = nitems;
   derek::note_launch(), kern<<<ng * R, NT, smem, st>>>(t, item_begin, nitems, ng, abuf, vloc);

@@ -126,6 +126,14 @@ template <typename R_, bool A, bool B> __device__ __forceinline__ cplx<R_> zsub(
     return mk<R_>((R_)0, (R_)0);
 }
 
+// SIGN i (a - b) with a or b a compile-time zero
+template <typename R_, int SIGN, bool A, bool B> __device__ __forceinline__ cplx<R_> zsub_si(cplx<R_> a, cplx<R_> b) {
+  if constexpr (A && B)
+    return csub_si<R_, SIGN>(a, b);
+  else
+    return mul_si<R_, SIGN>(zsub<R_, A, B>(a, b));
+}
+
 // a * exp(SIGN 2 pi i m / R); the quarter turns are exact moves
 template <typename R_, int R, int SIGN, int M0> __device__ __forceinline__ cplx<R_> turn(cplx<R_> a) {
   constexpr int m = ((M0 % R) + R) % R;
@@ -170,15 +178,15 @@ template <typename R_, int SIGN, unsigned M> struct DftZPart<R_, 3, SIGN, M> {
     constexpr bool a = dz_bit(M, 0), b = dz_bit(M, 1), c = dz_bit(M, 2);
     const R_ h = (R_)0.86602540378443864676;  // sqrt(3)/2
     const cplx<R_> t1 = zadd<R_, b, c>(v[1], v[2]);
-    const cplx<R_> t2 = cscale<R_>(mul_si<R_, SIGN>(zsub<R_, b, c>(v[1], v[2])), h);
+    const cplx<R_> t2 = zsub_si<R_, SIGN, b, c>(v[1], v[2]);
     cplx<R_> m;
     if constexpr (a)
-      m = mk<R_>(v[0].x - (R_)0.5 * t1.x, v[0].y - (R_)0.5 * t1.y);
+      m = caxpy<R_>(t1, (R_)-0.5, v[0]);
     else
       m = mk<R_>((R_)-0.5 * t1.x, (R_)-0.5 * t1.y);
     v[0] = zadd<R_, a, true>(v[0], t1);
-    v[1] = cadd<R_>(m, t2);
-    v[2] = csub<R_>(m, t2);
+    v[1] = caxpy<R_>(t2, h, m);
+    v[2] = caxpy<R_>(t2, -h, m);
   }
 };
 
@@ -190,7 +198,7 @@ template <typename R_, int SIGN, unsigned M> struct DftZPart<R_, 4, SIGN, M> {
     const cplx<R_> a = zadd<R_, b0, b2>(v[0], v[2]);
     const cplx<R_> b = zsub<R_, b0, b2>(v[0], v[2]);
     const cplx<R_> c = zadd<R_, b1, b3>(v[1], v[3]);
-    const cplx<R_> d = mul_si<R_, SIGN>(zsub<R_, b1, b3>(v[1], v[3]));
+    const cplx<R_> d = zsub_si<R_, SIGN, b1, b3>(v[1], v[3]);
     v[0] = zadd<R_, e, o>(a, c);
     v[2] = zsub<R_, e, o>(a, c);
     v[1] = zadd<R_, e, o>(b, d);
@@ -208,20 +216,29 @@ template <typename R_, int SIGN, unsigned M> struct DftZPart<R_, 8, SIGN, M> {
     cplx<R_> o[4] = {v[1], v[3], v[5], v[7]};
     DftZ<R_, 4, SIGN, me>::run(e);
     DftZ<R_, 4, SIGN, mo>::run(o);
+    // as Dft<8>: sqrt(1/2) of the eighth turns goes into the combination
     const R_ r = (R_)0.70710678118654752440;
-    const cplx<R_> w1 = mk<R_>(r, (R_)SIGN * r);
-    const cplx<R_> w3 = mk<R_>(-r, (R_)SIGN * r);
-    const cplx<R_> o1 = cmul<R_>(o[1], w1);
+    const cplx<R_> o1 = SIGN > 0 ? mk<R_>(o[1].x - o[1].y, o[1].x + o[1].y) : mk<R_>(o[1].x + o[1].y, o[1].y - o[1].x);
     const cplx<R_> o2 = mul_si<R_, SIGN>(o[2]);
-    const cplx<R_> o3 = cmul<R_>(o[3], w3);
+    const cplx<R_> o3 = SIGN > 0 ? mk<R_>(-o[3].x - o[3].y, o[3].x - o[3].y) : mk<R_>(o[3].y - o[3].x, -o[3].x - o[3].y);
     v[0] = zadd<R_, E, O>(e[0], o[0]);
     v[4] = zsub<R_, E, O>(e[0], o[0]);
-    v[1] = zadd<R_, E, O>(e[1], o1);
-    v[5] = zsub<R_, E, O>(e[1], o1);
-    v[2] = zadd<R_, E, O>(e[2], o2);
-    v[6] = zsub<R_, E, O>(e[2], o2);
-    v[3] = zadd<R_, E, O>(e[3], o3);
-    v[7] = zsub<R_, E, O>(e[3], o3);
+    if constexpr (E && O) {
+      v[1] = caxpy<R_>(o1, r, e[1]);
+      v[5] = caxpy<R_>(o1, -r, e[1]);
+      v[2] = mk<R_>(e[2].x + o2.x, e[2].y + o2.y);
+      v[6] = mk<R_>(e[2].x - o2.x, e[2].y - o2.y);
+      v[3] = caxpy<R_>(o3, r, e[3]);
+      v[7] = caxpy<R_>(o3, -r, e[3]);
+    } else {
+      const cplx<R_> s1 = cscale<R_>(o1, r), s3 = cscale<R_>(o3, r);
+      v[1] = zadd<R_, E, O>(e[1], s1);
+      v[5] = zsub<R_, E, O>(e[1], s1);
+      v[2] = zadd<R_, E, O>(e[2], o2);
+      v[6] = zsub<R_, E, O>(e[2], o2);
+      v[3] = zadd<R_, E, O>(e[3], s3);
+      v[7] = zsub<R_, E, O>(e[3], s3);
+    }
   }
 };
 
