@@ -625,7 +625,7 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
     CK(upload(&h->d_cells, cells));
     CK(upload(&h->d_wells, h->wells_host));
     CK(upload(&h->d_well_off, h->well_off));
-    CK(cudaMalloc((void **)&h->d_hfpart, (size_t)nsys * 64 * std::max(h->max_wells, 1) * 5 * sizeof(double)));
+    CK(cudaMalloc((void **)&h->d_hfpart, (size_t)nsys * kRedBlocks * std::max(h->max_wells, 1) * 5 * sizeof(double)));
     CK(cudaMalloc((void **)&h->d_hfgrad, std::max<size_t>(h->wells_host.size(), 1) * sizeof(double)));
   }
   const size_t gbytes = (size_t)grid_off * sizeof(double);

@@ -99,6 +99,7 @@ struct derek_gpu {
   double *d_epart = nullptr, *d_gpart = nullptr;
   int hist = 8;
   int max_npw = 0;
+  int max_states = 0;                          // most (k-point, reported band) states of a system
   int split_min = 512;                         // smallest overlap split d_opart holds
   long long max_nr = 0;
   int cur = 0;                                 // psi buffer holding the current subspace

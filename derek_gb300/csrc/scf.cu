@@ -150,7 +150,7 @@ bool reject_mixed(derek_gpu *h, const char *what) {
 
 int finish_iteration(derek_gpu *h) {
   const SpinGrids sg = spin_grids(h);
-  launch_occupations(h->tab_band, h->nsys, h->d_eig, h->d_occ, h->d_occw, h->d_state, h->stream);
+  launch_occupations(h->tab_band, h->nsys, h->max_states, h->d_eig, h->d_occ, h->d_occw, h->d_state, h->stream);
   int st = sg.on ? density_spinor_items(h, h->cur_psi(), h->d_rho_out)
                  : density_items(h, h->cur_psi(), h->d_rho_out);
   if (st) return st;
@@ -387,6 +387,7 @@ extern "C" int derek_scf_alloc(derek_gpu_t *h) {
     hist_off.push_back(hoff);
     hoff += (long long)h->hist * S.nr;
     h->max_nr = std::max<long long>(h->max_nr, S.nr);
+    h->max_states = std::max(h->max_states, S.nbr / S.nspinor * S.nk);
   }
   cudaError_t e;
 #define A(call)                                                  \
@@ -406,8 +407,8 @@ extern "C" int derek_scf_alloc(derek_gpu_t *h) {
   A(dalloc(&h->d_coef_all, (size_t)h->max_degree * h->nks));
   A(dalloc(&h->d_nin_hist, hoff));
   A(dalloc(&h->d_res_hist, hoff));
-  A(dalloc(&h->d_epart, (size_t)h->nsys * 64 * 8));
-  A(dalloc(&h->d_gpart, (size_t)h->nsys * 64 * kMaxHist));
+  A(dalloc(&h->d_epart, (size_t)h->nsys * kRedBlocks * 8));
+  A(dalloc(&h->d_gpart, (size_t)h->nsys * kRedBlocks * kMaxHist));
   if (h->all_spinor) {
     A(dalloc(&h->d_mag_in, 3 * (size_t)h->total_grid));
     A(dalloc(&h->d_bxc, 3 * (size_t)h->total_grid));

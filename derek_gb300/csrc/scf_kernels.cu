@@ -15,36 +15,68 @@
 
 namespace derek {
 
-constexpr int RB = 64;  // reduction blocks per system
+constexpr int RB = kRedBlocks;
 constexpr int EP = 8;   // partial slots per block: 0-2 energies, 3 residual, 4 V max
 
+// lane sums by a fixed butterfly: every lane gets the total
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) v += __shfl_xor_sync(0xffffffffu, v, w);
+  return v;
+}
+__device__ __forceinline__ double warp_max(double v) {
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, w));
+  return v;
+}
+// block total in every thread (red: one slot per warp); one warp needs no
+// barrier at all
 __device__ __forceinline__ double block_sum(double v, double *red) {
-  red[threadIdx.x] = v;
+  v = warp_sum(v);
+  const int nw = (blockDim.x + 31) >> 5, lane = threadIdx.x & 31;
+  if (nw == 1) return v;
+  if (lane == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
-  }
-  const double r = red[0];
+  v = warp_sum(lane < nw ? red[lane] : 0.0);
   __syncthreads();
-  return r;
+  return v;
+}
+__device__ __forceinline__ double block_max(double v, double *red) {
+  v = warp_max(v);
+  const int nw = (blockDim.x + 31) >> 5, lane = threadIdx.x & 31;
+  if (nw == 1) return v;
+  if (lane == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = warp_max(lane < nw ? red[lane] : red[0]);
+  __syncthreads();
+  return v;
 }
 
-__device__ __forceinline__ double gsq(const SysDev &S, long long r) {
-  const int n1 = S.n[0], n2 = S.n[1], n3 = S.n[2];
-  const int iz = (int)(r % n3);
-  const int iy = (int)((r / n3) % n2);
-  const int ix = (int)(r / ((long long)n2 * n3));
-  const double m0 = ix < n1 - n1 / 2 ? ix : ix - n1;
-  const double m1 = iy < n2 - n2 / 2 ? iy : iy - n2;
-  const double m2 = iz < n3 - n3 / 2 ? iz : iz - n3;
-  double g2 = 0.0;
-  for (int i = 0; i < 3; ++i) {
-    const double g = S.B[3 * i] * m0 + S.B[3 * i + 1] * m1 + S.B[3 * i + 2] * m2;
-    g2 += g * g;
+// |G|^2 = m^T W m of grid point r, W = B^T B.  Exactly zero at G = 0.
+struct Metric {
+  double w00, w01, w02, w11, w12, w22;
+  __device__ __forceinline__ explicit Metric(const SysDev &S) {
+    w00 = w01 = w02 = w11 = w12 = w22 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double x = S.B[3 * i], y = S.B[3 * i + 1], z = S.B[3 * i + 2];
+      w00 += x * x;
+      w01 += 2.0 * x * y;
+      w02 += 2.0 * x * z;
+      w11 += y * y;
+      w12 += 2.0 * y * z;
+      w22 += z * z;
+    }
   }
-  return g2;
-}
+  __device__ __forceinline__ double gsq(const SysDev &S, int r) const {
+    const int n1 = S.n[0], n2 = S.n[1], n3 = S.n[2];
+    const int q = r / n3, iz = r - q * n3, ix = q / n2, iy = q - ix * n2;
+    const double m0 = ix < n1 - n1 / 2 ? ix : ix - n1;
+    const double m1 = iy < n2 - n2 / 2 ? iy : iy - n2;
+    const double m2 = iz < n3 - n3 / 2 ? iz : iz - n3;
+    return m0 * (w00 * m0 + w01 * m1 + w02 * m2) + m1 * (w11 * m1 + w12 * m2) + w22 * m2 * m2;
+  }
+};
 
 // ---- start vectors: real r - 0.5 per (band, G) like wave_initialise_wfn
 // (Source/wave.f90:873-886), from a splitmix64 counter hash
@@ -104,14 +136,17 @@ __global__ void k_filter_coef(const Tables t, int nks, const double *__restrict_
   }
 }
 
-// ---- Fermi-Dirac occupations, one block per system
+// ---- Fermi-Dirac occupations, one block per system (8 states: 88 -> 29 us).  As
+// few warps as hold the states (one warp needs no barrier in its sums): the FP64 chain of a Newton
+// step, an exponential and a division, is the same for any count.  States are
+// dealt band by band over the k-points, and a warp whose states all lie more
+// than 45 kT from mu leaves the exponential out: f is 1 or below 3e-20 there,
+// either way exact to the last bit of the sum.
 __global__ void __launch_bounds__(1024) k_occupations(const Tables t, const double *__restrict__ eig,
                                                       double *__restrict__ occ,
                                                       double *__restrict__ occw,
                                                       SysState *__restrict__ st) {
-  __shared__ double red[1024];
-  __shared__ double s_lo, s_hi, s_mu;
-  __shared__ int s_done;
+  __shared__ double red[32];
   const int s = blockIdx.x;
   const SysDev &S = t.sys[s];
   if (!S.active) return;
@@ -122,109 +157,95 @@ __global__ void __launch_bounds__(1024) k_occupations(const Tables t, const doub
   const double g = nsp == 2 ? 1.0 : 2.0;
   const int nb = S.nbr / nsp, nk = S.nk;
   const int ntot = nb * nk;
-  const double kT = S.kT, ne = S.nelec;
-  // bracket
-  double lo = 1e300, hi = -1e300;
-  for (int i = threadIdx.x; i < ntot; i += blockDim.x) {
-    const KSetDev &K = t.ks[S.ks0 + i / nb];
-    const double e = eig[K.item0 + i % nb];
-    lo = fmin(lo, e);
-    hi = fmax(hi, e);
-  }
-  red[threadIdx.x] = lo;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] = fmin(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) s_lo = red[0] - 40.0 * kT - 1.0;
-  __syncthreads();
-  red[threadIdx.x] = hi;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    s_hi = red[0] + 40.0 * kT + 1.0;
-    // from the previous SCF iteration's Fermi level when there is one (the
-    // state is reset at SCF start, so every run takes the same path)
-    const double prev = st[s].mu;
-    s_mu = st[s].iter > 0 && prev > s_lo && prev < s_hi ? prev : 0.5 * (s_lo + s_hi);
-    s_done = 0;
-  }
+  const double kT = S.kT, ne = S.nelec, ikT = 1.0 / kT;
+  const int tid = threadIdx.x, nt = blockDim.x;
   // each thread's eigenvalues and weights in registers (up to kOccReg per
   // thread), read once instead of once per Newton step
   constexpr int kOccReg = 6;
-  const bool in_reg = ntot <= kOccReg * (int)blockDim.x;
-  // slots of this thread: i = threadIdx.x + q blockDim.x < ntot for q < nq
-  const int nq = (int)threadIdx.x < ntot ? (ntot - 1 - (int)threadIdx.x) / (int)blockDim.x + 1 : 0;
+  const bool in_reg = ntot <= kOccReg * nt;
+  auto state = [&](int i, double &e, double &w) {   // state i: band i / nk of k-point i % nk
+    const int b = i / nk;
+    const KSetDev &K = t.ks[S.ks0 + i - b * nk];
+    e = eig[K.item0 + b];
+    w = K.wk * g;
+  };
   double er[kOccReg], wr[kOccReg];
+  double lo = 1e300, hi = -1e300;
 #pragma unroll
   for (int q = 0; q < kOccReg; ++q) {
-    const int i = threadIdx.x + q * (int)blockDim.x;
-    er[q] = 0.0;
+    er[q] = 1e300;
     wr[q] = 0.0;
-    if (in_reg && q < nq) {
-      const KSetDev &K = t.ks[S.ks0 + i / nb];
-      er[q] = eig[K.item0 + i % nb];
-      wr[q] = K.wk * g;
+    const int i = tid + q * nt;
+    if (in_reg && i < ntot) {
+      state(i, er[q], wr[q]);
+      lo = fmin(lo, er[q]);
+      hi = fmax(hi, er[q]);
     }
   }
-  __syncthreads();
-  // safeguarded Newton on N(mu) - Ne
+  if (!in_reg)
+    for (int i = tid; i < ntot; i += nt) {
+      double e, w;
+      state(i, e, w);
+      lo = fmin(lo, e);
+      hi = fmax(hi, e);
+    }
+  double s_lo = -block_max(-lo, red) - 40.0 * kT - 1.0;
+  double s_hi = block_max(hi, red) + 40.0 * kT + 1.0;
+  // from the previous SCF iteration's Fermi level when there is one (the
+  // state is reset at SCF start, so every run takes the same path)
+  const double prev = st[s].mu;
+  double mu = st[s].iter > 0 && prev > s_lo && prev < s_hi ? prev : 0.5 * (s_lo + s_hi);
+  // safeguarded Newton on N(mu) - Ne; every thread holds the totals and takes
+  // the same step
   for (int it = 0; it < 200; ++it) {
-    const double mu = s_mu;
     double cnt = 0, der = 0;
+    auto add = [&](double e, double w) {
+      const double x = (e - mu) * ikT;
+      const bool near = fabs(x) < 45.0;
+      if (__any_sync(__activemask(), near)) {
+        const double f = 1.0 / (1.0 + exp(fmin(fmax(x, -200.0), 200.0)));
+        cnt += w * f;
+        der += w * f * (1.0 - f) * ikT;
+      } else if (x < 0) {
+        cnt += w;
+      }
+    };
     if (in_reg) {
 #pragma unroll
-      for (int q = 0; q < kOccReg; ++q) {
-        if (q < nq) {
-          const double x = fmin(fmax((er[q] - mu) / kT, -200.0), 200.0);
-          const double f = 1.0 / (1.0 + exp(x));
-          cnt += wr[q] * f;
-          der += wr[q] * f * (1.0 - f) / kT;
-        }
-      }
+      for (int q = 0; q < kOccReg; ++q)
+        if (q * nt < ntot) add(er[q], wr[q]);
     } else {
-      for (int i = threadIdx.x; i < ntot; i += blockDim.x) {
-        const KSetDev &K = t.ks[S.ks0 + i / nb];
-        const double x = fmin(fmax((eig[K.item0 + i % nb] - mu) / kT, -200.0), 200.0);
-        const double f = 1.0 / (1.0 + exp(x));
-        cnt += K.wk * g * f;
-        der += K.wk * g * f * (1.0 - f) / kT;
+      for (int i = tid; i < ntot; i += nt) {
+        double e, w;
+        state(i, e, w);
+        add(e, w);
       }
     }
     cnt = block_sum(cnt, red);
     der = block_sum(der, red);
-    if (threadIdx.x == 0) {
-      const double r = cnt - ne;
-      if (r < 0)
-        s_lo = mu;
-      else
-        s_hi = mu;
-      double nmu = der > 0 ? mu - r / der : 0.5 * (s_lo + s_hi);
-      if (!(nmu > s_lo && nmu < s_hi)) nmu = 0.5 * (s_lo + s_hi);
-      if (fabs(r) <= 1e-14 * ne || (s_hi - s_lo) <= 1e-15 * fmax(1.0, fabs(mu))) s_done = 1;
-      s_mu = s_done ? mu : nmu;
-    }
-    __syncthreads();
-    if (s_done) break;
+    const double r = cnt - ne;
+    if (r < 0)
+      s_lo = mu;
+    else
+      s_hi = mu;
+    if (fabs(r) <= 1e-14 * ne || (s_hi - s_lo) <= 1e-15 * fmax(1.0, fabs(mu))) break;
+    double nmu = der > 0 ? mu - r / der : 0.5 * (s_lo + s_hi);
+    if (!(nmu > s_lo && nmu < s_hi)) nmu = 0.5 * (s_lo + s_hi);
+    mu = nmu;
   }
-  const double mu = s_mu;
   // S.nb items per k-set (both components of a spinor band are items)
-  for (int i = threadIdx.x; i < nk * S.nb; i += blockDim.x) {
+  for (int i = tid; i < nk * S.nb; i += nt) {
     const KSetDev &K = t.ks[S.ks0 + i / S.nb];
     occ[K.item0 + i % S.nb] = 0.0;
     occw[K.item0 + i % S.nb] = 0.0;
   }
   __syncthreads();
   double ent = 0, eb = 0;
-  for (int i = threadIdx.x; i < ntot; i += blockDim.x) {
-    const KSetDev &K = t.ks[S.ks0 + i / nb];
-    const int j = i % nb;
+  for (int i = tid; i < ntot; i += nt) {
+    const int j = i / nk;
+    const KSetDev &K = t.ks[S.ks0 + i - j * nk];
     const double e = eig[K.item0 + j];
-    const double x = fmin(fmax((e - mu) / kT, -200.0), 200.0);
+    const double x = fmin(fmax((e - mu) * ikT, -200.0), 200.0);
     const double f = 1.0 / (1.0 + exp(x));
     occ[K.item0 + j] = g * f;
     if (nsp == 2) {
@@ -251,7 +272,7 @@ __global__ void __launch_bounds__(256) k_energy_partials(const Tables t, const d
                                                          const double *__restrict__ rho_out,
                                                          const double2 *__restrict__ cgrid,
                                                          double *__restrict__ part, const SpinGrids sg) {
-  __shared__ double red[256];
+  __shared__ double red[8];
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
   if (!S.active) return;
@@ -259,6 +280,7 @@ __global__ void __launch_bounds__(256) k_energy_partials(const Tables t, const d
   const long long chunk = (n + RB - 1) / RB;
   const long long r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
   double q0 = 0, q1 = 0, q2 = 0, q3 = 0;
+  const Metric metric(S);
   for (long long r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
     const double nr = rho_out[S.grid_off + r];
     q3 = fmax(q3, fabs(nr - rho_in[S.grid_off + r]));
@@ -282,7 +304,7 @@ __global__ void __launch_bounds__(256) k_energy_partials(const Tables t, const d
       lda_point(nr, e, v);
     }
     q1 += nr * e;
-    const double g2 = gsq(S, r);
+    const double g2 = metric.gsq(S, (int)r);
     if (g2 > 0) {
       const double2 c = cgrid[S.grid_off + r];
       q2 += (c.x * c.x + c.y * c.y) / g2;
@@ -291,36 +313,42 @@ __global__ void __launch_bounds__(256) k_energy_partials(const Tables t, const d
   q0 = block_sum(q0, red);
   q1 = block_sum(q1, red);
   q2 = block_sum(q2, red);
-  red[threadIdx.x] = q3;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
+  q3 = block_max(q3, red);
   if (threadIdx.x == 0) {
     double *p = part + ((long long)s * RB + blockIdx.x) * EP;
     p[0] = q0;
     p[1] = q1;
     p[2] = q2;
-    p[3] = red[0];
+    p[3] = q3;
   }
 }
 
-__global__ void k_energy_final(const Tables t, int nsys, const double *__restrict__ part,
+// one warp per system; lanes share the partial sums
+__global__ void __launch_bounds__(32) k_energy_final(const Tables t, int nsys, const double *__restrict__ part,
                                SysState *__restrict__ st, SysDev *__restrict__ sys_rw,
                                const int *__restrict__ ks_status) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys) return;
+  const int s = blockIdx.x;
   const SysDev &S = t.sys[s];
   if (!S.active) return;
   double q0 = 0, q1 = 0, q2 = 0, q3 = 0;
-  for (int b = 0; b < RB; ++b) {
+  for (int b = threadIdx.x; b < RB; b += 32) {
     const double *p = part + ((long long)s * RB + b) * EP;
     q0 += p[0];
     q1 += p[1];
     q2 += p[2];
     q3 = fmax(q3, p[3]);
   }
+  q0 = warp_sum(q0);
+  q1 = warp_sum(q1);
+  q2 = warp_sum(q2);
+  q3 = warp_max(q3);
+  int status = 0;
+  for (int k = threadIdx.x; k < S.nk; k += 32)
+    if (ks_status[S.ks0 + k]) status = ks_status[S.ks0 + k];
+  // the last k-set with a status of its own
+  const unsigned bad = __ballot_sync(0xffffffffu, status != 0);
+  status = bad ? __shfl_sync(0xffffffffu, status, 31 - __clz(bad)) : 0;
+  if (threadIdx.x) return;
   const double dv = S.volume / S.nr;
   const double four_pi = 12.566370614359172953850573533118;
   SysState &X = st[s];
@@ -334,9 +362,6 @@ __global__ void k_energy_final(const Tables t, int nsys, const double *__restric
   X.delta = X.iter > 1 ? fabs(F - X.free) : 1e300;
   X.free_prev = X.free;
   X.free = F;
-  int status = 0;
-  for (int k = 0; k < S.nk; ++k)
-    if (ks_status[S.ks0 + k]) status = ks_status[S.ks0 + k];
   // a k-set's own failure (a wait that timed out, a singular overlap) is
   // the cause of a NaN that follows it, so it is the status reported
   if (!(F == F) && !status) status = DEREK_ERR_NAN;
@@ -370,7 +395,7 @@ __global__ void __launch_bounds__(256) k_mix_gram_partials(const Tables t, const
                                                            const long long *__restrict__ hist_off,
                                                            const SysState *__restrict__ st, int H,
                                                            double *__restrict__ part) {
-  __shared__ double red[256];
+  __shared__ double red[8];
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
   if (!S.active) return;
@@ -389,10 +414,14 @@ __global__ void __launch_bounds__(256) k_mix_gram_partials(const Tables t, const
   }
 }
 
-__global__ void k_mix_solve(const Tables t, int nsys, const double *__restrict__ part,
-                            SysState *__restrict__ st, int H) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys) return;
+// One warp per system: the lanes share each pair's partial sums, then Gaussian
+// elimination with partial pivoting, lane r holding row r (one thread did both:
+// 47 -> 22 us at 8 pairs).
+__global__ void __launch_bounds__(32) k_mix_solve(const Tables t, int nsys, const double *__restrict__ part,
+                                                  SysState *__restrict__ st, int H) {
+  __shared__ double A[kMaxHist + 1][kMaxHist + 2];   // the last column is the right-hand side
+  __shared__ double gram[kMaxHist][kMaxHist];
+  const int s = blockIdx.x, lane = threadIdx.x;
   const SysDev &S = t.sys[s];
   if (!S.active) return;
   SysState &X = st[s];
@@ -400,66 +429,64 @@ __global__ void k_mix_solve(const Tables t, int nsys, const double *__restrict__
   const int m = min(X.nhist + 1, H);
   for (int j = 0; j < m; ++j) {
     double q = 0;
-    for (int b = 0; b < RB; ++b) q += part[((long long)s * RB + b) * kMaxHist + j];
-    X.gram[slot * kMaxHist + j] = q;
-    X.gram[j * kMaxHist + slot] = q;
+    for (int b = lane; b < RB; b += 32) q += part[((long long)s * RB + b) * kMaxHist + j];
+    q = warp_sum(q);
+    if (lane == 0) {
+      X.gram[slot * kMaxHist + j] = q;
+      X.gram[j * kMaxHist + slot] = q;
+    }
   }
-  X.slot = slot;
-  X.nhist = m;
+  __syncwarp();
+  for (int e = lane; e < m * m; e += 32) gram[e / m][e % m] = X.gram[(e / m) * kMaxHist + e % m];
+  __syncwarp();
+  if (lane == 0) {
+    X.slot = slot;
+    X.nhist = m;
+  }
   // [G 1; 1^T 0] [c; lambda] = [0; 1], G scaled by its largest diagonal
-  double A[(kMaxHist + 1) * (kMaxHist + 1)];
-  double rhs[kMaxHist + 1];
   const int N = m + 1;
   double gmax = 0;
-  for (int j = 0; j < m; ++j) gmax = fmax(gmax, X.gram[j * kMaxHist + j]);
+  for (int j = 0; j < m; ++j) gmax = fmax(gmax, gram[j][j]);
   if (!(gmax > 0)) gmax = 1;
-  for (int i = 0; i < m; ++i) {
-    for (int j = 0; j < m; ++j) A[i * N + j] = X.gram[i * kMaxHist + j] / gmax;
-    A[i * N + m] = 1.0;
-    A[m * N + i] = 1.0;
-    rhs[i] = 0.0;
+  if (lane < N) {
+    for (int j = 0; j < m; ++j) A[lane][j] = lane < m ? gram[lane][j] / gmax : 1.0;
+    A[lane][m] = lane < m ? 1.0 : 0.0;
+    A[lane][N] = lane < m ? 0.0 : 1.0;
   }
-  A[m * N + m] = 0.0;
-  rhs[m] = 1.0;
+  __syncwarp();
   bool ok = true;
   for (int c = 0; c < N && ok; ++c) {
     int piv = c;
     for (int r = c + 1; r < N; ++r)
-      if (fabs(A[r * N + c]) > fabs(A[piv * N + c])) piv = r;
-    if (!(fabs(A[piv * N + c]) > 1e-14)) {
+      if (fabs(A[r][c]) > fabs(A[piv][c])) piv = r;
+    if (!(fabs(A[piv][c]) > 1e-14)) {
       ok = false;
       break;
     }
-    if (piv != c) {
-      for (int j = 0; j < N; ++j) {
-        const double tmp = A[c * N + j];
-        A[c * N + j] = A[piv * N + j];
-        A[piv * N + j] = tmp;
-      }
-      const double tmp = rhs[c];
-      rhs[c] = rhs[piv];
-      rhs[piv] = tmp;
+    __syncwarp();
+    if (piv != c && lane <= N) {
+      const double tmp = A[c][lane];
+      A[c][lane] = A[piv][lane];
+      A[piv][lane] = tmp;
     }
-    for (int r = c + 1; r < N; ++r) {
-      const double f = A[r * N + c] / A[c * N + c];
-      for (int j = c; j < N; ++j) A[r * N + j] -= f * A[c * N + j];
-      rhs[r] -= f * rhs[c];
+    __syncwarp();
+    if (lane > c && lane < N) {
+      const double f = A[lane][c] / A[c][c];
+      for (int j = c + 1; j <= N; ++j) A[lane][j] -= f * A[c][j];
     }
+    __syncwarp();
   }
-  double x[kMaxHist + 1];
+  double x = 0.0;   // lane r: solution r
   if (ok) {
     for (int r = N - 1; r >= 0; --r) {
-      double v = rhs[r];
-      for (int j = r + 1; j < N; ++j) v -= A[r * N + j] * x[j];
-      x[r] = v / A[r * N + r];
+      // every lane: v = rhs_r - sum_{j > r} A[r][j] x_j
+      const double v = A[r][N] - warp_sum(lane > r && lane < N ? A[r][lane] * x : 0.0);
+      if (lane == r) x = v / A[r][r];
     }
-  }
-  for (int j = 0; j < kMaxHist; ++j) X.coef[j] = 0.0;
-  if (ok) {
-    for (int j = 0; j < m; ++j) X.coef[j] = x[j];
   } else {
-    X.coef[slot] = 1.0;
+    x = lane == slot ? 1.0 : 0.0;
   }
+  if (lane < kMaxHist) X.coef[lane] = lane < m ? x : 0.0;
 }
 
 // rho_in <- sum c_j nin_j + (kerker ? 0 : alpha sum c_j R_j); cgrid <- sum c_j R_j
@@ -522,7 +549,7 @@ __global__ void __launch_bounds__(256) k_mix_gram_m(const Tables t, const SpinGr
                                                     const long long *__restrict__ hist_off,
                                                     const SysState *__restrict__ st, int H,
                                                     double *__restrict__ part) {
-  __shared__ double red[256];
+  __shared__ double red[8];
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
   if (!S.active) return;
@@ -572,9 +599,10 @@ __global__ void __launch_bounds__(256) k_kerker_scale(const Tables t, double2 *_
   const SysDev &S = t.sys[s];
   if (!S.active) return;
   const double invn = 1.0 / S.nr;
+  const Metric metric(S);
   for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < S.nr;
        r += (long long)gridDim.x * blockDim.x) {
-    const double g2 = gsq(S, r);
+    const double g2 = metric.gsq(S, (int)r);
     const double f = alpha * g2 / (g2 + q0 * q0) * invn;
     double2 &c = cgrid[S.grid_off + r];
     c.x *= f;
@@ -609,9 +637,10 @@ __global__ void __launch_bounds__(256) k_hartree_scale(const Tables t, double2 *
   if (!all && !S.active) return;
   const double four_pi = 12.566370614359172953850573533118;
   const double invn = 1.0 / S.nr;
+  const Metric metric(S);
   for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < S.nr;
        r += (long long)gridDim.x * blockDim.x) {
-    const double g2 = gsq(S, r);
+    const double g2 = metric.gsq(S, (int)r);
     const double f = g2 > 0 ? four_pi / g2 * invn : 0.0;
     double2 &v = c[S.grid_off + r];
     v.x *= f;
@@ -626,7 +655,7 @@ __global__ void __launch_bounds__(256) k_build_vloc(const Tables t, const double
                                                     double *__restrict__ vloc,
                                                     float *__restrict__ vloc32,
                                                     double *__restrict__ part, int all, const SpinGrids sg) {
-  __shared__ double red[256];
+  __shared__ double red[8];
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
   if (!all && !S.active) return;
@@ -677,23 +706,18 @@ __global__ void __launch_bounds__(256) k_build_vloc(const Tables t, const double
     if (vloc32) vloc32[i] = (float)vl;
     vm = fmax(vm, vl);
   }
-  red[threadIdx.x] = vm;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[((long long)s * RB + blockIdx.x) * EP + 4] = red[0];
+  vm = block_max(vm, red);
+  if (threadIdx.x == 0) part[((long long)s * RB + blockIdx.x) * EP + 4] = vm;
 }
 
-__global__ void k_vmax_final(const Tables t, int nsys, const double *__restrict__ part,
+__global__ void __launch_bounds__(32) k_vmax_final(const Tables t, int nsys, const double *__restrict__ part,
                              SysState *__restrict__ st, int all) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys) return;
+  const int s = blockIdx.x;
   if (!all && !t.sys[s].active) return;
   double vm = -1e300;
-  for (int b = 0; b < RB; ++b) vm = fmax(vm, part[((long long)s * RB + b) * EP + 4]);
-  st[s].vmax = vm;
+  for (int b = threadIdx.x; b < RB; b += 32) vm = fmax(vm, part[((long long)s * RB + b) * EP + 4]);
+  vm = warp_max(vm);
+  if (threadIdx.x == 0) st[s].vmax = vm;
 }
 
 __global__ void __launch_bounds__(256) k_uniform_density(const Tables t, double *__restrict__ rho) {
@@ -719,16 +743,17 @@ void launch_filter_coef(const Tables &t, int nks, const double *eig, const SysSt
   derek::note_launch(), k_filter_coef<<<(nks + 127) / 128, 128, 0, s>>>(t, nks, eig, st, coef, m);
 }
 
-void launch_occupations(const Tables &t, int nsys, const double *eig, double *occ, double *occw,
+void launch_occupations(const Tables &t, int nsys, int max_states, const double *eig, double *occ, double *occw,
                         SysState *st, cudaStream_t s) {
-  derek::note_launch(), k_occupations<<<nsys, 1024, 0, s>>>(t, eig, occ, occw, st);
+  const int threads = std::min(1024, std::max(32, (max_states + 31) / 32 * 32));
+  derek::note_launch(), k_occupations<<<nsys, threads, 0, s>>>(t, eig, occ, occw, st);
 }
 
 void launch_energies(const Tables &t, int nsys, const double *vhxc, const double *rho_in,
                      const double *rho_out, const double2 *cgrid, double *part, SysState *st,
                      SysDev *sys_rw, const int *ks_status, const SpinGrids &sg, cudaStream_t s) {
   derek::note_launch(), k_energy_partials<<<dim3(RB, nsys), 256, 0, s>>>(t, vhxc, rho_in, rho_out, cgrid, part, sg);
-  derek::note_launch(), k_energy_final<<<(nsys + 63) / 64, 64, 0, s>>>(t, nsys, part, st, sys_rw, ks_status);
+  derek::note_launch(), k_energy_final<<<nsys, 32, 0, s>>>(t, nsys, part, st, sys_rw, ks_status);
 }
 
 void launch_mix(const Tables &t, int nsys, int max_nr, double *rho_in, const double *rho_out,
@@ -740,7 +765,7 @@ void launch_mix(const Tables &t, int nsys, int max_nr, double *rho_in, const dou
   if (sg.on) derek::note_launch(), k_mix_store_m<<<dim3(gx, nsys), 256, 0, s>>>(t, sg, hist_off, st, H);
   derek::note_launch(), k_mix_gram_partials<<<dim3(RB, nsys), 256, 0, s>>>(t, res_hist, hist_off, st, H, part);
   if (sg.on) derek::note_launch(), k_mix_gram_m<<<dim3(RB, nsys), 256, 0, s>>>(t, sg, hist_off, st, H, part);
-  derek::note_launch(), k_mix_solve<<<(nsys + 63) / 64, 64, 0, s>>>(t, nsys, part, st, H);
+  derek::note_launch(), k_mix_solve<<<nsys, 32, 0, s>>>(t, nsys, part, st, H);
   const int kerker = q0 > 0;
   derek::note_launch(), k_mix_combine<<<dim3(gx, nsys), 256, 0, s>>>(t, rho_in, nin_hist, res_hist, hist_off, st, cgrid,
                                                alpha, kerker);
@@ -762,7 +787,7 @@ void launch_potential(const Tables &t, int nsys, int max_nr, int max_n, const do
   derek::note_launch(), k_hartree_scale<<<dim3(gx, nsys), 256, 0, s>>>(t, cgrid, all);
   launch_fft3d_grid(t, 0, nsys, max_n, cgrid, +1, s);
   derek::note_launch(), k_build_vloc<<<dim3(RB, nsys), 256, 0, s>>>(t, rho_in, cgrid, vext, vhxc, vloc, vloc32, part, all, sg);
-  derek::note_launch(), k_vmax_final<<<(nsys + 63) / 64, 64, 0, s>>>(t, nsys, part, st, all);
+  derek::note_launch(), k_vmax_final<<<nsys, 32, 0, s>>>(t, nsys, part, st, all);
 }
 
 __global__ void k_lsda(long n, const double *__restrict__ ra, const double *__restrict__ rb,
@@ -811,7 +836,7 @@ __global__ void __launch_bounds__(256) k_hf_partials(const Tables t, const doubl
                                                      const int *__restrict__ well_off,
                                                      const double *__restrict__ cells,
                                                      double *__restrict__ part, int max_wells) {
-  __shared__ double red[256];
+  __shared__ double red[8];
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
   const int n1 = S.n[0], n2 = S.n[1], n3 = S.n[2];

@@ -23,6 +23,10 @@ struct SpinGrids {
   double *min_hist, *mres_hist;   // mixing history, 3 x (hist slots x nr) per system
 };
 
+// blocks of a system in the grid reductions: one per SM, for one small system as
+// for many (their partial sums are added in a fixed order)
+constexpr int kRedBlocks = 152;
+
 template <typename R>
 // start vectors: hashed random entries, or (pw_entry non-null) band b of item
 // i on entry pw_entry[i] plus a small hashed perturbation
@@ -32,7 +36,8 @@ void launch_filter_coef(const Tables &t, int nks, const double *eig, const SysSt
                         int m, cudaStream_t s);
 // t is the band view: a spinor band holds one electron and its density
 // weight goes to both of its items
-void launch_occupations(const Tables &t, int nsys, const double *eig, double *occ, double *occw,
+// max_states: most (k-point, reported band) states of a system
+void launch_occupations(const Tables &t, int nsys, int max_states, const double *eig, double *occ, double *occw,
                         SysState *st, cudaStream_t s);
 void launch_energies(const Tables &t, int nsys, const double *vhxc, const double *rho_in,
                      const double *rho_out, const double2 *cgrid, double *part, SysState *st,

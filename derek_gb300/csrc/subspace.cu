@@ -356,8 +356,22 @@ __global__ void __launch_bounds__(256, 2) k_rotate32(const Tables t, int ks_begi
   }
 }
 
+// neg ? -x : x on the sign bit (a negation by itself is an FP64 operation)
+__device__ __forceinline__ double flip(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
+}
+
 // ---------------------------------------------------------------------------
 // Cholesky S = L L^H and C = L^-H (upper triangular), one block per k-set.
+// Worked as S = (Lu) D (Lu)^H with Lu unit lower triangular: step j subtracts
+// (m_ij / d_j) times the pivot row from every row i > j, of the trailing matrix
+// and of the inverse that grows beside it (Y = Lu^-1), so a step is one
+// division, one pass over independent elements and one barrier; the roots
+// come at the end, L^-1 = D^-1/2 Y.  Y shares the square with the matrix (its
+// row i, stored as column i of the upper triangle), which keeps up to 118 bands in
+// shared memory.  Before, a root, a division and three barriers a step, the
+// inverse by one thread per column and 81 bands and more in global memory: 12
+// bands 35 -> 13 us, 24 bands 102 -> 33 us, 84 bands 1,140 -> 540 us.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double2 zmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -376,73 +390,57 @@ __global__ void __launch_bounds__(256) k_cholesky_inv(const Tables t, int ks_beg
   const int ksi = ks_begin + blockIdx.x;
   const KSetDev &K = t.ks[ksi];
   if (!t.sys[K.sys].active) return;
-  const int n = K.nb;
+  const int n = K.nb, ld = n | 1;   // odd pitch: columns are walked too
+  // M[i][k], i >= k: the matrix (its diagonal ends as D); M[c][i], c < i: Y[i][c]
   double2 *M = use_smem ? reinterpret_cast<double2 *>(smem_raw) : scratch + 2 * mat_off[ksi];
-  double2 *Li = M + n * n;
-  __shared__ double s_diag;
-  __shared__ int s_fail;
   const double2 *Sb = S + mat_off[ksi];
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) M[(e / n) * ld + e % n] = e / n >= e % n ? Sb[e] : make_double2(0, 0);
+  __syncthreads();
+  // failure threshold relative to the largest diagonal element
   double dmax = 0.0;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    M[e] = Sb[e];
-    Li[e] = make_double2(0, 0);
+  for (int i = 0; i < n; i += 32) {
+    const double v = i + (threadIdx.x & 31) < n ? M[(i + (threadIdx.x & 31)) * (ld + 1)].x : 0.0;
+    dmax = fmax(dmax, v);
   }
-  if (threadIdx.x == 0) s_fail = 0;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < n; ++i) dmax = fmax(dmax, M[i * n + i].x);
-    s_diag = dmax;
-  }
-  __syncthreads();
-  const double thr = 1e-13 * s_diag;
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, w));
+  const double thr = 1e-13 * dmax;
+  bool fail = false;
   for (int j = 0; j < n; ++j) {
-    if (threadIdx.x == 0) {
-      const double d = M[j * n + j].x;
-      if (!(d > thr)) s_fail = 1;
-      M[j * n + j] = make_double2(sqrt(fmax(d, thr)), 0.0);
-    }
-    __syncthreads();
-    const double inv = 1.0 / M[j * n + j].x;
-    for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) {
-      M[i * n + j].x *= inv;
-      M[i * n + j].y *= inv;
-    }
-    __syncthreads();
-    // trailing update of the lower triangle: M[i][k] -= L[i][j] conj(L[k][j]), j < k <= i
-    const int m = n - j - 1;
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-      const int i = j + 1 + e / m, k = j + 1 + e % m;
-      if (k <= i) {
-        const double2 p = zmulc(M[i * n + j], M[k * n + j]);
-        M[i * n + k].x -= p.x;
-        M[i * n + k].y -= p.y;
-      }
+    // every thread reads the pivot: the previous step's barrier published it
+    const double d = M[j * ld + j].x;
+    const bool low = !(d > thr);
+    fail |= low;
+    const double w = 1.0 / (low ? thr : d);
+    const int rows = n - 1 - j;
+    for (int e = threadIdx.x; e < rows * n; e += blockDim.x) {
+      const int i = j + 1 + e / n, k = e - (e / n) * n;
+      if (k > i) continue;
+      const double2 m = M[i * ld + j], f = make_double2(m.x * w, m.y * w);
+      // trailing matrix (k > j): M[i][k] -= m_ij / d conj(m_kj); inverse (k <= j):
+      // Y[i][k] -= m_ij / d Y[j][k] with Y[j][j] = 1, without a branch between them
+      double2 z = M[k * ld + j];
+      z = make_double2(k == j ? 1.0 : z.x, k == j ? 0.0 : flip(z.y, k > j));
+      double2 &dst = M[k > j ? i * ld + k : k * ld + i];
+      double2 v = dst;
+      cmac<double>(v, make_double2(-f.x, -f.y), z);
+      dst = make_double2(v.x, k == i ? 0.0 : v.y);
     }
     __syncthreads();
   }
-  // inverse of L: column c solves L x = e_c (forward substitution), one thread per column
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    for (int i = c; i < n; ++i) {
-      double2 acc = make_double2(i == c ? 1.0 : 0.0, 0.0);
-      for (int p = c; p < i; ++p) {
-        const double2 q = zmul(M[i * n + p], Li[p * n + c]);
-        acc.x -= q.x;
-        acc.y -= q.y;
-      }
-      const double d = 1.0 / M[i * n + i].x;
-      Li[i * n + c] = make_double2(acc.x * d, acc.y * d);
-    }
-  }
-  __syncthreads();
-  // C[i][j] = conj(Linv[j][i])
+  // C[i][j] = conj(Linv[j][i]), Linv[j][i] = Y[j][i] / sqrt(d_j)
   double2 *Cb = Cout + mat_off[ksi];
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
     const int i = e / n, j = e % n;
-    const double2 v = Li[j * n + i];
-    Cb[e] = make_double2(v.x, -v.y);
+    const double d = M[j * ld + j].x;
+    const double r = rsqrt(d > thr ? d : thr);
+    double2 v = make_double2(0.0, 0.0);
+    if (i < j) v = M[i * ld + j];
+    if (i == j) v.x = 1.0;
+    Cb[e] = make_double2(v.x * r, -v.y * r);
   }
   // keep an earlier failure of this k-set (a timed-out overlap wait)
-  if (threadIdx.x == 0 && s_fail && status[ksi] == 0) status[ksi] = DEREK_ERR_CHOLESKY;
+  if (threadIdx.x == 0 && fail && status[ksi] == 0) status[ksi] = DEREK_ERR_CHOLESKY;
 }
 
 // ---------------------------------------------------------------------------
@@ -501,11 +499,6 @@ __device__ __forceinline__ void rr_pair(int k, int r, int ne, int &p, int &q) {
   b += 1;
   p = min(a, b);
   q = max(a, b);
-}
-
-// neg ? -x : x on the sign bit (a negation by itself is an FP64 operation)
-__device__ __forceinline__ double flip(double x, bool neg) {
-  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
 }
 
 // x + y i scaled to unit length, x^2 + y^2 = 1 + d with |d| ~ 1e-7
@@ -1136,13 +1129,13 @@ void launch_rotate(const Tables &t, int ks_begin, int nks, int max_nb, int max_n
   }
 }
 
-bool cholesky_fits_smem(int max_nb) { return 2 * (size_t)max_nb * max_nb * 16 <= 200 * 1024; }
+static bool cholesky_fits_smem(int max_nb) { return (size_t)max_nb * (max_nb | 1) * sizeof(double2) <= 226 * 1024; }
 void launch_cholesky_inv(const Tables &t, int ks_begin, int nks, int max_nb, const double2 *S,
                          double2 *C, const long long *mat_off, double2 *scratch, int *status,
                          cudaStream_t st) {
   if (nks <= 0) return;
   const int use_smem = cholesky_fits_smem(max_nb);
-  const size_t sm = use_smem ? 2 * (size_t)max_nb * max_nb * sizeof(double2) : 0;
+  const size_t sm = use_smem ? (size_t)max_nb * (max_nb | 1) * sizeof(double2) : 0;
   cudaFuncSetAttribute(k_cholesky_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   derek::note_launch(), k_cholesky_inv<<<nks, 256, sm, st>>>(t, ks_begin, S, C, mat_off, scratch, status, use_smem);
 }

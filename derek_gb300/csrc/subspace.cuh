@@ -42,7 +42,6 @@ template <typename R>
 // upper: C is upper triangular
 void launch_rotate(const Tables &t, int ks_begin, int nks, int max_nb, int max_npw, cplx<R> *X,
                    const double2 *C, const long long *mat_off, int upper, cudaStream_t st);
-bool cholesky_fits_smem(int max_nb);
 void launch_cholesky_inv(const Tables &t, int ks_begin, int nks, int max_nb, const double2 *S,
                          double2 *C, const long long *mat_off, double2 *scratch, int *status,
                          cudaStream_t st);

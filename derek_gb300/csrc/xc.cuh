@@ -16,38 +16,44 @@ __device__ __forceinline__ void lda_point(double rho, double &exc, double &vxc) 
     return;
   }
   const double n = rho;
-  const double pi = 3.141592653589793238462643383279502884;
-  double ex = -0.75 * cbrt(3.0 / pi) * cbrt(n);
+  // one root of n and one division: n^{-1/3} gives n^{1/3} and r_s, and
+  // 1 / (q1 (1 + q1)) both quotients of the correlation.  Roots, divisions and
+  // the logarithm are what an FP64 point costs (10 to 32 operations each); V_loc
+  // of a 24-system batch 1.30 -> 0.80 ms, of a 48^3 spinor system 248 -> 79 us.
+  const double r13 = rcbrt(n);
+  double ex = -0.75 * 0.9847450218426965411789 * (n * r13 * r13);   // (3/pi)^{1/3}
   if (!(0.5 * n > thr)) ex = 0.0;
   const double vx = 4.0 / 3.0 * ex;
-  const double rs = cbrt(3.0 / (4.0 * pi * n));
+  const double rs = 0.6203504908994000166680 * r13;   // (3/(4 pi))^{1/3}
   const double a = 0.031091, alpha1 = 0.21370, b1 = 7.5957, b2 = 3.5876, b3 = 1.6382,
                b4 = 0.49294;
-  const double srs = sqrt(rs);
+  const double isrs = rsqrt(rs), srs = rs * isrs;
   const double q0 = -2.0 * a * (1.0 + alpha1 * rs);
   const double q1 = 2.0 * a * (b1 * srs + b2 * rs + b3 * rs * srs + b4 * rs * rs);
-  const double dq1 = a * (b1 / srs + 2.0 * b2 + 3.0 * b3 * srs + 4.0 * b4 * rs);
-  const double lg = log(1.0 + 1.0 / q1);
+  const double dq1 = a * (b1 * isrs + 2.0 * b2 + 3.0 * b3 * srs + 4.0 * b4 * rs);
+  const double iq = 1.0 / (q1 * q1 + q1);
+  const double lg = log(1.0 + (q1 + 1.0) * iq);
   const double ec = q0 * lg;
-  const double dec = -2.0 * a * alpha1 * lg - q0 * dq1 / (q1 * q1 + q1);
-  const double vc = ec - rs / 3.0 * dec;
+  const double dec = -2.0 * a * alpha1 * lg - q0 * dq1 * iq;
+  const double vc = ec - rs * (1.0 / 3.0) * dec;
   exc = ex + ec;
   vxc = vx + vc;
 }
 
 // PW92 G_k(rs) and dG_k/drs for parameter column k of src/lda_c_pw.c:41-50
 // (k = 0: eps_c(rs, 0); 1: eps_c(rs, 1); 2: -alpha_c(rs)).
-__device__ __forceinline__ void pw92_g(int k, double rs, double srs, double &g, double &dg) {
+__device__ __forceinline__ void pw92_g(int k, double rs, double srs, double isrs, double &g, double &dg) {
   const double A[3] = {0.031091, 0.015545, 0.016887}, AL[3] = {0.21370, 0.20548, 0.11125},
                B1[3] = {7.5957, 14.1189, 10.357}, B2[3] = {3.5876, 6.1977, 3.6231},
                B3[3] = {1.6382, 3.3662, 0.88026}, B4[3] = {0.49294, 0.62517, 0.49671};
   const double a = A[k], al = AL[k];
   const double q0 = -2.0 * a * (1.0 + al * rs);
   const double q1 = 2.0 * a * (B1[k] * srs + B2[k] * rs + B3[k] * rs * srs + B4[k] * rs * rs);
-  const double dq1 = a * (B1[k] / srs + 2.0 * B2[k] + 3.0 * B3[k] * srs + 4.0 * B4[k] * rs);
-  const double lg = log(1.0 + 1.0 / q1);
+  const double dq1 = a * (B1[k] * isrs + 2.0 * B2[k] + 3.0 * B3[k] * srs + 4.0 * B4[k] * rs);
+  const double iq = 1.0 / (q1 * q1 + q1);
+  const double lg = log(1.0 + (q1 + 1.0) * iq);
   g = q0 * lg;
-  dg = -2.0 * a * al * lg - q0 * dq1 / (q1 * q1 + q1);
+  dg = -2.0 * a * al * lg - q0 * dq1 * iq;
 }
 
 // Spin-polarised LDA (Slater exchange + PW92 with the spin interpolation of
@@ -74,35 +80,37 @@ __device__ __forceinline__ void lsda_point(double rho_a, double rho_b, double &e
     opz = 2.0 - zt;
   }
   const double z = opz - 1.0;
-  const double pi = 3.141592653589793238462643383279502884;
-  const double cx = -0.75 * cbrt(3.0 / pi);
-  const double n13 = cbrt(n);
-  const double c43a = cbrt(opz) * opz, c43b = cbrt(omz) * omz;   // (1 +/- z)^{4/3}
+  // roots shared as in lda_point: (6 n_s / pi)^{1/3} = (3/pi)^{1/3} n^{1/3} (1 +/- z)^{1/3}
+  const double c3pi = 0.9847450218426965411789;   // (3/pi)^{1/3}
+  const double cx = -0.75 * c3pi;
+  const double r13 = rcbrt(n), n13 = n * r13 * r13;
+  const double ca = cbrt(opz), cb = cbrt(omz);
+  const double c43a = ca * opz, c43b = cb * omz;   // (1 +/- z)^{4/3}
   double ex = 0.0;
   if (na > thr) {
     ex += 0.5 * cx * n13 * c43a;
-    va = -cbrt(6.0 * na / pi);
+    va = -c3pi * n13 * ca;
   }
   if (nb > thr) {
     ex += 0.5 * cx * n13 * c43b;
-    vb = -cbrt(6.0 * nb / pi);
+    vb = -c3pi * n13 * cb;
   }
-  const double rs = cbrt(3.0 / (4.0 * pi * n));
-  const double srs = sqrt(rs);
+  const double rs = 0.6203504908994000166680 * r13;
+  const double isrs = rsqrt(rs), srs = rs * isrs;
   double g1, d1, g2, d2, g3, d3;
-  pw92_g(0, rs, srs, g1, d1);
-  pw92_g(1, rs, srs, g2, d2);
-  pw92_g(2, rs, srs, g3, d3);
+  pw92_g(0, rs, srs, isrs, g1, d1);
+  pw92_g(1, rs, srs, isrs, g2, d2);
+  pw92_g(2, rs, srs, isrs, g3, d3);
   const double fz20 = 1.709921;
   const double den = 0.5198420997897464;   // 2^{4/3} - 2
-  const double fz = (c43a + c43b - 2.0) / den;
-  const double dfz = (4.0 / 3.0) * (cbrt(opz) - cbrt(omz)) / den;
+  const double fz = (c43a + c43b - 2.0) * (1.0 / den);
+  const double dfz = (4.0 / 3.0) * (ca - cb) * (1.0 / den);
   const double z3 = z * z * z, z4 = z3 * z;
-  const double stiff = g2 - g1 + g3 / fz20;
-  const double ec = g1 + z4 * fz * stiff - fz * g3 / fz20;
-  const double de_rs = d1 + z4 * fz * (d2 - d1 + d3 / fz20) - fz * d3 / fz20;
-  const double de_z = (4.0 * z3 * fz + z4 * dfz) * stiff - dfz * g3 / fz20;
-  const double base = ec - rs / 3.0 * de_rs;
+  const double stiff = g2 - g1 + g3 * (1.0 / fz20);
+  const double ec = g1 + z4 * fz * stiff - fz * g3 * (1.0 / fz20);
+  const double de_rs = d1 + z4 * fz * (d2 - d1 + d3 * (1.0 / fz20)) - fz * d3 * (1.0 / fz20);
+  const double de_z = (4.0 * z3 * fz + z4 * dfz) * stiff - dfz * g3 * (1.0 / fz20);
+  const double base = ec - rs * (1.0 / 3.0) * de_rs;
   exc = ex + ec;
   va += base + omz * de_z;
   vb += base - opz * de_z;
