@@ -170,11 +170,11 @@ __global__ void k_scale_grid(long long n, const double *__restrict__ a, double s
 
 // dV = g + V_H[dn] + f_xc dn
 __global__ void k_response_potential(long long n, const double *__restrict__ g,
-                                     const double2 *__restrict__ vh, const double *__restrict__ fxc,
+                                     const double *__restrict__ vh, const double *__restrict__ fxc,
                                      const double *__restrict__ dn, double *__restrict__ dv) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
-    dv[i] = g[i] + vh[i].x + fxc[i] * dn[i];
+    dv[i] = g[i] + vh[i] + fxc[i] * dn[i];
 }
 
 template <typename T> cudaError_t dmalloc(T **p, size_t n) {
@@ -382,8 +382,8 @@ extern "C" int derek_gpu_grad_density_loss(derek_gpu_t *h, int s, const double *
   bool converged = false;
   for (int iter = 0; iter < max_iter && !converged; ++iter) {
     CKA(cudaMemcpyAsync(W.dn, dn.data(), nr * sizeof(double), cudaMemcpyHostToDevice, st));
-    launch_hartree_only(t, 1, (int)nr, h->max_nmax, W.dn, h->d_cgrid, st);
-    derek::note_launch(), k_response_potential<<<152, 256, 0, st>>>(nr, W.g, h->d_cgrid, W.fxc, W.dn, W.dv);
+    launch_hartree(t, 1, h->max_nmax, W.dn - S.grid_off, h->d_cgrid, h->d_rwork, 1, st);
+    derek::note_launch(), k_response_potential<<<152, 256, 0, st>>>(nr, W.g, h->d_rwork + S.grid_off, W.fxc, W.dn, W.dv);
     // phi = dV psi
     {
       int e2 = apply_h_items_ex(h, t, 0, ni, psi, nullptr, W.phi, W.vcoef, W.dv);

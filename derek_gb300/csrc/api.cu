@@ -329,8 +329,8 @@ int derek_gpu_destroy(derek_gpu_t *h) {
   void *ptrs[] = {h->d_sys,   h->d_ks,      h->d_item_ks, h->d_item_band, h->d_ent_col,
                   h->d_col_start, h->d_ent_ix, h->d_col_y, h->d_col_z, h->d_col_x0, h->d_rows, h->d_pw_entry, h->d_kin64,     h->d_kin32,    h->d_perm,
                   h->d_tw64,  h->d_tw32,    h->d_vext,    h->d_vloc,      h->d_vhxc,
-                  h->d_vloc32, h->d_rho_in, h->d_rho_out, h->d_exc,       h->d_vxc,
-                  h->d_cgrid, h->d_partial, h->d_sys_part, h->d_sys_units, h->d_X,     h->d_Y,
+                  h->d_vloc32, h->d_rho_in, h->d_rho_out,
+                  h->d_cgrid, h->d_rwork,  h->d_partial, h->d_sys_part, h->d_sys_units, h->d_X,     h->d_Y,
                   h->d_Yp,    h->d_HX,      h->d_abuf,    h->d_occw,      h->d_eig,
                   h->d_occ,   h->d_coef,    h->d_cells,   h->d_wells,     h->d_well_off,
                   h->d_hfpart, h->d_hfgrad, h->d_vnc64, h->d_vnc32, h->d_mag, h->d_ks_band,
@@ -636,9 +636,8 @@ int derek_gpu_create(derek_gpu_t **out, const derek_sys_desc *desc, int nsys,
   CK(cudaMalloc((void **)&h->d_vloc32, (size_t)grid_off * sizeof(float)));
   CK(cudaMalloc((void **)&h->d_rho_in, gbytes));
   CK(cudaMalloc((void **)&h->d_rho_out, gbytes));
-  CK(cudaMalloc((void **)&h->d_exc, gbytes));
-  CK(cudaMalloc((void **)&h->d_vxc, gbytes));
   CK(cudaMalloc((void **)&h->d_cgrid, (size_t)grid_off * sizeof(double2)));
+  CK(cudaMalloc((void **)&h->d_rwork, gbytes));
   if (h->any_spinor) {
     // nc_pot starts as V_ext on the diagonal (Source/pot.f90:133-166)
     std::vector<double2> vnc((size_t)4 * grid_off, make_double2(0.0, 0.0));

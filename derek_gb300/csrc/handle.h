@@ -71,8 +71,8 @@ struct derek_gpu {
   double *d_mag_in = nullptr, *d_bxc = nullptr, *d_min_hist = nullptr, *d_mres_hist = nullptr;
   std::vector<std::vector<double>> start_mag;
   std::vector<std::vector<double>> start_rho;   // per system: SCF start density (empty = uniform)
-  double *d_exc = nullptr, *d_vxc = nullptr;
   double2 *d_cgrid = nullptr;      // complex work grid
+  double *d_rwork = nullptr;       // real work grid: V_H, the mixed residual
   double *d_partial = nullptr;     // density partials, one grid (spinor: four) per unit
   long long *d_sys_part = nullptr; // per system: offset of its first unit's partial grid
   int *d_sys_units = nullptr;      // per system: units

@@ -108,6 +108,14 @@ bool launch_density_reg(const Tables &t, const DensityUnit *units, int nunits, i
 // [sys_begin, sys_begin + nsys); grid s starts at data + sys[s].grid_off.
 void launch_fft3d_grid(const Tables &t, int sys_begin, int nsys, int max_n, double2 *data,
                        int sign, cudaStream_t st);
+// Real grids of every active system (all: of every system), through half
+// spectra in `work`: F[rho] at kz <= n3/2; V_H[rho] into vh; rho += F^-1[
+// alpha G^2 / (G^2 + q0^2) F[res]].
+void launch_real_spectrum(const Tables &t, int nsys, int max_n, const double *rho, double2 *work, cudaStream_t st);
+void launch_hartree(const Tables &t, int nsys, int max_n, const double *rho, double2 *work, double *vh, int all,
+                    cudaStream_t st);
+void launch_kerker_add(const Tables &t, int nsys, int max_n, const double *res, double2 *work, double alpha, double q0,
+                       double *rho, cudaStream_t st);
 
 // wavefunction slices of one k-set: `count` of the caller's rows from row0 on,
 // in the caller's layout, to or from the device slice (wfn_io.cu)

@@ -154,14 +154,13 @@ int finish_iteration(derek_gpu *h) {
   int st = sg.on ? density_spinor_items(h, h->cur_psi(), h->d_rho_out)
                  : density_items(h, h->cur_psi(), h->d_rho_out);
   if (st) return st;
-  launch_density_fft(h->tab, h->nsys, (int)h->max_nr, h->max_nmax, h->d_rho_out, h->d_cgrid,
-                     h->stream);
+  launch_real_spectrum(h->tab, h->nsys, h->max_nmax, h->d_rho_out, h->d_cgrid, h->stream);
   launch_energies(h->tab, h->nsys, h->d_vhxc, h->d_rho_in, h->d_rho_out, h->d_cgrid, h->d_epart, h->d_state,
                   h->d_sys, h->d_status, sg, h->stream);
   launch_mix(h->tab, h->nsys, (int)h->max_nr, h->d_rho_in, h->d_rho_out, h->d_nin_hist,
-             h->d_res_hist, h->d_hist_off, h->d_state, h->hist, h->d_gpart, h->d_cgrid,
+             h->d_res_hist, h->d_hist_off, h->d_state, h->hist, h->d_gpart, h->d_cgrid, h->d_rwork,
              h->opts.mix_alpha, h->opts.kerker_q0, h->max_nmax, sg, h->stream);
-  launch_potential(h->tab, h->nsys, (int)h->max_nr, h->max_nmax, h->d_rho_in, h->d_cgrid,
+  launch_potential(h->tab, h->nsys, h->max_nmax, h->d_rho_in, h->d_cgrid, h->d_rwork,
                    h->d_vext, h->d_vhxc, h->d_vloc, h->prec == DEREK_PREC_FP64 ? nullptr : h->d_vloc32,
                    h->d_epart, h->d_state, 0, sg, h->stream);
   DEREK_CUDA(h, cudaGetLastError());
@@ -258,7 +257,7 @@ int scf_start(derek_gpu *h, double etol) {
                                         (size_t)h->sys[s].nr * sizeof(double), cudaMemcpyHostToDevice,
                                         h->stream));
   }
-  launch_potential(h->tab, h->nsys, (int)h->max_nr, h->max_nmax, h->d_rho_in, h->d_cgrid,
+  launch_potential(h->tab, h->nsys, h->max_nmax, h->d_rho_in, h->d_cgrid, h->d_rwork,
                    h->d_vext, h->d_vhxc, h->d_vloc, h->prec == DEREK_PREC_FP64 ? nullptr : h->d_vloc32,
                    h->d_epart, h->d_state, 1, sg, h->stream);
   int s = start_vectors(h);

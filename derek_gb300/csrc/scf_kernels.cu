@@ -11,6 +11,7 @@
 //   E_H = Omega/2 sum_G 4 pi |n(G)|^2/|G|^2
 //   E = E_band - int V_Hxc[n_in] n_out + E_H[n_out] + E_xc[n_out],  F = E - kT S
 #include "scf_kernels.cuh"
+#include "metric.cuh"
 #include "xc.cuh"
 
 namespace derek {
@@ -51,32 +52,6 @@ __device__ __forceinline__ double block_max(double v, double *red) {
   __syncthreads();
   return v;
 }
-
-// |G|^2 = m^T W m of grid point r, W = B^T B.  Exactly zero at G = 0.
-struct Metric {
-  double w00, w01, w02, w11, w12, w22;
-  __device__ __forceinline__ explicit Metric(const SysDev &S) {
-    w00 = w01 = w02 = w11 = w12 = w22 = 0.0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const double x = S.B[3 * i], y = S.B[3 * i + 1], z = S.B[3 * i + 2];
-      w00 += x * x;
-      w01 += 2.0 * x * y;
-      w02 += 2.0 * x * z;
-      w11 += y * y;
-      w12 += 2.0 * y * z;
-      w22 += z * z;
-    }
-  }
-  __device__ __forceinline__ double gsq(const SysDev &S, int r) const {
-    const int n1 = S.n[0], n2 = S.n[1], n3 = S.n[2];
-    const int q = r / n3, iz = r - q * n3, ix = q / n2, iy = q - ix * n2;
-    const double m0 = ix < n1 - n1 / 2 ? ix : ix - n1;
-    const double m1 = iy < n2 - n2 / 2 ? iy : iy - n2;
-    const double m2 = iz < n3 - n3 / 2 ? iz : iz - n3;
-    return m0 * (w00 * m0 + w01 * m1 + w02 * m2) + m1 * (w11 * m1 + w12 * m2) + w22 * m2 * m2;
-  }
-};
 
 // ---- start vectors: real r - 0.5 per (band, G) like wave_initialise_wfn
 // (Source/wave.f90:873-886), from a splitmix64 counter hash
@@ -266,7 +241,8 @@ __global__ void __launch_bounds__(1024) k_occupations(const Tables t, const doub
   }
 }
 
-// ---- energies of the output density.  cgrid holds F[n_out] (unnormalised).
+// ---- energies of the output density.  cgrid holds the half spectrum F[n_out]
+// (kz <= n3/2, unnormalised).
 __global__ void __launch_bounds__(256) k_energy_partials(const Tables t, const double *__restrict__ vhxc,
                                                          const double *__restrict__ rho_in,
                                                          const double *__restrict__ rho_out,
@@ -280,6 +256,7 @@ __global__ void __launch_bounds__(256) k_energy_partials(const Tables t, const d
   const long long chunk = (n + RB - 1) / RB;
   const long long r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
   double q0 = 0, q1 = 0, q2 = 0, q3 = 0;
+  const int n1 = S.n[0], n2 = S.n[1], n3 = S.n[2];
   const Metric metric(S);
   for (long long r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
     const double nr = rho_out[S.grid_off + r];
@@ -304,10 +281,22 @@ __global__ void __launch_bounds__(256) k_energy_partials(const Tables t, const d
       lda_point(nr, e, v);
     }
     q1 += nr * e;
-    const double g2 = metric.gsq(S, (int)r);
-    if (g2 > 0) {
-      const double2 c = cgrid[S.grid_off + r];
-      q2 += (c.x * c.x + c.y * c.y) / g2;
+    // sum |c|^2 / G^2 over the whole grid: an entry with 0 < kz < n3/2 stands
+    // for its conjugate partner too
+    const int q = (int)r / n3, iz = (int)r - q * n3, ix = q / n2, iy = q - ix * n2;
+    if (2 * iz <= n3) {
+      const double g2 = metric.gsq(S, ix, iy, iz);
+      if (g2 > 0) {
+        const double2 c = cgrid[S.grid_off + r];
+        double w = 1.0 / g2;
+        if (iz > 0 && 2 * iz < n3) {
+          if (2 * ix == n1 || 2 * iy == n2)   // Nyquist: the partner's G is not -G
+            w += 1.0 / metric.gsq(S, ix ? n1 - ix : 0, iy ? n2 - iy : 0, n3 - iz);
+          else
+            w *= 2.0;
+        }
+        q2 += (c.x * c.x + c.y * c.y) * w;
+      }
     }
   }
   q0 = block_sum(q0, red);
@@ -489,13 +478,13 @@ __global__ void __launch_bounds__(32) k_mix_solve(const Tables t, int nsys, cons
   if (lane < kMaxHist) X.coef[lane] = lane < m ? x : 0.0;
 }
 
-// rho_in <- sum c_j nin_j + (kerker ? 0 : alpha sum c_j R_j); cgrid <- sum c_j R_j
+// rho_in <- sum c_j nin_j + (kerker ? 0 : alpha sum c_j R_j); rwork <- sum c_j R_j
 __global__ void __launch_bounds__(256) k_mix_combine(const Tables t, double *__restrict__ rho_in,
                                                      const double *__restrict__ nin_hist,
                                                      const double *__restrict__ res_hist,
                                                      const long long *__restrict__ hist_off,
                                                      const SysState *__restrict__ st,
-                                                     double2 *__restrict__ cgrid, double alpha,
+                                                     double *__restrict__ rwork, double alpha,
                                                      int kerker) {
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
@@ -515,7 +504,7 @@ __global__ void __launch_bounds__(256) k_mix_combine(const Tables t, double *__r
     }
     if (kerker) {
       rho_in[S.grid_off + r] = a;
-      cgrid[S.grid_off + r] = make_double2(b, 0.0);
+      rwork[S.grid_off + r] = b;
     } else {
       rho_in[S.grid_off + r] = a + alpha * b;
     }
@@ -592,64 +581,9 @@ __global__ void __launch_bounds__(256) k_mix_combine_m(const Tables t, const Spi
   }
 }
 
-// cgrid <- alpha G^2/(G^2 + q0^2) cgrid / N (the /N undoes the unnormalised pair)
-__global__ void __launch_bounds__(256) k_kerker_scale(const Tables t, double2 *__restrict__ cgrid,
-                                                      double alpha, double q0) {
-  const int s = blockIdx.y;
-  const SysDev &S = t.sys[s];
-  if (!S.active) return;
-  const double invn = 1.0 / S.nr;
-  const Metric metric(S);
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < S.nr;
-       r += (long long)gridDim.x * blockDim.x) {
-    const double g2 = metric.gsq(S, (int)r);
-    const double f = alpha * g2 / (g2 + q0 * q0) * invn;
-    double2 &c = cgrid[S.grid_off + r];
-    c.x *= f;
-    c.y *= f;
-  }
-}
-
-__global__ void __launch_bounds__(256) k_add_real(const Tables t, double *__restrict__ rho,
-                                                  const double2 *__restrict__ cgrid) {
-  const int s = blockIdx.y;
-  const SysDev &S = t.sys[s];
-  if (!S.active) return;
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < S.nr;
-       r += (long long)gridDim.x * blockDim.x)
-    rho[S.grid_off + r] += cgrid[S.grid_off + r].x;
-}
-
 // ---- potential
-__global__ void __launch_bounds__(256) k_real_to_complex(const Tables t, const double *__restrict__ a,
-                                                         double2 *__restrict__ c, int all) {
-  const int s = blockIdx.y;
-  const SysDev &S = t.sys[s];
-  if (!all && !S.active) return;
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < S.nr;
-       r += (long long)gridDim.x * blockDim.x)
-    c[S.grid_off + r] = make_double2(a[S.grid_off + r], 0.0);
-}
-
-__global__ void __launch_bounds__(256) k_hartree_scale(const Tables t, double2 *__restrict__ c, int all) {
-  const int s = blockIdx.y;
-  const SysDev &S = t.sys[s];
-  if (!all && !S.active) return;
-  const double four_pi = 12.566370614359172953850573533118;
-  const double invn = 1.0 / S.nr;
-  const Metric metric(S);
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < S.nr;
-       r += (long long)gridDim.x * blockDim.x) {
-    const double g2 = metric.gsq(S, (int)r);
-    const double f = g2 > 0 ? four_pi / g2 * invn : 0.0;
-    double2 &v = c[S.grid_off + r];
-    v.x *= f;
-    v.y *= f;
-  }
-}
-
 __global__ void __launch_bounds__(256) k_build_vloc(const Tables t, const double *__restrict__ rho_in,
-                                                    const double2 *__restrict__ vh,
+                                                    const double *__restrict__ vh,
                                                     const double *__restrict__ vext,
                                                     double *__restrict__ vhxc,
                                                     double *__restrict__ vloc,
@@ -675,7 +609,7 @@ __global__ void __launch_bounds__(256) k_build_vloc(const Tables t, const double
       const double n = rho_in[i];
       double va, vb;
       lsda_point(0.5 * (n + am), 0.5 * (n - am), e, va, vb);
-      const double hx = vh[i].x + 0.5 * (va + vb);
+      const double hx = vh[i] + 0.5 * (va + vb);
       const double sc = am > 0.0 ? 0.5 * (va - vb) / am : 0.0;
       const double bx = sc * mx, by = sc * my, bz = sc * mz;
       sg.bxc[i] = bx;
@@ -699,7 +633,7 @@ __global__ void __launch_bounds__(256) k_build_vloc(const Tables t, const double
       continue;
     }
     lda_point(rho_in[i], e, v);
-    const double hx = vh[i].x + v;
+    const double hx = vh[i] + v;
     vhxc[i] = hx;
     const double vl = vext[i] + hx;
     vloc[i] = vl;
@@ -758,7 +692,7 @@ void launch_energies(const Tables &t, int nsys, const double *vhxc, const double
 
 void launch_mix(const Tables &t, int nsys, int max_nr, double *rho_in, const double *rho_out,
                 double *nin_hist, double *res_hist, const long long *hist_off, SysState *st, int H,
-                double *part, double2 *cgrid, double alpha, double q0, int max_n, const SpinGrids &sg,
+                double *part, double2 *cgrid, double *rwork, double alpha, double q0, int max_n, const SpinGrids &sg,
                 cudaStream_t s) {
   const int gx = (int)std::min<long long>(((long long)max_nr + 255) / 256, 256);
   derek::note_launch(), k_mix_store<<<dim3(gx, nsys), 256, 0, s>>>(t, rho_in, rho_out, nin_hist, res_hist, hist_off, st, H);
@@ -767,26 +701,17 @@ void launch_mix(const Tables &t, int nsys, int max_nr, double *rho_in, const dou
   if (sg.on) derek::note_launch(), k_mix_gram_m<<<dim3(RB, nsys), 256, 0, s>>>(t, sg, hist_off, st, H, part);
   derek::note_launch(), k_mix_solve<<<nsys, 32, 0, s>>>(t, nsys, part, st, H);
   const int kerker = q0 > 0;
-  derek::note_launch(), k_mix_combine<<<dim3(gx, nsys), 256, 0, s>>>(t, rho_in, nin_hist, res_hist, hist_off, st, cgrid,
+  derek::note_launch(), k_mix_combine<<<dim3(gx, nsys), 256, 0, s>>>(t, rho_in, nin_hist, res_hist, hist_off, st, rwork,
                                                alpha, kerker);
   if (sg.on) derek::note_launch(), k_mix_combine_m<<<dim3(gx, nsys), 256, 0, s>>>(t, sg, hist_off, st, alpha);
-  if (kerker) {
-    launch_fft3d_grid(t, 0, nsys, max_n, cgrid, -1, s);
-    derek::note_launch(), k_kerker_scale<<<dim3(gx, nsys), 256, 0, s>>>(t, cgrid, alpha, q0);
-    launch_fft3d_grid(t, 0, nsys, max_n, cgrid, +1, s);
-    derek::note_launch(), k_add_real<<<dim3(gx, nsys), 256, 0, s>>>(t, rho_in, cgrid);
-  }
+  if (kerker) launch_kerker_add(t, nsys, max_n, rwork, cgrid, alpha, q0, rho_in, s);
 }
 
-void launch_potential(const Tables &t, int nsys, int max_nr, int max_n, const double *rho_in,
-                      double2 *cgrid, const double *vext, double *vhxc, double *vloc, float *vloc32,
+void launch_potential(const Tables &t, int nsys, int max_n, const double *rho_in,
+                      double2 *cgrid, double *rwork, const double *vext, double *vhxc, double *vloc, float *vloc32,
                       double *part, SysState *st, int all, const SpinGrids &sg, cudaStream_t s) {
-  const int gx = (int)std::min<long long>(((long long)max_nr + 255) / 256, 256);
-  derek::note_launch(), k_real_to_complex<<<dim3(gx, nsys), 256, 0, s>>>(t, rho_in, cgrid, all);
-  launch_fft3d_grid(t, 0, nsys, max_n, cgrid, -1, s);
-  derek::note_launch(), k_hartree_scale<<<dim3(gx, nsys), 256, 0, s>>>(t, cgrid, all);
-  launch_fft3d_grid(t, 0, nsys, max_n, cgrid, +1, s);
-  derek::note_launch(), k_build_vloc<<<dim3(RB, nsys), 256, 0, s>>>(t, rho_in, cgrid, vext, vhxc, vloc, vloc32, part, all, sg);
+  launch_hartree(t, nsys, max_n, rho_in, cgrid, rwork, all, s);
+  derek::note_launch(), k_build_vloc<<<dim3(RB, nsys), 256, 0, s>>>(t, rho_in, rwork, vext, vhxc, vloc, vloc32, part, all, sg);
   derek::note_launch(), k_vmax_final<<<nsys, 32, 0, s>>>(t, nsys, part, st, all);
 }
 
@@ -805,13 +730,6 @@ void launch_lsda(long n, const double *rho_a, const double *rho_b, double *exc, 
                  cudaStream_t s) {
   const int blocks = (int)std::min<long>((n + 255) / 256, 152 * 8);
   derek::note_launch(), k_lsda<<<blocks, 256, 0, s>>>(n, rho_a, rho_b, exc, va, vb);
-}
-
-void launch_density_fft(const Tables &t, int nsys, int max_nr, int max_n, const double *rho,
-                        double2 *cgrid, cudaStream_t s) {
-  const int gx = (int)std::min<long long>(((long long)max_nr + 255) / 256, 256);
-  derek::note_launch(), k_real_to_complex<<<dim3(gx, nsys), 256, 0, s>>>(t, rho, cgrid, 0);
-  launch_fft3d_grid(t, 0, nsys, max_n, cgrid, -1, s);
 }
 
 void launch_uniform_density(const Tables &t, int nsys, int max_nr, double *rho, cudaStream_t s) {
@@ -905,16 +823,6 @@ void launch_hf_gradient(const Tables &t, int nsys, const double *rho, const doub
 }  // namespace derek
 
 namespace derek {
-
-// V_H[rho] into cgrid (.x), every system (FP64 grids).
-void launch_hartree_only(const Tables &t, int nsys, int max_nr, int max_n, const double *rho,
-                         double2 *cgrid, cudaStream_t s) {
-  const int gx = (int)std::min<long long>(((long long)max_nr + 255) / 256, 256);
-  derek::note_launch(), k_real_to_complex<<<dim3(gx, nsys), 256, 0, s>>>(t, rho, cgrid, 1);
-  launch_fft3d_grid(t, 0, nsys, max_n, cgrid, -1, s);
-  derek::note_launch(), k_hartree_scale<<<dim3(gx, nsys), 256, 0, s>>>(t, cgrid, 1);
-  launch_fft3d_grid(t, 0, nsys, max_n, cgrid, +1, s);
-}
 
 // dv_xc/dn at rho (central difference, relative step 1e-4; zero below 1e-10)
 __global__ void k_fxc(long long n, const double *__restrict__ rho, double *__restrict__ fxc) {

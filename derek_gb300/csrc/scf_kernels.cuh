@@ -44,20 +44,16 @@ void launch_energies(const Tables &t, int nsys, const double *vhxc, const double
                      SysDev *sys_rw, const int *ks_status, const SpinGrids &sg, cudaStream_t s);
 void launch_mix(const Tables &t, int nsys, int max_nr, double *rho_in, const double *rho_out,
                 double *nin_hist, double *res_hist, const long long *hist_off, SysState *st, int H,
-                double *part, double2 *cgrid, double alpha, double q0, int max_n, const SpinGrids &sg,
+                double *part, double2 *cgrid, double *rwork, double alpha, double q0, int max_n, const SpinGrids &sg,
                 cudaStream_t s);
-void launch_potential(const Tables &t, int nsys, int max_nr, int max_n, const double *rho_in,
-                      double2 *cgrid, const double *vext, double *vhxc, double *vloc, float *vloc32,
+void launch_potential(const Tables &t, int nsys, int max_n, const double *rho_in,
+                      double2 *cgrid, double *rwork, const double *vext, double *vhxc, double *vloc, float *vloc32,
                       double *part, SysState *st, int all, const SpinGrids &sg, cudaStream_t s);
 void launch_lsda(long n, const double *rho_a, const double *rho_b, double *exc, double *va, double *vb,
                  cudaStream_t s);
-void launch_density_fft(const Tables &t, int nsys, int max_nr, int max_n, const double *rho,
-                        double2 *cgrid, cudaStream_t s);
 void launch_hf_gradient(const Tables &t, int nsys, const double *rho, const double *wells,
                         const int *well_off, const double *cells, double *part, int max_wells,
                         double *grad, cudaStream_t s);
-void launch_hartree_only(const Tables &t, int nsys, int max_nr, int max_n, const double *rho,
-                         double2 *cgrid, cudaStream_t s);
 void launch_fxc(long long n, const double *rho, double *fxc, cudaStream_t s);
 void launch_uniform_density(const Tables &t, int nsys, int max_nr, double *rho, cudaStream_t s);
 

@@ -121,3 +121,39 @@ def test_jacobi_solves(oracle, nb, nk):
             # Ritz vectors diagonalise H: rounding times ||H|| ~ 20 Ha
             assert np.max(np.abs(hs - np.diag(eig[k]))) < 1e-10
             assert np.all(np.diff(eig[k]) >= 0)
+
+
+# half spectra of real grids: odd and even axes (an odd count of rows leaves
+# one row without a partner), Nyquist planes of a sheared cell, several tiles.
+# The Hartree potential and E_H of a density against full complex transforms
+@pytest.mark.parametrize("n", [(11, 13, 9), (16, 12, 20), (27, 32, 25), (36, 33, 40)])
+@pytest.mark.parametrize("kerker", [0.0, 0.8])
+def test_hartree_half_spectra(oracle, n, kerker):
+    import derek_gb300 as dg
+    cell = np.array([[6.0, 0.9, 0.3], [0.0, 6.5, -0.8], [0.2, 0.0, 5.5]])
+    wells = np.array([[0.3, 0.4, 0.5, 1.5, 1.2]])
+    spec = dg.SystemSpec(cell, 1.1, [[0, 0, 0]], 4, 2.0, kT=0.05, wells=wells, n_fine=n)
+    nr = int(np.prod(n))
+    with dg.Handle(spec, kerker_q0=kerker, mix_alpha=0.5, first_passes=1) as h:
+        rng = np.random.default_rng(nr)
+        rho0 = np.abs(1.0 + 0.5 * rng.standard_normal(nr)) * 2.0 / abs(np.linalg.det(cell))
+        h.set_start_density(rho0)
+        rep = h.scf_iterate()[0]
+        rho1, v1, vext = h.density(), h.get_vloc(), h.get_vext()
+    inv = 2 * np.pi * np.linalg.inv(cell).T
+    ax = [np.where(np.arange(k) < k - k // 2, np.arange(k), np.arange(k) - k) for k in n]
+    g2 = ((np.stack(np.meshgrid(*ax, indexing="ij"), -1) @ inv.T) ** 2).sum(-1)
+    ig2 = np.divide(1.0, g2, out=np.zeros_like(g2), where=g2 > 0)
+
+    def conv(f, kernel):
+        return np.fft.ifftn(np.fft.fftn(f.reshape(n)) * kernel).real.ravel()
+
+    vol = abs(np.linalg.det(cell))
+    eh = 2 * np.pi * vol * np.sum(np.abs(np.fft.fftn(rho1.reshape(n)) / nr) ** 2 * ig2)
+    assert abs(rep["e_hartree"] - eh) < 1e-11 * abs(eh)
+    # the next input density (linear mixing, one stored pair) and its potential
+    res = rho1 - rho0
+    rho_in = rho0 + (conv(res, 0.5 * g2 / (g2 + kerker ** 2)) if kerker > 0 else 0.5 * res)
+    vh = conv(rho_in, 4 * np.pi * ig2)
+    vxc = oracle.lda_exc_vxc(rho_in)[1]
+    assert rel_err(v1, vext + vh + vxc) < 1e-11
