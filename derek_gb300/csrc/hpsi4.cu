@@ -28,10 +28,11 @@
 
 namespace derek {
 
-constexpr int kCC = kColChunk;
 
-// 16 warps on an SM, the two blocks its shared memory holds at 72^2 FP64 planes
-constexpr int kLineThreads = 256;
+// Three blocks of six warps per SM where the planes fit (two at 72^2 FP64), whose
+// barriers overlap.  FP64 plane pass, threads x blocks 192 x 3, 256 x 2, 128 x 4,
+// 384 x 1: 12 items of 32^3 47, 54, 47, 67 us; 336 of 72^3 11.8, 11.8, 11.9, 12.7 ms.
+constexpr int kLineThreads = 192, kLineBlocks = 3;
 
 template <typename R>
 __device__ __forceinline__ void load_tw(cplx<R> *dst, const cplx<R> *src, int n) {
@@ -40,14 +41,14 @@ __device__ __forceinline__ void load_tw(cplx<R> *dst, const cplx<R> *src, int n)
 
 // ---- pass 1: backward x transforms of the sphere's columns ----------------
 template <typename R>
-__global__ void __launch_bounds__(kLineThreads, 2) k_x_inv(Tables t, int item_begin, const cplx<R> *__restrict__ psi,
+__global__ void __launch_bounds__(kLineThreads, kLineBlocks) k_x_inv(Tables t, int item_begin, int cc, const cplx<R> *__restrict__ psi,
                                                         cplx<R> *__restrict__ abuf,
                                                         const double *__restrict__ occ_skip) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int item = t.item_list ? t.item_list[blockIdx.x] : item_begin + blockIdx.x;
   const int ksi = t.item_ks[item];
   const KSetDev &K = t.ks[ksi];
-  const int c0 = blockIdx.y * kCC;
+  const int c0 = blockIdx.y * cc;
   if (c0 >= K.ncol) return;
   const SysDev &S = t.sys[K.sys];
   if (!S.active) return;
@@ -55,9 +56,9 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_x_inv(Tables t, int item_be
   const int b = t.item_band[item];
   const int n1 = S.n[0];
   const int pl = n1 | 1;  // odd line pitch
-  const int nc = min(kCC, K.ncol - c0);
+  const int nc = min(cc, K.ncol - c0);
   cplx<R> *L = reinterpret_cast<cplx<R> *>(smem_raw);
-  cplx<R> *tw = L + kCC * pl;
+  cplx<R> *tw = L + cc * pl;
   for (int i = threadIdx.x; i < nc * pl; i += blockDim.x) L[i] = mk<R>(0, 0);
   load_tw<R>(tw, twtab<R>(t) + S.lp[0].tw_off, n1);
   __syncthreads();
@@ -82,7 +83,7 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_x_inv(Tables t, int item_be
 // register lines).  One plane per block, several blocks per SM: while one
 // waits at a step's barrier the others keep the pipe busy.
 template <typename R>
-__global__ void __launch_bounds__(kLineThreads, 2) k_plane(Tables t, int item_begin, cplx<R> *__restrict__ abuf,
+__global__ void __launch_bounds__(kLineThreads, kLineBlocks) k_plane(Tables t, int item_begin, cplx<R> *__restrict__ abuf,
                                                         const R *__restrict__ vloc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int item = t.item_list ? t.item_list[blockIdx.x] : item_begin + blockIdx.x;
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_plane(Tables t, int item_be
 
 // ---- pass 3: forward x transforms, gather, kinetic, epilogue --------------
 template <typename R>
-__global__ void __launch_bounds__(kLineThreads, 2) k_x_fwd(Tables t, int item_begin, const cplx<R> *__restrict__ abuf,
+__global__ void __launch_bounds__(kLineThreads, kLineBlocks) k_x_fwd(Tables t, int item_begin, int cc, const cplx<R> *__restrict__ abuf,
                                                         const cplx<R> *__restrict__ psi,
                                                         const cplx<R> *__restrict__ prev,
                                                         cplx<R> *__restrict__ out,
@@ -126,16 +127,16 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_x_fwd(Tables t, int item_be
   const int item = t.item_list ? t.item_list[blockIdx.x] : item_begin + blockIdx.x;
   const int ksi = t.item_ks[item];
   const KSetDev &K = t.ks[ksi];
-  const int c0 = blockIdx.y * kCC;
+  const int c0 = blockIdx.y * cc;
   if (c0 >= K.ncol) return;
   const SysDev &S = t.sys[K.sys];
   if (!S.active) return;
   const int b = t.item_band[item];
   const int n1 = S.n[0];
   const int pl = n1 | 1;
-  const int nc = min(kCC, K.ncol - c0);
+  const int nc = min(cc, K.ncol - c0);
   cplx<R> *L = reinterpret_cast<cplx<R> *>(smem_raw);
-  cplx<R> *tw = L + kCC * pl;
+  cplx<R> *tw = L + cc * pl;
   load_tw<R>(tw, twtab<R>(t) + S.lp[0].tw_off, n1);
   const cplx<R> *src = abuf + K.a_off + (long long)b * n1 * K.ncol_pad + c0;
   for (int x = threadIdx.x >> 5; x < n1; x += blockDim.x >> 5) {
@@ -182,7 +183,7 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_x_fwd(Tables t, int item_be
 __host__ __device__ constexpr int density_acc_count(int points) { return (points + 1) & ~1; }
 
 template <typename R>
-__global__ void __launch_bounds__(kLineThreads, 2) k_density_plane(Tables t, const DensityUnit *__restrict__ units,
+__global__ void __launch_bounds__(kLineThreads, kLineBlocks) k_density_plane(Tables t, const DensityUnit *__restrict__ units,
                                                        const cplx<R> *__restrict__ abuf,
                                                        const double *__restrict__ occ,
                                                        double *__restrict__ partial) {
@@ -233,8 +234,16 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_density_plane(Tables t, con
 }
 
 // ---- launchers --------------------------------------------------------------
-template <typename R> static size_t smem_x(int max_n1) {
-  return ((size_t)kCC * (max_n1 | 1) + max_n1) * sizeof(cplx<R>);
+// Columns of an x-pass block: 64, or 32 or 16 where the wider chunks would leave
+// SMs without a block (12 items of a 32^3 grid are 36 blocks of 64 columns: x
+// passes 17 and 21 us, 12 and 15 us with 16)
+static int x_columns(int nitems, int max_ncol) {
+  int cc = kColChunk;
+  while (cc > 16 && (long long)nitems * ((max_ncol + cc - 1) / cc) < 2 * sm_count()) cc /= 2;
+  return cc;
+}
+template <typename R> static size_t smem_x(int max_n1, int cc) {
+  return ((size_t)cc * (max_n1 | 1) + max_n1) * sizeof(cplx<R>);
 }
 template <typename R> static size_t smem_plane(int max_n2, int max_n3) {
   return ((size_t)max_n2 * (max_n3 | 1) + max_n2 + max_n3) * sizeof(cplx<R>);
@@ -248,12 +257,13 @@ void launch_x_inv(const Tables &t, int item_begin, int nitems, int max_nchunk, i
   if (nitems <= 0) return;
   if constexpr (std::is_same<R, float>::value) {
     if (max_n1 == min_n1 &&
-        launch_xinv_reg(t, item_begin, nitems, max_nchunk * kCC, max_n1, max_m, psi, abuf, occ_skip, st))
+        launch_xinv_reg(t, item_begin, nitems, max_nchunk * kColChunk, max_n1, max_m, psi, abuf, occ_skip, st))
       return;
   }
-  const size_t sm = smem_x<R>(max_n1);
+  const int ncol = max_nchunk * kColChunk, cc = x_columns(nitems, ncol);
+  const size_t sm = smem_x<R>(max_n1, cc);
   cudaFuncSetAttribute(k_x_inv<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::note_launch(), k_x_inv<R><<<dim3(nitems, max_nchunk), kLineThreads, sm, st>>>(t, item_begin, psi, abuf, occ_skip);
+  derek::note_launch(), k_x_inv<R><<<dim3(nitems, (ncol + cc - 1) / cc), kLineThreads, sm, st>>>(t, item_begin, cc, psi, abuf, occ_skip);
 }
 
 template <typename R>
@@ -263,12 +273,13 @@ void launch_x_fwd(const Tables &t, int item_begin, int nitems, int max_nchunk, i
   if (nitems <= 0) return;
   if constexpr (std::is_same<R, float>::value) {
     if (max_n1 == min_n1 &&
-        launch_xfwd_reg(t, item_begin, nitems, max_nchunk * kCC, max_n1, max_m, abuf, psi, prev, out, coef, st))
+        launch_xfwd_reg(t, item_begin, nitems, max_nchunk * kColChunk, max_n1, max_m, abuf, psi, prev, out, coef, st))
       return;
   }
-  const size_t sm = smem_x<R>(max_n1);
+  const int ncol = max_nchunk * kColChunk, cc = x_columns(nitems, ncol);
+  const size_t sm = smem_x<R>(max_n1, cc);
   cudaFuncSetAttribute(k_x_fwd<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::note_launch(), k_x_fwd<R><<<dim3(nitems, max_nchunk), kLineThreads, sm, st>>>(t, item_begin, abuf, psi, prev, out, coef);
+  derek::note_launch(), k_x_fwd<R><<<dim3(nitems, (ncol + cc - 1) / cc), kLineThreads, sm, st>>>(t, item_begin, cc, abuf, psi, prev, out, coef);
 }
 
 template <typename R>

@@ -88,7 +88,7 @@ void launch_density_spinor(const Tables &t, const DensityUnit *units, int nunits
                            const cplx<R> *abuf, const double *occ, double *partial, cudaStream_t st);
 size_t spinor_plane_smem(int n2, int n3, size_t elem);
 
-constexpr int kColChunk = 64;   // columns per x-line chunk (kCC in hpsi4.cu)
+constexpr int kColChunk = 64;   // most columns per x-line chunk (hpsi4.cu)
 
 // FP32 (y,z)-plane passes with register-resident line transforms
 // (hpsi_reg.cu), for cubic-plane lengths n in {24, 27, 32, 36, 48, 54, 64, 72};
