@@ -32,6 +32,7 @@ namespace {
 
 __global__ void k_lincomb(long long n, double a, const double2 *__restrict__ X, double b,
                           const double2 *__restrict__ Y, double2 *__restrict__ out) {
+  grid_dependency();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     const double2 x = X[i];
@@ -43,6 +44,7 @@ __global__ void k_lincomb(long long n, double a, const double2 *__restrict__ X, 
 // d[item] = Re <X_item | Y_item>
 __global__ void k_item_dot(const Tables t, const double2 *__restrict__ X, const double2 *__restrict__ Y,
                            double *__restrict__ d) {
+  grid_dependency();
   __shared__ double red[256];
   const int item = blockIdx.x;
   const KSetDev &K = t.ks[t.item_ks[item]];
@@ -64,6 +66,7 @@ __global__ void k_item_dot(const Tables t, const double2 *__restrict__ X, const 
 // Y_item += sign * c[item] * X_item   (or, with xpay, Y = X + c Y)
 __global__ void k_item_axpy(const Tables t, const double *__restrict__ c, double sign,
                             const double2 *__restrict__ X, double2 *__restrict__ Y, int xpay) {
+  grid_dependency();
   const int item = blockIdx.x;
   const KSetDev &K = t.ks[t.item_ks[item]];
   const long long off = K.psi_off + (long long)t.item_band[item] * K.npw_pad;
@@ -84,6 +87,7 @@ __global__ void k_item_axpy(const Tables t, const double *__restrict__ c, double
 // Z = R / (1/2|k+G|^2 + 1), rows of items with mask[item] == 0 set to zero
 __global__ void k_precond(const Tables t, const double2 *__restrict__ R, const double *__restrict__ mask,
                           double2 *__restrict__ Z) {
+  grid_dependency();
   const int item = blockIdx.x;
   const KSetDev &K = t.ks[t.item_ks[item]];
   const long long off = K.psi_off + (long long)t.item_band[item] * K.npw_pad;
@@ -101,6 +105,7 @@ __global__ void __launch_bounds__(256) k_gemm_sub(const Tables t, const double2 
                                                   const double2 *__restrict__ C,
                                                   const long long *__restrict__ mat_off,
                                                   double2 *__restrict__ Y) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ksi = blockIdx.y;
   const KSetDev &K = t.ks[ksi];
@@ -131,6 +136,7 @@ __global__ void __launch_bounds__(256) k_gemm_sub(const Tables t, const double2 
 __global__ void k_pair_weights(const Tables t, const double *__restrict__ eig,
                                const double *__restrict__ occ, const double2 *__restrict__ V,
                                const long long *__restrict__ mat_off, double2 *__restrict__ W) {
+  grid_dependency();
   const int ksi = blockIdx.x;
   const KSetDev &K = t.ks[ksi];
   const SysDev &S = t.sys[K.sys];
@@ -155,6 +161,7 @@ __global__ void k_pair_weights(const Tables t, const double *__restrict__ eig,
 // CG scalar updates per item: alpha = rz / pAp (masked), beta = rz_new / rz
 __global__ void k_cg_ratio(int n, const double *__restrict__ num, const double *__restrict__ den,
                            const double *__restrict__ mask, double *__restrict__ out) {
+  grid_dependency();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double d = den[i];
@@ -163,6 +170,7 @@ __global__ void k_cg_ratio(int n, const double *__restrict__ num, const double *
 
 __global__ void k_scale_grid(long long n, const double *__restrict__ a, double sa,
                              const double *__restrict__ b, double sb, double *__restrict__ out) {
+  grid_dependency();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     out[i] = sa * a[i] + (b ? sb * b[i] : 0.0);
@@ -172,6 +180,7 @@ __global__ void k_scale_grid(long long n, const double *__restrict__ a, double s
 __global__ void k_response_potential(long long n, const double *__restrict__ g,
                                      const double *__restrict__ vh, const double *__restrict__ fxc,
                                      const double *__restrict__ dn, double *__restrict__ dv) {
+  grid_dependency();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     dv[i] = g[i] + vh[i] + fxc[i] * dn[i];
@@ -287,7 +296,7 @@ extern "C" int derek_gpu_grad_density_loss(derek_gpu_t *h, int s, const double *
     ts.item_shift = W.shift;
     int e0 = apply_h_items_ex(h, ts, 0, ni, psi, nullptr, W.ap, nullptr, h->d_vloc);
     if (e0) return e0;
-    derek::note_launch(), k_item_dot<<<ni, 256, 0, st>>>(t, W.ap, W.ap, W.pap);
+    derek::launch(k_item_dot, ni, 256, 0, st, t, W.ap, W.ap, W.pap);
     CKA(cudaMemcpyAsync(rres.data(), W.pap, ni * sizeof(double), cudaMemcpyDeviceToHost, st));
     CKA(cudaStreamSynchronize(st));
   }
@@ -346,14 +355,14 @@ extern "C" int derek_gpu_grad_density_loss(derek_gpu_t *h, int s, const double *
   auto cross_density = [&](const double2 *a, const double2 *b, const std::vector<double> &wts,
                            double *out) -> int {
     const int blocks = 152 * 8;
-    derek::note_launch(), k_lincomb<<<blocks, 256, 0, st>>>(np, 1.0, a, 1.0, b, W.sp);
-    derek::note_launch(), k_lincomb<<<blocks, 256, 0, st>>>(np, 1.0, a, -1.0, b, W.sm);
+    derek::launch(k_lincomb, blocks, 256, 0, st, np, 1.0, a, 1.0, b, W.sp);
+    derek::launch(k_lincomb, blocks, 256, 0, st, np, 1.0, a, -1.0, b, W.sm);
     int e = density_with(W.sp, wts, h->d_rho_in);  // scratch grid
     if (e) return e;
-    derek::note_launch(), k_scale_grid<<<152, 256, 0, st>>>(nr, h->d_rho_in + S.grid_off, 1.0, nullptr, 0.0, W.tmp);
+    derek::launch(k_scale_grid, 152, 256, 0, st, nr, h->d_rho_in + S.grid_off, 1.0, nullptr, 0.0, W.tmp);
     e = density_with(W.sm, wts, h->d_rho_in);
     if (e) return e;
-    derek::note_launch(), k_scale_grid<<<152, 256, 0, st>>>(nr, W.tmp, 1.0, h->d_rho_in + S.grid_off, -1.0, out);
+    derek::launch(k_scale_grid, 152, 256, 0, st, nr, W.tmp, 1.0, h->d_rho_in + S.grid_off, -1.0, out);
     return 0;
   };
   // P_c y = y - Psi (Psi^H y)
@@ -362,7 +371,7 @@ extern "C" int derek_gpu_grad_density_loss(derek_gpu_t *h, int s, const double *
                            h->d_opart_off, h->d_S, h->d_mat_off, 0, st);
     const size_t sm = (size_t)h->max_nb * h->max_nb * sizeof(double2);
     cudaFuncSetAttribute(k_gemm_sub, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    derek::note_launch(), k_gemm_sub<<<dim3((h->max_npw + 31) / 32, h->nks), 256, sm, st>>>(tM, psi, h->d_S, h->d_mat_off, y);
+    derek::launch(k_gemm_sub, dim3((h->max_npw + 31) / 32, h->nks), 256, sm, st, tM, psi, h->d_S, h->d_mat_off, y);
   };
   // Fermi-level density n_F (fixed for the whole solve); rho_in and the item
   // weights are used as scratch and restored at the end
@@ -383,7 +392,7 @@ extern "C" int derek_gpu_grad_density_loss(derek_gpu_t *h, int s, const double *
   for (int iter = 0; iter < max_iter && !converged; ++iter) {
     CKA(cudaMemcpyAsync(W.dn, dn.data(), nr * sizeof(double), cudaMemcpyHostToDevice, st));
     launch_hartree(t, 1, h->max_nmax, W.dn - S.grid_off, h->d_cgrid, h->d_rwork, 1, st);
-    derek::note_launch(), k_response_potential<<<152, 256, 0, st>>>(nr, W.g, h->d_rwork + S.grid_off, W.fxc, W.dn, W.dv);
+    derek::launch(k_response_potential, 152, 256, 0, st, nr, W.g, h->d_rwork + S.grid_off, W.fxc, W.dn, W.dv);
     // phi = dV psi
     {
       int e2 = apply_h_items_ex(h, t, 0, ni, psi, nullptr, W.phi, W.vcoef, W.dv);
@@ -392,7 +401,7 @@ extern "C" int derek_gpu_grad_density_loss(derek_gpu_t *h, int s, const double *
     // V_mn and the pair orbitals xi = psi W
     launch_overlap<double>(tM, 0, h->nks, h->max_nb, h->max_npw, h->tune.ksplit, h->split_min, psi, W.phi, h->d_opart,
                            h->d_opart_off, h->d_Hs, h->d_mat_off, 1, st);
-    derek::note_launch(), k_pair_weights<<<h->nks, 256, 0, st>>>(tM, h->d_eig, h->d_occ, h->d_Hs, h->d_mat_off, h->d_C);
+    derek::launch(k_pair_weights, h->nks, 256, 0, st, tM, h->d_eig, h->d_occ, h->d_Hs, h->d_mat_off, h->d_C);
     CKA(cudaMemcpyAsync(W.xi, psi, np * sizeof(double2), cudaMemcpyDeviceToDevice, st));
     launch_rotate<double>(tM, 0, h->nks, h->max_nb, h->max_npw, W.xi, h->d_C, h->d_mat_off, 0, st);
     e = cross_density(psi, W.xi, w_pair, W.dn_out);
@@ -420,17 +429,17 @@ extern "C" int derek_gpu_grad_density_loss(derek_gpu_t *h, int s, const double *
       CKA(cudaMemcpyAsync(W.alpha, negmask.data(), ni * sizeof(double), cudaMemcpyHostToDevice, st));
       CKA(cudaMemsetAsync(W.x, 0, np * sizeof(double2), st));
       // x = 0 + (-mask) * r  -> x holds b; then r = b
-      derek::note_launch(), k_item_axpy<<<ni, 256, 0, st>>>(t, W.alpha, 1.0, W.r, W.x, 0);
+      derek::launch(k_item_axpy, ni, 256, 0, st, t, W.alpha, 1.0, W.r, W.x, 0);
       CKA(cudaMemcpyAsync(W.r, W.x, np * sizeof(double2), cudaMemcpyDeviceToDevice, st));
       CKA(cudaMemsetAsync(W.x, 0, np * sizeof(double2), st));
     }
-    derek::note_launch(), k_item_dot<<<ni, 256, 0, st>>>(t, W.r, W.r, W.rz2);  // |b|^2
+    derek::launch(k_item_dot, ni, 256, 0, st, t, W.r, W.r, W.rz2);  // |b|^2
     std::vector<double> bnorm(ni), rnorm(ni);
     CKA(cudaMemcpyAsync(bnorm.data(), W.rz2, ni * sizeof(double), cudaMemcpyDeviceToHost, st));
-    derek::note_launch(), k_precond<<<ni, 256, 0, st>>>(t, W.r, W.mask, W.z);
+    derek::launch(k_precond, ni, 256, 0, st, t, W.r, W.mask, W.z);
     project(W.z);
     CKA(cudaMemcpyAsync(W.p, W.z, np * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-    derek::note_launch(), k_item_dot<<<ni, 256, 0, st>>>(t, W.r, W.z, W.rz);
+    derek::launch(k_item_dot, ni, 256, 0, st, t, W.r, W.z, W.rz);
     const double cg_tol = std::max(std::min(1e-6, tol * 0.1), 1e-12);
     for (int cg = 0; cg < 200; ++cg) {
       // ap = P_c (H - e_n) p
@@ -441,29 +450,29 @@ extern "C" int derek_gpu_grad_density_loss(derek_gpu_t *h, int s, const double *
         if (e2) return e2;
       }
       project(W.ap);
-      derek::note_launch(), k_item_dot<<<ni, 256, 0, st>>>(t, W.p, W.ap, W.pap);
-      derek::note_launch(), k_cg_ratio<<<(ni + 127) / 128, 128, 0, st>>>(ni, W.rz, W.pap, W.mask, W.alpha);
-      derek::note_launch(), k_item_axpy<<<ni, 256, 0, st>>>(t, W.alpha, 1.0, W.p, W.x, 0);
-      derek::note_launch(), k_item_axpy<<<ni, 256, 0, st>>>(t, W.alpha, -1.0, W.ap, W.r, 0);
-      derek::note_launch(), k_item_dot<<<ni, 256, 0, st>>>(t, W.r, W.r, W.pap);
+      derek::launch(k_item_dot, ni, 256, 0, st, t, W.p, W.ap, W.pap);
+      derek::launch(k_cg_ratio, (ni + 127) / 128, 128, 0, st, ni, W.rz, W.pap, W.mask, W.alpha);
+      derek::launch(k_item_axpy, ni, 256, 0, st, t, W.alpha, 1.0, W.p, W.x, 0);
+      derek::launch(k_item_axpy, ni, 256, 0, st, t, W.alpha, -1.0, W.ap, W.r, 0);
+      derek::launch(k_item_dot, ni, 256, 0, st, t, W.r, W.r, W.pap);
       CKA(cudaMemcpyAsync(rnorm.data(), W.pap, ni * sizeof(double), cudaMemcpyDeviceToHost, st));
       CKA(cudaStreamSynchronize(st));
       bool done = true;
       for (int it = 0; it < ni; ++it)
         if (mask[it] != 0.0 && rnorm[it] > cg_tol * cg_tol * std::max(bnorm[it], 1e-300)) done = false;
       if (done) break;
-      derek::note_launch(), k_precond<<<ni, 256, 0, st>>>(t, W.r, W.mask, W.z);
+      derek::launch(k_precond, ni, 256, 0, st, t, W.r, W.mask, W.z);
       project(W.z);
-      derek::note_launch(), k_item_dot<<<ni, 256, 0, st>>>(t, W.r, W.z, W.rz2);
-      derek::note_launch(), k_cg_ratio<<<(ni + 127) / 128, 128, 0, st>>>(ni, W.rz2, W.rz, W.mask, W.beta);
-      derek::note_launch(), k_item_axpy<<<ni, 256, 0, st>>>(t, W.beta, 1.0, W.z, W.p, 1);
+      derek::launch(k_item_dot, ni, 256, 0, st, t, W.r, W.z, W.rz2);
+      derek::launch(k_cg_ratio, (ni + 127) / 128, 128, 0, st, ni, W.rz2, W.rz, W.mask, W.beta);
+      derek::launch(k_item_axpy, ni, 256, 0, st, t, W.beta, 1.0, W.z, W.p, 1);
       std::swap(W.rz, W.rz2);
     }
     e = cross_density(psi, W.x, w_stern, W.tmp);
     if (e) return e;
     // dn_out = pair + Sternheimer - dmu n_F
-    derek::note_launch(), k_scale_grid<<<152, 256, 0, st>>>(nr, W.dn_out, 1.0, W.tmp, 1.0, W.dn_out);
-    derek::note_launch(), k_scale_grid<<<152, 256, 0, st>>>(nr, W.dn_out, 1.0, W.nf, -dmu, W.dn_out);
+    derek::launch(k_scale_grid, 152, 256, 0, st, nr, W.dn_out, 1.0, W.tmp, 1.0, W.dn_out);
+    derek::launch(k_scale_grid, 152, 256, 0, st, nr, W.dn_out, 1.0, W.nf, -dmu, W.dn_out);
     CKA(cudaMemcpyAsync(dn_out.data(), W.dn_out, nr * sizeof(double), cudaMemcpyDeviceToHost, st));
     CKA(cudaStreamSynchronize(st));
     // convergence and Anderson update on the host

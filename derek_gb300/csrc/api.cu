@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(256) k_reduce_partials(const SysDev *__restric
                                                          const int *__restrict__ sys_units,
                                                          double *__restrict__ rho, double *__restrict__ mag,
                                                          long long mag_stride) {
+  grid_dependency();
   const SysDev &S = sys[blockIdx.y];
   const int c = blockIdx.z, nc = S.nspinor == 2 ? 4 : 1;
   if (!S.active || c >= nc || (gridDim.z == 4 && nc == 1)) return;
@@ -50,6 +51,7 @@ __global__ void __launch_bounds__(256) k_reduce_partials(const SysDev *__restric
 }
 
 __global__ void k_to_float(long long n, const double *__restrict__ a, float *__restrict__ b) {
+  grid_dependency();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     b[i] = (float)a[i];
@@ -169,8 +171,7 @@ template <typename R> static void density_t(derek_gpu *h, const void *psi) {
 // partial grids of every active system into rho (and h->d_mag)
 static void reduce_partials(derek_gpu *h, double *rho, int components) {
   const int gx = (int)std::min<long long>((h->max_nr + 255) / 256, 152 * 4);
-  derek::note_launch(), k_reduce_partials<<<dim3(gx, h->nsys, components), 256, 0, h->stream>>>(
-      h->d_sys, h->d_partial, h->d_sys_part, h->d_sys_units, rho, h->d_mag, h->total_grid);
+  derek::launch(k_reduce_partials, dim3(gx, h->nsys, components), 256, 0, h->stream, h->d_sys, h->d_partial, h->d_sys_part, h->d_sys_units, rho, h->d_mag, h->total_grid);
 }
 
 int density_items(derek_gpu *h, const void *psi, double *rho) {
@@ -258,7 +259,7 @@ bool reject_spinor(derek_gpu *h, const char *what) {
 
 int refresh_vloc32(derek_gpu *h) {
   if (h->prec != DEREK_PREC_FP64)
-    derek::note_launch(), k_to_float<<<152 * 4, 256, 0, h->stream>>>(h->total_grid, h->d_vloc, h->d_vloc32);
+    derek::launch(k_to_float, 152 * 4, 256, 0, h->stream, h->total_grid, h->d_vloc, h->d_vloc32);
   DEREK_CUDA(h, cudaGetLastError());
   return DEREK_OK;
 }

@@ -171,6 +171,65 @@ struct DensityUnit {
 void note_launch(long long n = 1);
 unsigned long long launch_total();
 
+// Programmatic dependent launch.  Every kernel begins with grid_dependency():
+// it lets the stream's next kernel become resident as soon as the last of this
+// one's blocks has started, and then waits until the previous kernel has
+// completed and its writes are visible.  Nothing runs ahead of the wait, so the
+// order of work is the stream's; what goes is the launch gap between kernels.
+// Only for grids of at most a block per SM, straight into a stream (the adjoint
+// gradient's thousands of small kernels 138 -> 119 ms, a Gamma SCF's first pass 6.4 ->
+// 6.1 ms in all).  Larger grids start unevenly around
+// the waiting predecessor's blocks (band structure 23.4 against 25.1 ms, spinor
+// SCF 21.6 against 22.7 ms), and a graph's own edges are faster than programmatic
+// ones (Gamma SCF 6.4 against 6.9 ms, 64 k-points 320 against 327 ms).  Launched
+// plainly, grid_dependency() does nothing.
+__device__ __forceinline__ void grid_dependency() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+inline int sm_count() {
+  static int n = [] {
+    int dev = 0, c = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
+    return c > 0 ? c : 1;
+  }();
+  return n;
+}
+
+inline bool programmatic_launch(dim3 grid, cudaStream_t stream) {
+  if ((long long)grid.x * grid.y * grid.z > sm_count()) return false;
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(stream, &c) == cudaSuccess && c == cudaStreamCaptureStatusNone;
+}
+template <typename... P, typename... A>
+void launch_with(bool programmatic, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                 A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = programmatic ? 1 : 0;
+  note_launch();
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+  launch_with(programmatic_launch(grid, stream), kernel, grid, block, smem, stream, args...);
+}
+// Long FP64 solves want an SM to each block, which the scheduler gives them once
+// the predecessor has left (a band structure of 40 k-points, whose solves doubled
+// up on SMs otherwise: 23.4 against 29.1 ms)
+template <typename... P, typename... A>
+void launch_plain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+  launch_with(false, kernel, grid, block, smem, stream, args...);
+}
+
 // Error codes mirrored from the C ABI.
 enum Status : int {
   OK = DEREK_OK,

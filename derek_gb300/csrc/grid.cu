@@ -26,6 +26,7 @@ __device__ __forceinline__ void load_plan_tw(double2 *tw, const Tables &t, const
 // z pass, complex rows in place
 template <int SIGN>
 __global__ void __launch_bounds__(kGridThreads) k_rows(Tables t, int sys_begin, double2 *__restrict__ data) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SysDev &S = t.sys[sys_begin + blockIdx.y];
   const int n3 = S.n[2], rows = S.n[0] * S.n[1], l0 = blockIdx.x * kRowTile;
@@ -44,6 +45,7 @@ __global__ void __launch_bounds__(kGridThreads) k_rows(Tables t, int sys_begin, 
 // Z = A + i B; A(k) = (Z(k) + conj Z(-k)) / 2, B(k) = (Z(k) - conj Z(-k)) / 2i
 __global__ void __launch_bounds__(kGridThreads) k_rows_r2c(Tables t, const double *__restrict__ rho,
                                                            double2 *__restrict__ data, int all) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SysDev &S = t.sys[blockIdx.y];
   if (!all && !S.active) return;
@@ -73,6 +75,7 @@ __global__ void __launch_bounds__(kGridThreads) k_rows_r2c(Tables t, const doubl
 template <bool ADD>
 __global__ void __launch_bounds__(kGridThreads) k_rows_c2r(Tables t, const double2 *__restrict__ data,
                                                            double *__restrict__ out, int all) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SysDev &S = t.sys[blockIdx.y];
   if (!all && !S.active) return;
@@ -109,6 +112,7 @@ __global__ void __launch_bounds__(kGridThreads) k_rows_c2r(Tables t, const doubl
 template <int SIGN>
 __global__ void __launch_bounds__(kGridThreads) k_cols_y(Tables t, int sys_begin, double2 *__restrict__ data, int tz,
                                                          int half, int all) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SysDev &S = t.sys[sys_begin + blockIdx.z];
   const int n2 = S.n[1], n3 = S.n[2], nz = half ? n3 / 2 + 1 : n3, x = blockIdx.y, z0 = blockIdx.x * tz;
@@ -131,6 +135,7 @@ enum { kPlain = 0, kHartree = 1, kKerker = 2 };
 template <int SIGN, int MODE>
 __global__ void __launch_bounds__(kGridThreads) k_cols_x(Tables t, int sys_begin, double2 *__restrict__ data, int tz,
                                                          int half, int all, double alpha, double q0) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SysDev &S = t.sys[sys_begin + blockIdx.z];
   const int n1 = S.n[0], n2 = S.n[1], n3 = S.n[2], nz = half ? n3 / 2 + 1 : n3, y = blockIdx.y, z0 = blockIdx.x * tz;
@@ -188,22 +193,22 @@ struct GridShape {
 
 template <int SIGN> void cols_y(const GridShape &g, const Tables &t, int s0, double2 *data, int half, int all, cudaStream_t st) {
   cudaFuncSetAttribute(k_cols_y<SIGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.cols);
-  derek::note_launch(), k_cols_y<SIGN><<<g.col_grid(half), kGridThreads, g.cols, st>>>(t, s0, data, g.tz, half, all);
+  derek::launch(k_cols_y<SIGN>, g.col_grid(half), kGridThreads, g.cols, st, t, s0, data, g.tz, half, all);
 }
 template <int SIGN, int MODE>
 void cols_x(const GridShape &g, const Tables &t, int s0, double2 *data, int half, int all, double alpha, double q0,
             cudaStream_t st) {
   cudaFuncSetAttribute(k_cols_x<SIGN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.cols);
-  derek::note_launch(), k_cols_x<SIGN, MODE><<<g.col_grid(half), kGridThreads, g.cols, st>>>(t, s0, data, g.tz, half,
+  derek::launch(k_cols_x<SIGN, MODE>, g.col_grid(half), kGridThreads, g.cols, st, t, s0, data, g.tz, half,
                                                                                             all, alpha, q0);
 }
 void rows_r2c(const GridShape &g, const Tables &t, const double *rho, double2 *data, int all, cudaStream_t st) {
   cudaFuncSetAttribute(k_rows_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.rows);
-  derek::note_launch(), k_rows_r2c<<<g.row_grid(1), kGridThreads, g.rows, st>>>(t, rho, data, all);
+  derek::launch(k_rows_r2c, g.row_grid(1), kGridThreads, g.rows, st, t, rho, data, all);
 }
 template <bool ADD> void rows_c2r(const GridShape &g, const Tables &t, const double2 *data, double *out, int all, cudaStream_t st) {
   cudaFuncSetAttribute(k_rows_c2r<ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.rows);
-  derek::note_launch(), k_rows_c2r<ADD><<<g.row_grid(1), kGridThreads, g.rows, st>>>(t, data, out, all);
+  derek::launch(k_rows_c2r<ADD>, g.row_grid(1), kGridThreads, g.rows, st, t, data, out, all);
 }
 
 }  // namespace
@@ -214,12 +219,12 @@ void launch_fft3d_grid(const Tables &t, int sys_begin, int nsys, int max_n, doub
   const GridShape g(nsys, max_n);
   if (sign < 0) {
     cudaFuncSetAttribute(k_rows<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.rows);
-    derek::note_launch(), k_rows<-1><<<g.row_grid(0), kGridThreads, g.rows, st>>>(t, sys_begin, data);
+    derek::launch(k_rows<-1>, g.row_grid(0), kGridThreads, g.rows, st, t, sys_begin, data);
     cols_y<-1>(g, t, sys_begin, data, 0, 1, st);
     cols_x<-1, kPlain>(g, t, sys_begin, data, 0, 1, 0.0, 0.0, st);
   } else {
     cudaFuncSetAttribute(k_rows<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.rows);
-    derek::note_launch(), k_rows<1><<<g.row_grid(0), kGridThreads, g.rows, st>>>(t, sys_begin, data);
+    derek::launch(k_rows<1>, g.row_grid(0), kGridThreads, g.rows, st, t, sys_begin, data);
     cols_y<1>(g, t, sys_begin, data, 0, 1, st);
     cols_x<1, kPlain>(g, t, sys_begin, data, 0, 1, 0.0, 0.0, st);
   }
@@ -257,6 +262,7 @@ void launch_kerker_add(const Tables &t, int nsys, int max_n, const double *res, 
 
 __global__ void k_lda(long n, const double *__restrict__ rho, double *__restrict__ exc,
                       double *__restrict__ vxc) {
+  grid_dependency();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     double e, v;
     lda_point(rho[i], e, v);
@@ -269,7 +275,7 @@ void launch_lda(long n, const double *rho, double *exc, double *vxc, cudaStream_
   if (n <= 0) return;
   long blocks = (n + 255) / 256;
   if (blocks > 152 * 16) blocks = 152 * 16;
-  derek::note_launch(), k_lda<<<(int)blocks, 256, 0, st>>>(n, rho, exc, vxc);
+  derek::launch(k_lda, (int)blocks, 256, 0, st, n, rho, exc, vxc);
 }
 
 }  // namespace derek

@@ -44,6 +44,7 @@ template <typename R>
 __global__ void __launch_bounds__(kLineThreads, kLineBlocks) k_x_inv(Tables t, int item_begin, int cc, const cplx<R> *__restrict__ psi,
                                                         cplx<R> *__restrict__ abuf,
                                                         const double *__restrict__ occ_skip) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int item = t.item_list ? t.item_list[blockIdx.x] : item_begin + blockIdx.x;
   const int ksi = t.item_ks[item];
@@ -85,6 +86,7 @@ __global__ void __launch_bounds__(kLineThreads, kLineBlocks) k_x_inv(Tables t, i
 template <typename R>
 __global__ void __launch_bounds__(kLineThreads, kLineBlocks) k_plane(Tables t, int item_begin, cplx<R> *__restrict__ abuf,
                                                         const R *__restrict__ vloc) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int item = t.item_list ? t.item_list[blockIdx.x] : item_begin + blockIdx.x;
   const int x = blockIdx.y;
@@ -123,6 +125,7 @@ __global__ void __launch_bounds__(kLineThreads, kLineBlocks) k_x_fwd(Tables t, i
                                                         const cplx<R> *__restrict__ prev,
                                                         cplx<R> *__restrict__ out,
                                                         const Axpby *__restrict__ coef) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int item = t.item_list ? t.item_list[blockIdx.x] : item_begin + blockIdx.x;
   const int ksi = t.item_ks[item];
@@ -187,6 +190,7 @@ __global__ void __launch_bounds__(kLineThreads, kLineBlocks) k_density_plane(Tab
                                                        const cplx<R> *__restrict__ abuf,
                                                        const double *__restrict__ occ,
                                                        double *__restrict__ partial) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DensityUnit U = units[blockIdx.x];
   const int x = blockIdx.y;
@@ -263,7 +267,7 @@ void launch_x_inv(const Tables &t, int item_begin, int nitems, int max_nchunk, i
   const int ncol = max_nchunk * kColChunk, cc = x_columns(nitems, ncol);
   const size_t sm = smem_x<R>(max_n1, cc);
   cudaFuncSetAttribute(k_x_inv<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::note_launch(), k_x_inv<R><<<dim3(nitems, (ncol + cc - 1) / cc), kLineThreads, sm, st>>>(t, item_begin, cc, psi, abuf, occ_skip);
+  derek::launch(k_x_inv<R>, dim3(nitems, (ncol + cc - 1) / cc), kLineThreads, sm, st, t, item_begin, cc, psi, abuf, occ_skip);
 }
 
 template <typename R>
@@ -279,7 +283,7 @@ void launch_x_fwd(const Tables &t, int item_begin, int nitems, int max_nchunk, i
   const int ncol = max_nchunk * kColChunk, cc = x_columns(nitems, ncol);
   const size_t sm = smem_x<R>(max_n1, cc);
   cudaFuncSetAttribute(k_x_fwd<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::note_launch(), k_x_fwd<R><<<dim3(nitems, (ncol + cc - 1) / cc), kLineThreads, sm, st>>>(t, item_begin, cc, abuf, psi, prev, out, coef);
+  derek::launch(k_x_fwd<R>, dim3(nitems, (ncol + cc - 1) / cc), kLineThreads, sm, st, t, item_begin, cc, abuf, psi, prev, out, coef);
 }
 
 template <typename R>
@@ -293,7 +297,7 @@ void launch_plane(const Tables &t, int item_begin, int nitems, int max_n1, int m
   }
   const size_t sm = smem_plane<R>(max_n2, max_n3);
   cudaFuncSetAttribute(k_plane<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::note_launch(), k_plane<R><<<dim3(nitems, max_n1), kLineThreads, sm, st>>>(t, item_begin, abuf, vloc);
+  derek::launch(k_plane<R>, dim3(nitems, max_n1), kLineThreads, sm, st, t, item_begin, abuf, vloc);
 }
 
 
@@ -307,7 +311,7 @@ void launch_density_plane(const Tables &t, const DensityUnit *units, int nunits,
   }
   const size_t sm = (size_t)density_acc_count(n[1] * n[2]) * sizeof(double) + smem_plane<R>(n[1], n[2]);
   cudaFuncSetAttribute(k_density_plane<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::note_launch(), k_density_plane<R><<<dim3(nunits, n[0]), kLineThreads, sm, st>>>(t, units, abuf, occ, partial);
+  derek::launch(k_density_plane<R>, dim3(nunits, n[0]), kLineThreads, sm, st, t, units, abuf, occ, partial);
 }
 
 #define DEREK_INST(R)                                                                             \

@@ -17,6 +17,7 @@ __global__ void __launch_bounds__(NT, 1) k_density_rows(Tables t, const DensityU
                                                         const float2 *__restrict__ abuf,
                                                         const double *__restrict__ occ,
                                                         double *__restrict__ partial) {
+  grid_dependency();
   using Lay = RowsLayout<N, RY>;
   constexpr int PZ = Lay::PZ, PP = Lay::PP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -105,7 +106,7 @@ static void density_rows_go(const Tables &t, const DensityUnit *units, int nunit
   auto kern = k_density_rows<N, RY, Sh::XP, Sh::NT>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM);
   const int ng = (n1 + Sh::XP - 1) / Sh::XP;
-  derek::note_launch(), kern<<<dim3(nunits, ng), Sh::NT, Sh::SMEM, st>>>(t, units, abuf, occ, partial);
+  derek::launch(kern, dim3(nunits, ng), Sh::NT, Sh::SMEM, st, t, units, abuf, occ, partial);
 }
 
 template <int N>

@@ -48,6 +48,7 @@ template <int N, int RX>
 __global__ void __launch_bounds__(kXThreads, 3) k_xinv_reg(Tables t, int item_begin, const float2 *__restrict__ psi,
                                                            float2 *__restrict__ abuf,
                                                            const double *__restrict__ occ_skip) {
+  grid_dependency();
   const int item = t.item_list ? t.item_list[blockIdx.x] : item_begin + blockIdx.x;
   const int ksi = t.item_ks[item];
   const KSetDev &K = t.ks[ksi];
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(kXThreads, 3) k_xfwd_reg(Tables t, int item_be
                                                            const float2 *__restrict__ prev,
                                                            float2 *__restrict__ out,
                                                            const Axpby *__restrict__ coef) {
+  grid_dependency();
   extern __shared__ __align__(16) float2 run_vals[];   // kXThreads * (2 RX + 1)
   const int item = t.item_list ? t.item_list[blockIdx.x] : item_begin + blockIdx.x;
   const int ksi = t.item_ks[item];
@@ -170,7 +172,7 @@ template <int N, int RX>
 static void xinv_go(const Tables &t, int item_begin, int nitems, int max_ncol, const float2 *psi,
                     float2 *abuf, const double *occ_skip, cudaStream_t st) {
   const int nchunk = (max_ncol + kXThreads - 1) / kXThreads;
-  derek::note_launch(), k_xinv_reg<N, RX><<<dim3(nitems, nchunk), kXThreads, 0, st>>>(t, item_begin, psi, abuf, occ_skip);
+  derek::launch(k_xinv_reg<N, RX>, dim3(nitems, nchunk), kXThreads, 0, st, t, item_begin, psi, abuf, occ_skip);
 }
 
 template <int N, int RX>
@@ -181,7 +183,7 @@ static void xfwd_go(const Tables &t, int item_begin, int nitems, int max_ncol, c
   const int smem = kXThreads * (2 * RX + 1) * (int)sizeof(float2);
   auto kern = k_xfwd_reg<N, RX>;
   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  derek::note_launch(), kern<<<dim3(nitems, nchunk), kXThreads, smem, st>>>(t, item_begin, abuf, psi, prev, out, coef);
+  derek::launch(kern, dim3(nitems, nchunk), kXThreads, smem, st, t, item_begin, abuf, psi, prev, out, coef);
 }
 
 template <int N>

@@ -5,16 +5,6 @@
 
 namespace derek {
 
-inline int sm_count() {
-  static int n = [] {
-    int dev = 0, c = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-    return c > 0 ? c : 1;
-  }();
-  return n;
-}
-
 // Read-only tables describing a batch (one copy in device memory).
 struct Tables {
   const SysDev *sys;

@@ -66,6 +66,7 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long x) {
 template <typename R>
 __global__ void k_init_psi(const Tables t, cplx<R> *__restrict__ X, unsigned long long seed,
                            const int *__restrict__ pw_entry) {
+  grid_dependency();
   const int item = blockIdx.x;
   const int ksi = t.item_ks[item];
   const KSetDev &K = t.ks[ksi];
@@ -90,6 +91,7 @@ __global__ void k_init_psi(const Tables t, cplx<R> *__restrict__ X, unsigned lon
 // Chelikowsky, J. Comput. Phys. 219 (2006) 172): damp [a, b], scale at a0.
 __global__ void k_filter_coef(const Tables t, int nks, const double *__restrict__ eig,
                               const SysState *__restrict__ st, Axpby *__restrict__ coef, int m) {
+  grid_dependency();
   const int ksi = blockIdx.x * blockDim.x + threadIdx.x;
   if (ksi >= nks) return;
   const KSetDev &K = t.ks[ksi];
@@ -121,6 +123,7 @@ __global__ void __launch_bounds__(1024) k_occupations(const Tables t, const doub
                                                       double *__restrict__ occ,
                                                       double *__restrict__ occw,
                                                       SysState *__restrict__ st) {
+  grid_dependency();
   __shared__ double red[32];
   const int s = blockIdx.x;
   const SysDev &S = t.sys[s];
@@ -248,6 +251,7 @@ __global__ void __launch_bounds__(256) k_energy_partials(const Tables t, const d
                                                          const double *__restrict__ rho_out,
                                                          const double2 *__restrict__ cgrid,
                                                          double *__restrict__ part, const SpinGrids sg) {
+  grid_dependency();
   __shared__ double red[8];
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
@@ -316,6 +320,7 @@ __global__ void __launch_bounds__(256) k_energy_partials(const Tables t, const d
 __global__ void __launch_bounds__(32) k_energy_final(const Tables t, int nsys, const double *__restrict__ part,
                                SysState *__restrict__ st, SysDev *__restrict__ sys_rw,
                                const int *__restrict__ ks_status) {
+  grid_dependency();
   const int s = blockIdx.x;
   const SysDev &S = t.sys[s];
   if (!S.active) return;
@@ -366,6 +371,7 @@ __global__ void __launch_bounds__(256) k_mix_store(const Tables t, const double 
                                                    double *__restrict__ res_hist,
                                                    const long long *__restrict__ hist_off,
                                                    const SysState *__restrict__ st, int H) {
+  grid_dependency();
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
   if (!S.active) return;
@@ -384,6 +390,7 @@ __global__ void __launch_bounds__(256) k_mix_gram_partials(const Tables t, const
                                                            const long long *__restrict__ hist_off,
                                                            const SysState *__restrict__ st, int H,
                                                            double *__restrict__ part) {
+  grid_dependency();
   __shared__ double red[8];
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
@@ -408,6 +415,7 @@ __global__ void __launch_bounds__(256) k_mix_gram_partials(const Tables t, const
 // 47 -> 22 us at 8 pairs).
 __global__ void __launch_bounds__(32) k_mix_solve(const Tables t, int nsys, const double *__restrict__ part,
                                                   SysState *__restrict__ st, int H) {
+  grid_dependency();
   __shared__ double A[kMaxHist + 1][kMaxHist + 2];   // the last column is the right-hand side
   __shared__ double gram[kMaxHist][kMaxHist];
   const int s = blockIdx.x, lane = threadIdx.x;
@@ -486,6 +494,7 @@ __global__ void __launch_bounds__(256) k_mix_combine(const Tables t, double *__r
                                                      const SysState *__restrict__ st,
                                                      double *__restrict__ rwork, double alpha,
                                                      int kerker) {
+  grid_dependency();
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
   if (!S.active) return;
@@ -518,6 +527,7 @@ __global__ void __launch_bounds__(256) k_mix_combine(const Tables t, double *__r
 __global__ void __launch_bounds__(256) k_mix_store_m(const Tables t, const SpinGrids sg,
                                                      const long long *__restrict__ hist_off,
                                                      const SysState *__restrict__ st, int H) {
+  grid_dependency();
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
   if (!S.active) return;
@@ -538,6 +548,7 @@ __global__ void __launch_bounds__(256) k_mix_gram_m(const Tables t, const SpinGr
                                                     const long long *__restrict__ hist_off,
                                                     const SysState *__restrict__ st, int H,
                                                     double *__restrict__ part) {
+  grid_dependency();
   __shared__ double red[8];
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
@@ -560,6 +571,7 @@ __global__ void __launch_bounds__(256) k_mix_gram_m(const Tables t, const SpinGr
 __global__ void __launch_bounds__(256) k_mix_combine_m(const Tables t, const SpinGrids sg,
                                                        const long long *__restrict__ hist_off,
                                                        const SysState *__restrict__ st, double alpha) {
+  grid_dependency();
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
   if (!S.active) return;
@@ -589,6 +601,7 @@ __global__ void __launch_bounds__(256) k_build_vloc(const Tables t, const double
                                                     double *__restrict__ vloc,
                                                     float *__restrict__ vloc32,
                                                     double *__restrict__ part, int all, const SpinGrids sg) {
+  grid_dependency();
   __shared__ double red[8];
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
@@ -646,6 +659,7 @@ __global__ void __launch_bounds__(256) k_build_vloc(const Tables t, const double
 
 __global__ void __launch_bounds__(32) k_vmax_final(const Tables t, int nsys, const double *__restrict__ part,
                              SysState *__restrict__ st, int all) {
+  grid_dependency();
   const int s = blockIdx.x;
   if (!all && !t.sys[s].active) return;
   double vm = -1e300;
@@ -655,6 +669,7 @@ __global__ void __launch_bounds__(32) k_vmax_final(const Tables t, int nsys, con
 }
 
 __global__ void __launch_bounds__(256) k_uniform_density(const Tables t, double *__restrict__ rho) {
+  grid_dependency();
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
   const double v = S.nelec / S.volume;
@@ -667,27 +682,27 @@ __global__ void __launch_bounds__(256) k_uniform_density(const Tables t, double 
 template <typename R>
 void launch_init_psi(const Tables &t, int nitems, void *X, unsigned long long seed, const int *pw_entry,
                      cudaStream_t st) {
-  derek::note_launch(), k_init_psi<R><<<nitems, 256, 0, st>>>(t, (cplx<R> *)X, seed, pw_entry);
+  derek::launch(k_init_psi<R>, nitems, 256, 0, st, t, (cplx<R> *)X, seed, pw_entry);
 }
 template void launch_init_psi<float>(const Tables &, int, void *, unsigned long long, const int *, cudaStream_t);
 template void launch_init_psi<double>(const Tables &, int, void *, unsigned long long, const int *, cudaStream_t);
 
 void launch_filter_coef(const Tables &t, int nks, const double *eig, const SysState *st, Axpby *coef,
                         int m, cudaStream_t s) {
-  derek::note_launch(), k_filter_coef<<<(nks + 127) / 128, 128, 0, s>>>(t, nks, eig, st, coef, m);
+  derek::launch(k_filter_coef, (nks + 127) / 128, 128, 0, s, t, nks, eig, st, coef, m);
 }
 
 void launch_occupations(const Tables &t, int nsys, int max_states, const double *eig, double *occ, double *occw,
                         SysState *st, cudaStream_t s) {
   const int threads = std::min(1024, std::max(32, (max_states + 31) / 32 * 32));
-  derek::note_launch(), k_occupations<<<nsys, threads, 0, s>>>(t, eig, occ, occw, st);
+  derek::launch(k_occupations, nsys, threads, 0, s, t, eig, occ, occw, st);
 }
 
 void launch_energies(const Tables &t, int nsys, const double *vhxc, const double *rho_in,
                      const double *rho_out, const double2 *cgrid, double *part, SysState *st,
                      SysDev *sys_rw, const int *ks_status, const SpinGrids &sg, cudaStream_t s) {
-  derek::note_launch(), k_energy_partials<<<dim3(RB, nsys), 256, 0, s>>>(t, vhxc, rho_in, rho_out, cgrid, part, sg);
-  derek::note_launch(), k_energy_final<<<nsys, 32, 0, s>>>(t, nsys, part, st, sys_rw, ks_status);
+  derek::launch(k_energy_partials, dim3(RB, nsys), 256, 0, s, t, vhxc, rho_in, rho_out, cgrid, part, sg);
+  derek::launch(k_energy_final, nsys, 32, 0, s, t, nsys, part, st, sys_rw, ks_status);
 }
 
 void launch_mix(const Tables &t, int nsys, int max_nr, double *rho_in, const double *rho_out,
@@ -695,15 +710,15 @@ void launch_mix(const Tables &t, int nsys, int max_nr, double *rho_in, const dou
                 double *part, double2 *cgrid, double *rwork, double alpha, double q0, int max_n, const SpinGrids &sg,
                 cudaStream_t s) {
   const int gx = (int)std::min<long long>(((long long)max_nr + 255) / 256, 256);
-  derek::note_launch(), k_mix_store<<<dim3(gx, nsys), 256, 0, s>>>(t, rho_in, rho_out, nin_hist, res_hist, hist_off, st, H);
-  if (sg.on) derek::note_launch(), k_mix_store_m<<<dim3(gx, nsys), 256, 0, s>>>(t, sg, hist_off, st, H);
-  derek::note_launch(), k_mix_gram_partials<<<dim3(RB, nsys), 256, 0, s>>>(t, res_hist, hist_off, st, H, part);
-  if (sg.on) derek::note_launch(), k_mix_gram_m<<<dim3(RB, nsys), 256, 0, s>>>(t, sg, hist_off, st, H, part);
-  derek::note_launch(), k_mix_solve<<<nsys, 32, 0, s>>>(t, nsys, part, st, H);
+  derek::launch(k_mix_store, dim3(gx, nsys), 256, 0, s, t, rho_in, rho_out, nin_hist, res_hist, hist_off, st, H);
+  if (sg.on) derek::launch(k_mix_store_m, dim3(gx, nsys), 256, 0, s, t, sg, hist_off, st, H);
+  derek::launch(k_mix_gram_partials, dim3(RB, nsys), 256, 0, s, t, res_hist, hist_off, st, H, part);
+  if (sg.on) derek::launch(k_mix_gram_m, dim3(RB, nsys), 256, 0, s, t, sg, hist_off, st, H, part);
+  derek::launch(k_mix_solve, nsys, 32, 0, s, t, nsys, part, st, H);
   const int kerker = q0 > 0;
-  derek::note_launch(), k_mix_combine<<<dim3(gx, nsys), 256, 0, s>>>(t, rho_in, nin_hist, res_hist, hist_off, st, rwork,
+  derek::launch(k_mix_combine, dim3(gx, nsys), 256, 0, s, t, rho_in, nin_hist, res_hist, hist_off, st, rwork,
                                                alpha, kerker);
-  if (sg.on) derek::note_launch(), k_mix_combine_m<<<dim3(gx, nsys), 256, 0, s>>>(t, sg, hist_off, st, alpha);
+  if (sg.on) derek::launch(k_mix_combine_m, dim3(gx, nsys), 256, 0, s, t, sg, hist_off, st, alpha);
   if (kerker) launch_kerker_add(t, nsys, max_n, rwork, cgrid, alpha, q0, rho_in, s);
 }
 
@@ -711,12 +726,13 @@ void launch_potential(const Tables &t, int nsys, int max_n, const double *rho_in
                       double2 *cgrid, double *rwork, const double *vext, double *vhxc, double *vloc, float *vloc32,
                       double *part, SysState *st, int all, const SpinGrids &sg, cudaStream_t s) {
   launch_hartree(t, nsys, max_n, rho_in, cgrid, rwork, all, s);
-  derek::note_launch(), k_build_vloc<<<dim3(RB, nsys), 256, 0, s>>>(t, rho_in, rwork, vext, vhxc, vloc, vloc32, part, all, sg);
-  derek::note_launch(), k_vmax_final<<<nsys, 32, 0, s>>>(t, nsys, part, st, all);
+  derek::launch(k_build_vloc, dim3(RB, nsys), 256, 0, s, t, rho_in, rwork, vext, vhxc, vloc, vloc32, part, all, sg);
+  derek::launch(k_vmax_final, nsys, 32, 0, s, t, nsys, part, st, all);
 }
 
 __global__ void k_lsda(long n, const double *__restrict__ ra, const double *__restrict__ rb,
                        double *__restrict__ exc, double *__restrict__ va, double *__restrict__ vb) {
+  grid_dependency();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     double e, a, b;
     lsda_point(ra[i], rb[i], e, a, b);
@@ -729,12 +745,12 @@ __global__ void k_lsda(long n, const double *__restrict__ ra, const double *__re
 void launch_lsda(long n, const double *rho_a, const double *rho_b, double *exc, double *va, double *vb,
                  cudaStream_t s) {
   const int blocks = (int)std::min<long>((n + 255) / 256, 152 * 8);
-  derek::note_launch(), k_lsda<<<blocks, 256, 0, s>>>(n, rho_a, rho_b, exc, va, vb);
+  derek::launch(k_lsda, blocks, 256, 0, s, n, rho_a, rho_b, exc, va, vb);
 }
 
 void launch_uniform_density(const Tables &t, int nsys, int max_nr, double *rho, cudaStream_t s) {
   const int gx = (int)std::min<long long>(((long long)max_nr + 255) / 256, 256);
-  derek::note_launch(), k_uniform_density<<<dim3(gx, nsys), 256, 0, s>>>(t, rho);
+  derek::launch(k_uniform_density, dim3(gx, nsys), 256, 0, s, t, rho);
 }
 
 }  // namespace derek
@@ -754,6 +770,7 @@ __global__ void __launch_bounds__(256) k_hf_partials(const Tables t, const doubl
                                                      const int *__restrict__ well_off,
                                                      const double *__restrict__ cells,
                                                      double *__restrict__ part, int max_wells) {
+  grid_dependency();
   __shared__ double red[8];
   const int s = blockIdx.y;
   const SysDev &S = t.sys[s];
@@ -800,6 +817,7 @@ __global__ void __launch_bounds__(256) k_hf_partials(const Tables t, const doubl
 __global__ void k_hf_final(const Tables t, int nsys, const double *__restrict__ part,
                            const int *__restrict__ well_off, double *__restrict__ grad,
                            int max_wells) {
+  grid_dependency();
   const int s = blockIdx.x;
   if (s >= nsys) return;
   const SysDev &S = t.sys[s];
@@ -816,8 +834,8 @@ void launch_hf_gradient(const Tables &t, int nsys, const double *rho, const doub
                         const int *well_off, const double *cells, double *part, int max_wells,
                         double *grad, cudaStream_t s) {
   if (max_wells <= 0) return;
-  derek::note_launch(), k_hf_partials<<<dim3(RB, nsys), 256, 0, s>>>(t, rho, wells, well_off, cells, part, max_wells);
-  derek::note_launch(), k_hf_final<<<nsys, 128, 0, s>>>(t, nsys, part, well_off, grad, max_wells);
+  derek::launch(k_hf_partials, dim3(RB, nsys), 256, 0, s, t, rho, wells, well_off, cells, part, max_wells);
+  derek::launch(k_hf_final, nsys, 128, 0, s, t, nsys, part, well_off, grad, max_wells);
 }
 
 }  // namespace derek
@@ -826,6 +844,7 @@ namespace derek {
 
 // dv_xc/dn at rho (central difference, relative step 1e-4; zero below 1e-10)
 __global__ void k_fxc(long long n, const double *__restrict__ rho, double *__restrict__ fxc) {
+  grid_dependency();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     const double r = rho[i];
@@ -843,7 +862,7 @@ __global__ void k_fxc(long long n, const double *__restrict__ rho, double *__res
 
 void launch_fxc(long long n, const double *rho, double *fxc, cudaStream_t s) {
   const int blocks = (int)std::min<long long>((n + 255) / 256, 152 * 8);
-  derek::note_launch(), k_fxc<<<blocks, 256, 0, s>>>(n, rho, fxc);
+  derek::launch(k_fxc, blocks, 256, 0, s, n, rho, fxc);
 }
 
 }  // namespace derek

@@ -68,6 +68,7 @@ __device__ __forceinline__ void spinor_planes_backward(const Tables &t, const KS
 template <typename R>
 __global__ void __launch_bounds__(512) k_plane_spinor(Tables t, int item_begin, cplx<R> *__restrict__ abuf,
                                                       const cplx<R> *__restrict__ vnc) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int slot = 2 * blockIdx.x;
   const int item = t.item_list ? t.item_list[slot] : item_begin + slot;
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(512) k_density_spinor(Tables t, const DensityU
                                                         const cplx<R> *__restrict__ abuf,
                                                         const double *__restrict__ occ,
                                                         double *__restrict__ partial) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DensityUnit U = units[blockIdx.x];
   const int x = blockIdx.y;
@@ -179,7 +181,7 @@ void launch_plane_spinor(const Tables &t, int item_begin, int nitems, const int 
   }
   const size_t sm = spinor_plane_smem(n[1], n[2], sizeof(cplx<R>));
   cudaFuncSetAttribute(k_plane_spinor<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::note_launch(), k_plane_spinor<R><<<dim3(nitems / 2, n[0]), 512, sm, st>>>(t, item_begin, abuf, vnc);
+  derek::launch(k_plane_spinor<R>, dim3(nitems / 2, n[0]), 512, sm, st, t, item_begin, abuf, vnc);
 }
 
 template <typename R>
@@ -188,7 +190,7 @@ void launch_density_spinor(const Tables &t, const DensityUnit *units, int nunits
   if (nunits <= 0) return;
   const size_t sm = spinor_plane_smem(n[1], n[2], sizeof(cplx<R>));
   cudaFuncSetAttribute(k_density_spinor<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::note_launch(), k_density_spinor<R><<<dim3(nunits, n[0]), 512, sm, st>>>(t, units, abuf, occ, partial);
+  derek::launch(k_density_spinor<R>, dim3(nunits, n[0]), 512, sm, st, t, units, abuf, occ, partial);
 }
 
 #define DEREK_INST(R)                                                                                  \

@@ -24,6 +24,7 @@ namespace {
 template <int N, int RY, int XP, int NT, int BLOCKS>
 __global__ void __launch_bounds__(NT, BLOCKS) k_plane_spinor_reg(Tables t, int item_begin, float2 *__restrict__ abuf,
                                                          const float4 *__restrict__ vnc) {
+  grid_dependency();
   using Lay = RowsLayout<N, RY>;
   constexpr int PZ = Lay::PZ, PP1 = Lay::PP, PP0 = PlaneLayout<N>::PP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -151,8 +152,7 @@ void spinor_go(const Tables &t, int item_begin, int nitems, int n1, float2 *abuf
   constexpr int NT = (N * XP + 31) / 32 * 32;
   auto kern = k_plane_spinor_reg<N, RY, XP, NT, HALF >= 2 ? 2 : 1>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XP * PLANE);
-  derek::note_launch(), kern<<<dim3(nitems / 2, (n1 + XP - 1) / XP), NT, XP * PLANE, st>>>(
-      t, item_begin, abuf, reinterpret_cast<const float4 *>(vnc));
+  derek::launch(kern, dim3(nitems / 2, (n1 + XP - 1) / XP), NT, XP * PLANE, st, t, item_begin, abuf, reinterpret_cast<const float4 *>(vnc));
 }
 
 template <int N>

@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(256) k_overlap_pairs(const Tables t, int ks_be
                                                        double2 *__restrict__ part,
                                                        const long long *__restrict__ part_off,
                                                        int ksplit) {
+  grid_dependency();
   constexpr int MT = OverlapShape<R>::MT, OKC = OverlapShape<R>::OKC, LD = OKC + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ksi = ks_begin + blockIdx.z;
@@ -175,6 +176,7 @@ __global__ void __launch_bounds__(256) k_overlap_reduce(const Tables t, int ks_b
                                                         double2 *__restrict__ out,
                                                         const long long *__restrict__ mat_off, int hermitize,
                                                         int half) {
+  grid_dependency();
   const int ksi = ks_begin + blockIdx.x;
   const KSetDev &K = t.ks[ksi];
   if (!t.sys[K.sys].active) return;
@@ -243,6 +245,7 @@ template <int JQ>
 __global__ void __launch_bounds__(256, 2) k_rotate64(const Tables t, int ks_begin, double2 *__restrict__ X,
                                                      const double2 *__restrict__ C,
                                                      const long long *__restrict__ mat_off, int upper) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ksi = ks_begin + blockIdx.y;
   const KSetDev &K = t.ks[ksi];
@@ -292,6 +295,7 @@ template <int JQ>
 __global__ void __launch_bounds__(256, 2) k_rotate32(const Tables t, int ks_begin, float2 *__restrict__ X,
                                                      const double2 *__restrict__ C,
                                                      const long long *__restrict__ mat_off, int upper) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ksi = ks_begin + blockIdx.y;
   const KSetDev &K = t.ks[ksi];
@@ -386,6 +390,7 @@ __global__ void __launch_bounds__(256) k_cholesky_inv(const Tables t, int ks_beg
                                                       const long long *__restrict__ mat_off,
                                                       double2 *__restrict__ scratch,
                                                       int *__restrict__ status, int use_smem) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ksi = ks_begin + blockIdx.x;
   const KSetDev &K = t.ks[ksi];
@@ -514,6 +519,7 @@ __global__ void __launch_bounds__(256) k_jacobi(const Tables t, int ks_begin, co
                                                 double2 *__restrict__ Cout, const long long *__restrict__ mat_off,
                                                 double *__restrict__ eig, int max_sweeps, double tol,
                                                 int *__restrict__ sweeps_out) {
+  grid_dependency();
   namespace cg = cooperative_groups;
   constexpr int NT = 256;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -858,6 +864,7 @@ __global__ void __launch_bounds__(256) k_jacobi_global(const Tables t, int ks_be
                                                 double *__restrict__ eig,
                                                 double2 *__restrict__ scratch, int max_sweeps,
                                                 double tol, int *__restrict__ sweeps_out) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ksi = ks_begin + blockIdx.x;
   const KSetDev &K = t.ks[ksi];
@@ -1059,7 +1066,7 @@ static void overlap_go(const Tables &t, int ks_begin, int nks, int max_nb, int m
   const dim3 grid(groups, (max_npw + ksplit - 1) / ksplit, nks);
   auto go = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    derek::note_launch(), kern<<<grid, threads, sm, st>>>(t, ks_begin, A, B, part, part_off, ksplit);
+    derek::launch(kern, grid, threads, sm, st, t, ks_begin, A, B, part, part_off, ksplit);
   };
   switch (P) {
     case 1: go(k_overlap_pairs<R, 1, SAME>); break;
@@ -1087,7 +1094,7 @@ void launch_overlap_reduce(const Tables &t, int ks_begin, int nks, int max_nb, c
                            const long long *part_off, int ksplit, double2 *out,
                            const long long *mat_off, int hermitize, int half, cudaStream_t st) {
   const dim3 grid(nks, (max_nb * max_nb * kReduceLanes + 255) / 256);
-  derek::note_launch(), k_overlap_reduce<<<grid, 256, 0, st>>>(t, ks_begin, part, part_off, ksplit, out, mat_off, hermitize, half);
+  derek::launch(k_overlap_reduce, grid, 256, 0, st, t, ks_begin, part, part_off, ksplit, out, mat_off, hermitize, half);
 }
 
 template <typename R>
@@ -1104,7 +1111,7 @@ void launch_rotate(const Tables &t, int ks_begin, int nks, int max_nb, int max_n
   const int gx = F64 ? tiles : std::min(tiles, std::max(1, (4 * sm_count() + nks - 1) / nks));
   auto go = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    derek::note_launch(), kern<<<dim3(gx, nks), 256, sm, st>>>(t, ks_begin, X, C, mat_off, upper);
+    derek::launch(kern, dim3(gx, nks), 256, sm, st, t, ks_begin, X, C, mat_off, upper);
   };
   if constexpr (F64) {
     switch ((max_nb + RWARPS - 1) / RWARPS) {
@@ -1137,7 +1144,7 @@ void launch_cholesky_inv(const Tables &t, int ks_begin, int nks, int max_nb, con
   const int use_smem = cholesky_fits_smem(max_nb);
   const size_t sm = use_smem ? (size_t)max_nb * (max_nb | 1) * sizeof(double2) : 0;
   cudaFuncSetAttribute(k_cholesky_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::note_launch(), k_cholesky_inv<<<nks, 256, sm, st>>>(t, ks_begin, S, C, mat_off, scratch, status, use_smem);
+  derek::launch_plain(k_cholesky_inv, nks, 256, sm, st, t, ks_begin, S, C, mat_off, scratch, status, use_smem);
 }
 
 // tables of the Jacobi kernels: two rounds' rotations and the block list
@@ -1184,7 +1191,7 @@ void launch_jacobi(const Tables &t, int ks_begin, int nks, int max_nb, const dou
   const size_t sm = jacobi_smem(max_nb, cs);
   if (sm > kJacobiSmem) {
     const size_t tab = jacobi_tables(max_nb);
-    derek::note_launch(), k_jacobi_global<<<nks, 256, tab, st>>>(t, ks_begin, Hs, C, mat_off, eig, scratch, max_sweeps,
+    derek::launch(k_jacobi_global, nks, 256, tab, st, t, ks_begin, Hs, C, mat_off, eig, scratch, max_sweeps,
                                                                  tol, sweeps_out);
     return;
   }

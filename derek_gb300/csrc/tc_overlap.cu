@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     k_overlap_tc(const Tables t, int ks_begin, const float2 *__restrict__ X, const float2 *__restrict__ Y,
                  double2 *__restrict__ part, const long long *__restrict__ part_off, int ksplit,
                  int *__restrict__ status) {
+  grid_dependency();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bars[3];
   __shared__ uint32_t tmem_slot;
@@ -360,7 +361,7 @@ void launch_overlap_tc(const Tables &t, int ks_begin, int nks, int max_nb, int m
   const size_t sm = overlap_tc_smem(max_nb);
   cudaFuncSetAttribute(k_overlap_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   dim3 grid((max_npw + ksplit - 1) / ksplit, nks);
-  derek::note_launch(), k_overlap_tc<<<grid, TC_THREADS, sm, st>>>(t, ks_begin, X, Y, part, part_off, ksplit, status);
+  derek::launch(k_overlap_tc, grid, TC_THREADS, sm, st, t, ks_begin, X, Y, part, part_off, ksplit, status);
   launch_overlap_reduce(t, ks_begin, nks, max_nb, part, part_off, ksplit, out, mat_off, hermitize, 0, st);
 }
 
@@ -398,6 +399,7 @@ size_t rotate_tc_image_bytes(int max_nb) {
 __global__ void __launch_bounds__(256) k_rotate_operand(const Tables t, int ks_begin, const double2 *__restrict__ C,
                                                         const long long *__restrict__ mat_off,
                                                         unsigned char *__restrict__ img, long long stride) {
+  grid_dependency();
   const int ksi = ks_begin + blockIdx.y;
   const KSetDev &K = t.ks[ksi];
   if (!t.sys[K.sys].active) return;
@@ -436,6 +438,7 @@ __global__ void __launch_bounds__(256) k_rotate_operand(const Tables t, int ks_b
 __global__ void __launch_bounds__(TC_THREADS, 1)
     k_rotate_tc(const Tables t, int ks_begin, float2 *__restrict__ X, const unsigned char *__restrict__ img,
                 long long img_stride, int *__restrict__ status) {
+  grid_dependency();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bars[3];
   __shared__ uint32_t tmem_slot;
@@ -577,11 +580,11 @@ void launch_rotate_tc(const Tables &t, int ks_begin, int nks, int max_nb, int ma
                       cudaStream_t st) {
   if (nks <= 0) return;
   const long long stride = (long long)rotate_tc_image_bytes(max_nb);
-  derek::note_launch(), k_rotate_operand<<<dim3(4, nks), 256, 0, st>>>(t, ks_begin, C, mat_off, img, stride);
+  derek::launch(k_rotate_operand, dim3(4, nks), 256, 0, st, t, ks_begin, C, mat_off, img, stride);
   const size_t sm = overlap_tc_smem(max_nb);
   cudaFuncSetAttribute(k_rotate_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   dim3 grid((max_npw + TC_M - 1) / TC_M, nks);
-  derek::note_launch(), k_rotate_tc<<<grid, TC_THREADS, sm, st>>>(t, ks_begin, X, img, stride, status);
+  derek::launch(k_rotate_tc, grid, TC_THREADS, sm, st, t, ks_begin, X, img, stride, status);
 }
 
 }  // namespace derek

@@ -21,6 +21,7 @@ __device__ __forceinline__ int device_row(int r, int nrows, int nsp) {
 template <typename R>
 __global__ void __launch_bounds__(256) k_wfn_in(const double2 *__restrict__ src, const int *__restrict__ perm, int npw,
                                                 int npw_pad, int row0, int nrows, int nsp, cplx<R> *__restrict__ dst) {
+  grid_dependency();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= npw_pad) return;
   cplx<R> v = mk<R>(0, 0);
@@ -35,6 +36,7 @@ template <typename R>
 __global__ void __launch_bounds__(256) k_wfn_out(const cplx<R> *__restrict__ src, const int *__restrict__ perm,
                                                  int npw, int npw_pad, int row0, int nrows, int nsp,
                                                  double2 *__restrict__ dst) {
+  grid_dependency();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= npw) return;
   const cplx<R> s = src[(long long)device_row(row0 + blockIdx.y, nrows, nsp) * npw_pad + g];
@@ -44,21 +46,19 @@ __global__ void __launch_bounds__(256) k_wfn_out(const cplx<R> *__restrict__ src
 void launch_wfn_in(int fp64, const double2 *src, const int *perm, const KSetDev &K, int nsp, int row0, int count,
                    void *dst, cudaStream_t st) {
   const dim3 grid((K.npw_pad + 255) / 256, count);
-  derek::note_launch();
   if (fp64)
-    k_wfn_in<double><<<grid, 256, 0, st>>>(src, perm, K.npw, K.npw_pad, row0, K.nbr, nsp, (double2 *)dst);
+    derek::launch(k_wfn_in<double>, grid, 256, 0, st, src, perm, K.npw, K.npw_pad, row0, K.nbr, nsp, (double2 *)dst);
   else
-    k_wfn_in<float><<<grid, 256, 0, st>>>(src, perm, K.npw, K.npw_pad, row0, K.nbr, nsp, (float2 *)dst);
+    derek::launch(k_wfn_in<float>, grid, 256, 0, st, src, perm, K.npw, K.npw_pad, row0, K.nbr, nsp, (float2 *)dst);
 }
 
 void launch_wfn_out(int fp64, const void *src, const int *perm, const KSetDev &K, int nsp, int row0, int count,
                     double2 *dst, cudaStream_t st) {
   const dim3 grid((K.npw + 255) / 256, count);
-  derek::note_launch();
   if (fp64)
-    k_wfn_out<double><<<grid, 256, 0, st>>>((const double2 *)src, perm, K.npw, K.npw_pad, row0, K.nbr, nsp, dst);
+    derek::launch(k_wfn_out<double>, grid, 256, 0, st, (const double2 *)src, perm, K.npw, K.npw_pad, row0, K.nbr, nsp, dst);
   else
-    k_wfn_out<float><<<grid, 256, 0, st>>>((const float2 *)src, perm, K.npw, K.npw_pad, row0, K.nbr, nsp, dst);
+    derek::launch(k_wfn_out<float>, grid, 256, 0, st, (const float2 *)src, perm, K.npw, K.npw_pad, row0, K.nbr, nsp, dst);
 }
 
 }  // namespace derek
