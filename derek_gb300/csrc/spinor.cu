@@ -28,6 +28,13 @@
 
 namespace derek {
 
+// Three blocks of 192 threads per SM as in the scalar line passes (hpsi4.cu), so
+// that one's transforms run beside another's products; one of 512 where two do
+// not fit the shared memory.  SCF, 3 x 192 against 512 threads: FP32 35^3 11.6 /
+// 17.9 ms, FP64 32^3 34.7 / 44.9 ms, 44^3 119 / 132 ms, 64^3 327 / 280 ms.
+constexpr int kSpinorThreads = 192;
+inline bool spinor_small(size_t smem) { return 2 * smem <= 226 * 1024; }
+
 size_t spinor_plane_smem(int n2, int n3, size_t elem) {
   return (2 * (size_t)n2 * (n3 | 1) + (size_t)n2 + n3) * elem;
 }
@@ -65,8 +72,8 @@ __device__ __forceinline__ void spinor_planes_backward(const Tables &t, const KS
 // (y,z)-plane pass of one band (items 2q, 2q + 1 of the launch) at x-plane
 // blockIdx.y: backward yz of both components, the 2x2 product, forward yz,
 // columns written back in place.
-template <typename R>
-__global__ void __launch_bounds__(512) k_plane_spinor(Tables t, int item_begin, cplx<R> *__restrict__ abuf,
+template <typename R, int NT>
+__global__ void __launch_bounds__(NT, NT == kSpinorThreads ? 3 : 1) k_plane_spinor(Tables t, int item_begin, cplx<R> *__restrict__ abuf,
                                                       const cplx<R> *__restrict__ vnc) {
   grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -122,8 +129,8 @@ __global__ void __launch_bounds__(512) k_plane_spinor(Tables t, int item_begin, 
 // with per-item weights occ (equal on both items of a band), written as four
 // planes of nr values at the unit's partial grids.  Each thread owns the
 // same grid points in every band, so the sums need no synchronisation.
-template <typename R>
-__global__ void __launch_bounds__(512) k_density_spinor(Tables t, const DensityUnit *__restrict__ units,
+template <typename R, int NT>
+__global__ void __launch_bounds__(NT, NT == kSpinorThreads ? 3 : 1) k_density_spinor(Tables t, const DensityUnit *__restrict__ units,
                                                         const cplx<R> *__restrict__ abuf,
                                                         const double *__restrict__ occ,
                                                         double *__restrict__ partial) {
@@ -180,8 +187,14 @@ void launch_plane_spinor(const Tables &t, int item_begin, int nitems, const int 
     if (launch_plane_spinor_reg(t, item_begin, nitems, n, max_m, abuf, vnc, st)) return;
   }
   const size_t sm = spinor_plane_smem(n[1], n[2], sizeof(cplx<R>));
-  cudaFuncSetAttribute(k_plane_spinor<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::launch(k_plane_spinor<R>, dim3(nitems / 2, n[0]), 512, sm, st, t, item_begin, abuf, vnc);
+  auto go = [&](auto kern, int threads) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    derek::launch(kern, dim3(nitems / 2, n[0]), threads, sm, st, t, item_begin, abuf, vnc);
+  };
+  if (spinor_small(sm))
+    go(k_plane_spinor<R, kSpinorThreads>, kSpinorThreads);
+  else
+    go(k_plane_spinor<R, 512>, 512);
 }
 
 template <typename R>
@@ -189,8 +202,14 @@ void launch_density_spinor(const Tables &t, const DensityUnit *units, int nunits
                            const cplx<R> *abuf, const double *occ, double *partial, cudaStream_t st) {
   if (nunits <= 0) return;
   const size_t sm = spinor_plane_smem(n[1], n[2], sizeof(cplx<R>));
-  cudaFuncSetAttribute(k_density_spinor<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  derek::launch(k_density_spinor<R>, dim3(nunits, n[0]), 512, sm, st, t, units, abuf, occ, partial);
+  auto go = [&](auto kern, int threads) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    derek::launch(kern, dim3(nunits, n[0]), threads, sm, st, t, units, abuf, occ, partial);
+  };
+  if (spinor_small(sm))
+    go(k_density_spinor<R, kSpinorThreads>, kSpinorThreads);
+  else
+    go(k_density_spinor<R, 512>, 512);
 }
 
 #define DEREK_INST(R)                                                                                  \
