@@ -133,7 +133,7 @@ struct SysDev {
   double kT;
   long long grid_off;      // offset of this system's grids (nr entries)
   FftPlan plan[3];         // Stockham plans (full-grid transforms)
-  LinePlan lp[3];          // four-step plans (H.psi and density)
+  LinePlan lp[3];          // line splits (H.psi and density)
 };
 
 // One (system, k-point) pair: its plane-wave sphere and buffers.  The
@@ -176,7 +176,8 @@ unsigned long long launch_total();
 // one's blocks has started, and then waits until the previous kernel has
 // completed and its writes are visible.  Nothing runs ahead of the wait, so the
 // order of work is the stream's; what goes is the launch gap between kernels.
-// Only for grids of at most a block per SM, straight into a stream (the adjoint
+// Only for grids of at most a block per SM (the grid FFTs' short blocks: eight),
+// straight into a stream (the adjoint
 // gradient's thousands of small kernels 138 -> 119 ms, a Gamma SCF's first pass 6.4 ->
 // 6.1 ms in all).  Larger grids start unevenly around
 // the waiting predecessor's blocks (band structure 23.4 against 25.1 ms, spinor
@@ -197,8 +198,9 @@ inline int sm_count() {
   return n;
 }
 
-inline bool programmatic_launch(dim3 grid, cudaStream_t stream) {
-  if ((long long)grid.x * grid.y * grid.z > sm_count()) return false;
+// per_sm: blocks per SM up to which a grid counts as small
+inline bool programmatic_launch(dim3 grid, cudaStream_t stream, int per_sm = 1) {
+  if ((long long)grid.x * grid.y * grid.z > per_sm * sm_count()) return false;
   cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(stream, &c) == cudaSuccess && c == cudaStreamCaptureStatusNone;
 }

@@ -191,24 +191,30 @@ struct GridShape {
   }
 };
 
+// The passes are a chain of short kernels with all their blocks resident at once
+// up to 8 per SM, so each starts beside its predecessor (common.cuh): a 32^3 grid
+// forward and back through the ABI 178 -> 174 us.  The shared-memory limit is raised
+// only for lines that need it (the call is host time before every launch).
+template <typename... P, typename... A>
+void grid_pass(void (*kernel)(P...), dim3 grid, size_t smem, cudaStream_t st, A &&...args) {
+  if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  derek::launch_with(derek::programmatic_launch(grid, st, 8), kernel, grid, kGridThreads, smem, st, args...);
+}
+
 template <int SIGN> void cols_y(const GridShape &g, const Tables &t, int s0, double2 *data, int half, int all, cudaStream_t st) {
-  cudaFuncSetAttribute(k_cols_y<SIGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.cols);
-  derek::launch(k_cols_y<SIGN>, g.col_grid(half), kGridThreads, g.cols, st, t, s0, data, g.tz, half, all);
+  grid_pass(k_cols_y<SIGN>, g.col_grid(half), g.cols, st, t, s0, data, g.tz, half, all);
 }
 template <int SIGN, int MODE>
 void cols_x(const GridShape &g, const Tables &t, int s0, double2 *data, int half, int all, double alpha, double q0,
             cudaStream_t st) {
-  cudaFuncSetAttribute(k_cols_x<SIGN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.cols);
-  derek::launch(k_cols_x<SIGN, MODE>, g.col_grid(half), kGridThreads, g.cols, st, t, s0, data, g.tz, half,
+  grid_pass(k_cols_x<SIGN, MODE>, g.col_grid(half), g.cols, st, t, s0, data, g.tz, half,
                                                                                             all, alpha, q0);
 }
 void rows_r2c(const GridShape &g, const Tables &t, const double *rho, double2 *data, int all, cudaStream_t st) {
-  cudaFuncSetAttribute(k_rows_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.rows);
-  derek::launch(k_rows_r2c, g.row_grid(1), kGridThreads, g.rows, st, t, rho, data, all);
+  grid_pass(k_rows_r2c, g.row_grid(1), g.rows, st, t, rho, data, all);
 }
 template <bool ADD> void rows_c2r(const GridShape &g, const Tables &t, const double2 *data, double *out, int all, cudaStream_t st) {
-  cudaFuncSetAttribute(k_rows_c2r<ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.rows);
-  derek::launch(k_rows_c2r<ADD>, g.row_grid(1), kGridThreads, g.rows, st, t, data, out, all);
+  grid_pass(k_rows_c2r<ADD>, g.row_grid(1), g.rows, st, t, data, out, all);
 }
 
 }  // namespace
@@ -218,13 +224,11 @@ void launch_fft3d_grid(const Tables &t, int sys_begin, int nsys, int max_n, doub
   if (nsys <= 0) return;
   const GridShape g(nsys, max_n);
   if (sign < 0) {
-    cudaFuncSetAttribute(k_rows<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.rows);
-    derek::launch(k_rows<-1>, g.row_grid(0), kGridThreads, g.rows, st, t, sys_begin, data);
+    grid_pass(k_rows<-1>, g.row_grid(0), g.rows, st, t, sys_begin, data);
     cols_y<-1>(g, t, sys_begin, data, 0, 1, st);
     cols_x<-1, kPlain>(g, t, sys_begin, data, 0, 1, 0.0, 0.0, st);
   } else {
-    cudaFuncSetAttribute(k_rows<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.rows);
-    derek::launch(k_rows<1>, g.row_grid(0), kGridThreads, g.rows, st, t, sys_begin, data);
+    grid_pass(k_rows<1>, g.row_grid(0), g.rows, st, t, sys_begin, data);
     cols_y<1>(g, t, sys_begin, data, 0, 1, st);
     cols_x<1, kPlain>(g, t, sys_begin, data, 0, 1, 0.0, 0.0, st);
   }
