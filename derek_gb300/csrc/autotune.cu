@@ -20,7 +20,7 @@
 //          coefficients per CTA) of S = X^H X (tensor cores only for
 //          subspaces of 64 bands or more: accuracy, see kTcMinBands);
 //   rotate tensor cores or CUDA cores for X <- X C (the same rule);
-//   jacobi one CTA per k-set or a two-CTA cluster.
+//   jacobi one CTA per k-set, or the cluster of CTAs launch_jacobi picks.
 // The reference plans its FFTs with FFTW_ESTIMATE (Source/fft.f90:204-212),
 // which picks a plan by heuristics without timing; it has no GPU kernels.
 //

@@ -142,10 +142,10 @@ struct derek_gpu {
   // ---- plan choices the autotuner (autotune.cu) may change; the defaults
   // are the untuned plan
   struct Tune {
-    int ksplit = 2048;       // overlap split-K: complex coefficients per CTA (>= kOverlapSplit)
+    int ksplit = 2048;       // overlap split-K: complex coefficients per CTA (CUDA cores: at most)
     int overlap_tc = -1;     // -1: opts.use_tensor_cores decides; 0/1: CUDA cores / tensor cores
     int rotate_tc = -1;
-    int jacobi_single = 0;   // 1: one CTA per k-set even where the two-CTA cluster fits
+    int jacobi_single = 0;   // 1: one CTA per k-set where a solve fits one
     int generic_lines = 0;   // 1: shared-memory line kernels with the runtime splits sys[].lp
     int hpsi_chunk = 0;      // H.psi items per chunk of the three stage launches (0: a class at once)
     std::string source = "default";   // "default", "tuned" or "cache"

@@ -330,7 +330,7 @@ struct AllKept {
 
 // Split N = A * B (A, B <= 16) for the register transforms: a coprime pair
 // when one exists (prime-factor algorithm, no twiddles), the smaller larger
-// factor first; otherwise the four-step split plan_a (Cooley-Tukey).
+// factor first; otherwise the split plan_a (Cooley-Tukey).
 constexpr int reg_split_a(int n) {
   int best = 0, span = 1 << 30;
   for (int x = 2; x <= 16; ++x) {
