@@ -79,6 +79,30 @@ def test_spinor_register_planes(oracle, n, rows):
     assert rel_err(got, oracle.apply_h_spinor(s, kb, nc, psi)) < 2e-5
 
 
+# the largest planes that two blocks of an SM hold (192 threads) and the next
+# smooth length (512 threads)
+@pytest.mark.parametrize("n,precision,tol", [(56, 0, 1e-11), (60, 0, 1e-11), (84, 1, 2e-5), (88, 1, 2e-5)])
+def test_spinor_block_sizes(oracle, n, precision, tol):
+    import derek_gb300 as dg
+    from test_gpu_primitives import make_pair
+    s, spec = make_pair(oracle, L=6.0, ecut=2.9, nb=3, n_fine=(8, n, n), seed=n)
+    spec.nspinor = 2
+    spec.nelec = 2.0
+    kb = oracle.KBasis(s, 0)
+    rng = np.random.default_rng(n + 1)
+    psi = rng.standard_normal((2, s.nbands, kb.npw)) + 1j * rng.standard_normal((2, s.nbands, kb.npw))
+    nc = rng.standard_normal((s.nr, 2, 2)) + 1j * rng.standard_normal((s.nr, 2, 2))
+    occ = np.array([[1.0, 0.0, 0.7]])
+    with dg.Handle(spec, precision=precision) as h:
+        h.set_nc_pot(nc)
+        h.set_wfn(psi)
+        got = h.pot_apply_wfn()
+        rho, mag = h.density_spinor(occ)
+    n_ref, m_ref = oracle.spinor_density(s, kb, psi, occ[0])
+    assert rel_err(got, oracle.apply_h_spinor(s, kb, nc, psi)) < tol
+    assert rel_err(rho, n_ref) < tol and rel_err(mag, m_ref) < tol
+
+
 # every count of bands per thread of the rotations, odd ones among them, and a
 # last G tile that is partly filled: band energies (the lower half, well inside
 # the subspace) against the dense Hamiltonian, bounds as tests/test_gpu_nscf.py
